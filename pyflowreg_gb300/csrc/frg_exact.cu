@@ -1031,7 +1031,7 @@ struct ChannelScale {
 };
 
 __global__ void kx_pad_to_diag(const double* __restrict__ src, int K, int h, int w, DiagGeom g, double* __restrict__ dst,
-                               ChannelScale sc, int scaled)
+                               ChannelScale sc, int scaled, double common)
 {
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
     const int r = blockIdx.y;
@@ -1039,20 +1039,68 @@ __global__ void kx_pad_to_diag(const double* __restrict__ src, int K, int h, int
     if (c >= w || k >= K) return;
     const long long n = w + 2, mn = (long long)(h + 2) * n;
     const long long plane = (long long)g.D * g.P, di = diag_index(g, r, c);
-    const double v = src[k * mn + (long long)(r + 1) * n + c + 1];
+    const double v = dmul(src[k * mn + (long long)(r + 1) * n + c + 1], common);
     dst[k * plane + di] = v;
     if (scaled) dst[(K + k) * plane + di] = dmul(v, sc.s[k]);
 }
 
 cudaError_t launch_x_pad_to_diag(const double* src, int K, int h, int w, DiagGeom g, double* dst, cudaStream_t st,
-                                 const double* scale)
+                                 const double* scale, double common)
 {
     if (K < 1 || K > kMaxK) return cudaErrorInvalidValue;
     ChannelScale sc = {};
     if (scale)
         for (int k = 0; k < K; ++k) sc.s[k] = scale[k];
     dim3 blk(128), grd((w + 127) / 128, h, K);
-    kx_pad_to_diag<<<grd, blk, 0, st>>>(src, K, h, w, g, dst, sc, scale ? 1 : 0);
+    kx_pad_to_diag<<<grd, blk, 0, st>>>(src, K, h, w, g, dst, sc, scale ? 1 : 0, common);
+    return cudaGetLastError();
+}
+
+// The level solver seam's arrays, (m, n, K) with a ring, to the chained SOR's
+// diagonal-major form: J (J11, J22, J33 + 1e-5, 2 J12, 2 J13, 2 J23), W and
+// W a_data, and the smoothness constants of u, v (core/level_solver.py:317-340).
+__global__ void kx_seam_to_diag(const double* __restrict__ J, const double* __restrict__ wgt, const double* __restrict__ u,
+                                const double* __restrict__ v, int K, int h, int w, DiagGeom g, double wx, double wy,
+                                ChannelScale ad, double* __restrict__ Jd, double* __restrict__ Wd,
+                                double* __restrict__ Wfx, double per_wsum, double* __restrict__ lap)
+{
+    const int c = blockIdx.x * blockDim.x + threadIdx.x;
+    const int r = blockIdx.y;
+    if (c >= w) return;
+    const long long n = w + 2, mn = (long long)(h + 2) * n;
+    const long long plane = (long long)g.D * g.P, di = diag_index(g, r, c);
+    const long long o = (long long)(r + 1) * n + c + 1;
+    for (int k = 0; k < K; ++k) {
+        for (int q = 0; q < 6; ++q) {
+            const double x = J[(q * mn + o) * K + k];
+            Jd[(q * K + k) * plane + di] = q < 2 ? x : (q == 2 ? dadd(x, 0.00001) : dadd(x, x));
+        }
+        const double x = wgt[o * K + k];
+        Wd[k * plane + di] = x;
+        Wd[(K + k) * plane + di] = dmul(x, ad.s[k]);
+        Wfx[k * plane + di] = dmul(x, per_wsum);
+        Wfx[(K + k) * plane + di] = dmul(dmul(x, ad.s[k]), per_wsum);
+    }
+    for (int q = 0; q < 2; ++q) {
+        const double* a = q ? v : u;
+        const double x = a[o];
+        double s = dmul(wx, dsub(a[o - 1], x));
+        s = dadd(s, dmul(wx, dsub(a[o + 1], x)));
+        s = dadd(s, dmul(wy, dsub(a[o + n], x)));
+        s = dadd(s, dmul(wy, dsub(a[o - n], x)));
+        lap[q * plane + di] = s;
+    }
+}
+
+cudaError_t launch_x_seam_to_diag(const double* J, const double* wgt, const double* u, const double* v, int K, int h,
+                                  int w, DiagGeom g, double wx, double wy, const double* a_data, double* Jd, double* Wd,
+                                  double* Wfx, double* lap, cudaStream_t st)
+{
+    if (K < 1 || K > kMaxK) return cudaErrorInvalidValue;
+    ChannelScale sc = {};
+    for (int k = 0; k < K; ++k) sc.s[k] = a_data[k];
+    dim3 blk(128), grd((w + 127) / 128, h);
+    kx_seam_to_diag<<<grd, blk, 0, st>>>(J, wgt, u, v, K, h, w, g, wx, wy, sc, Jd, Wd, Wfx, 1.0 / (((wx + wx) + wy) + wy), lap);
     return cudaGetLastError();
 }
 

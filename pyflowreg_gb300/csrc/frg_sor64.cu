@@ -170,6 +170,8 @@ struct Sor64Args {
     double a_m1[kMaxK];  // a_data - 1
     PowTab64 pw[kMaxK];  // the power's table per channel (null table: the general power)
     int nc;              // row strips (CTAs) per frame
+    const int* marks;    // frames to compute (fx_recompute); null: all
+    int ring;            // the final pass also writes the border copies around the output
 };
 
 struct Chain64Table {
@@ -331,6 +333,7 @@ __global__ void __launch_bounds__(NTM, StripBounds<NTM>::blocks) k_sor_chain64(S
     const int strip = CL ? (int)(blockIdx.x % nc) : 0;
     const int f = CL ? (int)(blockIdx.x / nc) : (int)blockIdx.x;
     const int r = strip * NT + t;  // the level row of this thread
+    if (A.marks && !fx_recompute(A.marks[f])) return;  // the same for every CTA of a cluster
     double2* CA = reinterpret_cast<double2*>(sm64);
     double2* CB = CA + S * NT;
     double* CC = reinterpret_cast<double*>(CB + S * NT);
@@ -492,6 +495,15 @@ __global__ void __launch_bounds__(NTM, StripBounds<NTM>::blocks) k_sor_chain64(S
                             if (final_out) {
                                 odu[(long long)r * A.out_rs + c] = V0[gi].x;
                                 odv[(long long)r * A.out_rs + c] = V0[gi].y;
+                                if (A.ring && (c == 0 || c == w - 1 || r == 0 || r == h - 1)) {
+                                    const long long o = (long long)r * A.out_rs + c;
+                                    for (int yr = r == 0 ? -1 : 0; yr <= (r == h - 1 ? 1 : 0); ++yr)
+                                        for (int xc = c == 0 ? -1 : 0; xc <= (c == w - 1 ? 1 : 0); ++xc)
+                                            if (yr | xc) {
+                                                odu[o + (long long)yr * A.out_rs + xc] = own.x;
+                                                odv[o + (long long)yr * A.out_rs + xc] = own.y;
+                                            }
+                                }
                             } else {
                                 dur[(r + c) * P] = V0[gi].x;
                                 dvr[(r + c) * P] = V0[gi].y;
@@ -633,7 +645,7 @@ cudaError_t launch_sor_chain64(const double* J, long long J_fs, const double* W,
                                long long st_fs, int n_frames, int K, DiagGeom g, const ChainPass* passes,
                                int n_passes, const double* a_data, double wx, double wy, double omega,
                                cudaStream_t st, double* out_du, double* out_dv, long long out_fs, int out_rs,
-                               int rows, const PowTab64* pows)
+                               int rows, const PowTab64* pows, const int* marks, int ring)
 {
     if (!sor_chain64_supports(K, g, n_passes) || n_frames < 1) return cudaErrorInvalidValue;
     if (rows == 0) rows = kLane64;
@@ -669,6 +681,8 @@ cudaError_t launch_sor_chain64(const double* J, long long J_fs, const double* W,
     A.out_dv = out_dv;
     A.out_fs = out_fs;
     A.out_rs = out_rs;
+    A.marks = marks;
+    A.ring = ring;
     A.g = g;
     A.wa = wy;  // the thread index runs along rows: row neighbours carry the y weight
     A.wb = wx;

@@ -1,0 +1,936 @@
+// Exact-order chained SOR of the float64 path with the updates in 64-bit
+// fixed point.
+//
+// compute_flow (core/level_solver.py:158-369) sweeps columns outer, rows inner,
+// in place, in float64.  On GB300 one float64 instruction holds a scheduler's
+// float64 pipe for 64 clocks (2 lanes per clock per SM; a dependent chain sees
+// the same 64 clocks), while a 32 x 32 -> 64-bit product issues every 2 clocks.
+// An update of 14 float64 operations therefore costs 896 clocks per warp; the
+// same update on two-limb integers costs about 60 instructions.  So the state
+// (du, dv) is held in 64-bit fixed point and updated on the integer pipe, and
+// only the fold of the coefficients, once per pass of up to five updates, uses
+// float64.
+//
+// Number format.  A state value x is an integer multiple of 2^-q, split as
+// x = h 2^30 + l with a balanced low limb l in [-2^29, 2^29).  Coefficients are
+// multiples of 2^-60 below 1, split the same way.  With
+//   c = omega w / den,  a 2^k = -omega A12 / den,  p = omega B / den
+// folded per pixel and pass (k the smallest exponent with |a| < 1), an update is
+//   du <- (1 - omega) du + c (up + down + left + right) + a 2^k dv + p
+// (c per axis when the two smoothness weights differ).  The products h h and
+// h l + l h are summed exactly in 64-bit accumulators and rounded once, to the
+// nearest multiple of 2^-q; the l l products (below one unit of 2^-q for the
+// sums, 2^(k - 2) units for a, with a sign that varies with both limbs) are left
+// out.  Exact zeros stay zero.  The error of an update is thus about one unit of
+// 2^-q (2^-56 px on the finest levels), where float64 rounds |du| ~ 1 px sums to
+// 2^-53 several times.
+//
+// Range.  States are held below 2^lim units, |a 2^k| below 2^kmax and p below
+// 2^62 units, with lim + kmax = 63: then the sum of the true terms stays below
+// 2^64 - 2^lim, so a sum that wraps cannot land in the range of a state.  A
+// frame's unit follows its size: q = lim - reach, where 2^reach px bounds the
+// largest |du|, |dv| that the frame reached on the coarser level, with a bit to
+// spare.  A coefficient or a state outside its range, or anything not finite,
+// marks the frame, and so does a level whose result is nowhere above 2^42 units
+// but not zero (so small that a float64 state would hold more bits).  Marked
+// frames are solved again by a second launch with a wider format, and what that
+// one marks by k_sor_chain64.
+//
+// Schedule: that of k_sor_chain64 (row r's local time is tau = s - r; pixel
+// (r, c) of pipelined iteration gi of a pass is updated at tau = start + c +
+// 2 gi), with the work split over specialised warps.  Every 32 rows have NU
+// update warps, which share the five pipelined iterations, and FC fold warps,
+// which run ahead of them: fold warp j takes steps j, j + FC, ..., and writes
+// each entering pixel's coefficients and pass-start state into a ring of kFxRing
+// slots in shared memory (mbarriers both ways).  The folds' float64
+// instructions and loads are off the update's critical path, and the float64
+// pipes of all four schedulers work on one row strip.  An update's neighbours
+// come from shared memory: each iteration writes its new values to a buffer of
+// the last three steps, from which the next iteration reads the right, lower
+// and own values and the row below the upper one; one barrier per step.  A
+// frame's strips in other CTAs of its cluster get the edge rows through
+// distributed shared memory (st.async with a transaction barrier).
+#include "frg_internal.h"
+
+#include <cooperative_groups.h>
+
+#include <algorithm>
+#include <cmath>
+
+namespace frg {
+
+namespace {
+
+constexpr int kFxRing = 16;          // ring slots: a pixel's coefficients are read for 2 (G - 1) + 1 = 9 steps
+constexpr int kFxUse = 2 * (kGMax - 1);
+constexpr int kFxAhead = kFxRing - kFxUse;  // steps a fold may run ahead of the update
+constexpr int kFxMaxStrips = 64;
+constexpr int kFxMaxCluster = 16;
+constexpr int kFxKmax = 4, kFxLim = 63 - kFxKmax;  // |omega A12 / den| stays below 16 but for rare pixels of coarse levels
+constexpr int kFxWider = 3;          // bits by which the second launch widens both
+constexpr int kFxReachMin = 1, kFxReachMax = 10;
+constexpr unsigned kFxSpin = 500000u;       // bound of every wait, in tries of at most 2 us; a wait that runs out marks the frame
+
+struct FxArgs {
+    const double* J;
+    long long J_fs;
+    const double* W;     // [2][K][D*P]: W / wsum, W a_data / wsum
+    long long W_fs;
+    const double* lap;
+    long long lap_fs;
+    double* wp;          // [K][D*P]: weights times psi of passes that continue a group
+    long long wp_fs;
+    long long* du;       // [D*P] pass-to-pass state, multiples of 2^-q
+    long long* dv;
+    long long st_fs;
+    double* out_du;      // final pass, at out + r * out_rs + c
+    double* out_dv;
+    long long out_fs;
+    int out_rs;
+    int ring;            // also write the border copies around the output (rows -1 and h, columns -1 and w)
+    DiagGeom g;
+    double lap_scale;    // 2 / wsum
+    long long half_omega, ca, cb;  // omega / 2, 2 wa / wsum, 2 wb / wsum: 61 fraction bits
+    int oh, ol;          // 1 - omega
+    FxPow pw[4];
+    FxState fs;
+    int lim, kmax, reach;  // reach < 0: from the frame's previous level
+    int second;          // second launch: frames the first one marked, format wider by kFxWider bits
+    int nc;              // CTAs per frame
+};
+
+struct FxTable {
+    int n;
+    int pk[kMaxChain];  // G << 8 | store << 3 | coef << 2 | tick << 1 | zero
+};
+
+constexpr int kPkZero = 1, kPkTick = 2, kPkCoef = 4, kPkStore = 8;
+
+__device__ __forceinline__ unsigned smem_addr(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
+
+__device__ __forceinline__ void mbar_init(unsigned mb, unsigned count)
+{
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(mb), "r"(count) : "memory");
+}
+
+__device__ __forceinline__ void mbar_arrive(unsigned mb)
+{
+    asm volatile("{\n\t.reg .b64 t;\n\tmbarrier.arrive.release.cta.shared::cta.b64 t, [%0];\n\t}" ::"r"(mb) : "memory");
+}
+
+__device__ __forceinline__ void mbar_expect(unsigned mb, unsigned bytes)
+{
+    asm volatile("{\n\t.reg .b64 t;\n\tmbarrier.arrive.expect_tx.relaxed.cta.shared::cta.b64 t, [%0], %1;\n\t}" ::"r"(mb),
+                 "r"(bytes)
+                 : "memory");
+}
+
+__device__ __forceinline__ void mbar_arrive_expect(unsigned mb, unsigned bytes)
+{
+    asm volatile("{\n\t.reg .b64 t;\n\tmbarrier.arrive.expect_tx.release.cta.shared::cta.b64 t, [%0], %1;\n\t}" ::"r"(mb),
+                 "r"(bytes)
+                 : "memory");
+}
+
+// 16 bytes into another CTA's shared memory, counted by a barrier there.  A
+// predicated instruction: a branch around it costs the step about 50 clocks.
+__device__ __forceinline__ void st_async_if(bool p, unsigned addr, int4 v, unsigned mb)
+{
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.s32 p, %6, 0;\n\t"
+                 "@p st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v4.b32 [%0], {%1, %2, %3, %4}, [%5];\n\t}" ::"r"(addr),
+                 "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w), "r"(mb), "r"((int)p)
+                 : "memory");
+}
+
+__device__ __forceinline__ void st_global_if(bool p, long long* a, long long v)
+{
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.s32 p, %2, 0;\n\t@p st.global.b64 [%0], %1;\n\t}" ::"l"(a), "l"(v), "r"((int)p)
+                 : "memory");
+}
+
+__device__ __forceinline__ bool mbar_test(unsigned mb, unsigned parity)
+{
+    unsigned ok;
+    asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2, 2000;\n\t"
+                 "selp.u32 %0, 1, 0, p;\n\t}"
+                 : "=r"(ok)
+                 : "r"(mb), "r"(parity)
+                 : "memory");
+    return ok != 0;
+}
+
+// Waits for the phase with this parity to complete.  After one wait has run
+// out no further one is made (the frame is marked and recomputed).
+__device__ __forceinline__ void mbar_wait(unsigned mb, unsigned parity, bool& dead)
+{
+    if (dead) return;
+    for (unsigned i = 0; i < kFxSpin; ++i)
+        if (mbar_test(mb, parity)) return;
+    dead = true;
+}
+
+__device__ __forceinline__ long long mulw(int a, int b) { return (long long)a * b; }
+
+// Limbs of an integer: v = h 2^30 + l, l in [-2^29, 2^29).
+__device__ __forceinline__ int2 limbs(long long v)
+{
+    const long long u = v + (1 << 29);
+    return make_int2((int)(u >> 30), (int)((unsigned)u & 0x3fffffffu) - (1 << 29));
+}
+
+// Top 64 bits of a 128-bit product, shifted left by k: a b 2^(k - 64) for
+// |a|, |b| < 2^62, within about 2^(k + 1) units.
+template <int k>
+__device__ __forceinline__ long long mulh(long long a, long long b)
+{
+    const int ah = (int)(a >> 32), bh = (int)(b >> 32);
+    const int al = (int)((unsigned)a >> 1), bl = (int)((unsigned)b >> 1);
+    return (mulw(ah, bh) << k) + ((mulw(ah, bl) + mulw(bh, al)) >> (31 - k));
+}
+
+// Integer times 2^-q as a double, to nearest; on the integer pipe.
+__device__ __forceinline__ double fx_to_double(long long v, int q)
+{
+    if (v == 0) return 0.0;
+    const unsigned long long m = (unsigned long long)(v < 0 ? -v : v);
+    const int n = __clzll((long long)m);
+    const unsigned long long x = m << n, t = (x >> 11) + ((x >> 10) & 1);  // 53 bits (2^53 when it rounds up)
+    const unsigned long long e = (unsigned long long)(63 - n - q + 1022);
+    return __longlong_as_double((long long)(((e << 52) + t) | (v < 0 ? 0x8000000000000000ull : 0ull)));
+}
+
+// Magnitude of a double's mantissa with 61 fraction bits below its leading one
+// (in [2^61, 2^62)); d = +-m 2^(e - 1084), e the biased exponent (0: d is taken
+// as zero or too small to matter).
+__device__ __forceinline__ long long mantissa61(double d)
+{
+    return (long long)(((unsigned long long)(((unsigned)__double2hiint(d) & 0xfffffu) | 0x100000u) << 41) |
+                       ((unsigned long long)(unsigned)__double2loint(d) << 9));
+}
+__device__ __forceinline__ int exponent_of(double d) { return (__double2hiint(d) >> 20) & 0x7ff; }
+
+// +-m 2^-n as whole units (rounded down) and a 30-bit fraction, the latter plus
+// 2^29 (half a unit, for the update's rounding); m < 2^62, n >= 1.
+__device__ __forceinline__ void split_units(long long m, int n, bool neg, long long& whole, int& frac)
+{
+    const unsigned long long v = n > 63 ? 0ull : (unsigned long long)m >> n;
+    const unsigned long long lost = n > 94 ? 0ull : (n > 63 ? (unsigned long long)m >> (n - 64) : (unsigned long long)m << (64 - n));
+    int f = (int)(lost >> 34);
+    whole = (long long)v;
+    if (neg) {
+        whole = ~whole + (f == 0);
+        f = (-f) & 0x3fffffff;
+    }
+    frac = f + (1 << 29);
+}
+
+// w x^b for 1e-5 <= x < 2^47 and |b| <= 1 on the integer pipe: x = 2^e m,
+// m in [1, 2), R an integer near 2^16 / m from the top 8 bits of m's fraction,
+// r = m R 2^-16 - 1 exactly (|r| < 2^-8.9; the product's low 64 bits), and
+//   x^b = 2^(e b) (2^16 / R)^b (1 + r)^b
+// with both factors tabulated and (1 + r)^b - 1 by its binomial series to r^6
+// (the next term is below 2^-62).  All steps carry at least 2^-58 relative
+// precision; the product with w is rounded once to float64.  7 float64
+// operations (448 clocks of a scheduler's pipe) become about 80 integer
+// instructions.
+__device__ __forceinline__ double fx_wpow(double w, double x, const FxPow& P, int& bad)
+{
+    const int hi = __double2hiint(x);
+    const unsigned e = (unsigned)((hi >> 20) - (1023 + kPowEMin));
+    bad |= e >= 64u;
+    const unsigned ec = e & 63u;
+    const unsigned j = ((unsigned)hi >> 12) & 0xffu;
+    const unsigned mh = ((unsigned)hi & 0xfffffu) | 0x100000u;
+    const unsigned ml = (unsigned)__double2loint(x);
+    const unsigned R = P.R[j];
+    const long long B = P.B[j];
+    const longlong2 Am = P.A[ec];
+    // r 2^68
+    const long long r = (long long)((unsigned long long)ml * R + ((unsigned long long)(mh * R) << 32));
+    const int rh = (int)(r >> 29);  // r 2^39
+    int t = P.c5 + ((int)(mulw(rh, P.c6) >> 32) >> 7);
+    t = P.c4 + ((int)(mulw(rh, t) >> 32) >> 7);
+    t = P.c3 + ((int)(mulw(rh, t) >> 32) >> 7);
+    const long long p2 = P.c2 + (mulw(rh, t) >> 9);       // 2^60
+    const long long p1 = P.c1 + (mulh<0>(r, p2) >> 4);    // 2^60
+    const long long s = mulh<0>(r, p1);                   // 2^64
+    const long long AB = mulh<3>(Am.x, B);                // 2^60, in [2^59, 2^62)
+    const int ew = exponent_of(w);
+    bad |= ew > 1023 + 60;
+    const long long v = mulh<2>(AB + mulh<0>(AB, s), mantissa61(w));
+    const double d = fx_to_double(v, 1082 - ew - (int)Am.y);
+    return ew == 0 ? 0.0 : (__double2hiint(w) < 0 ? -d : d);
+}
+
+// (omega / 2) / d for d >= 1 as v 2^-(62 + ex), v in [2^60, 2^62): a float32
+// reciprocal of d's mantissa, its exact error 1 - m y (the product's low 64
+// bits) and y + y (e + e^2), to 2^-60; about 45 integer instructions for 4
+// float64 operations (256 clocks).
+__device__ __forceinline__ long long fx_half_omega_over(double d, long long half_omega, int& ex, int& bad)
+{
+    const int hi = __double2hiint(d);
+    const unsigned lo = (unsigned)__double2loint(d);
+    ex = (hi >> 20) - 1023;
+    bad |= (unsigned)ex > 60u;
+    float yf;
+    asm("rcp.approx.ftz.f32 %0, %1;"
+        : "=f"(yf)
+        : "f"(__uint_as_float(0x3f800000u | ((unsigned)hi & 0xfffffu) << 3 | lo >> 29)));
+    const int y0 = __float_as_int(yf + 1.0f) - 0x3f800000;  // y 2^23
+    const unsigned mh = ((unsigned)hi & 0xfffffu) | 0x100000u;
+    const long long e = -(long long)((unsigned long long)lo * (unsigned)y0 + ((unsigned long long)(mh * (unsigned)y0) << 32));
+    const int eh = (int)(e >> 24);                           // e 2^75 before, 2^51 here; |e| < 2^-20
+    const long long t = e + (mulw(eh, eh) >> 27);
+    const long long tl = (long long)((unsigned long long)(unsigned)t * (unsigned)y0);
+    const long long y = ((long long)y0 << 39) + ((mulw(y0, (int)(t >> 32)) + (long long)((unsigned long long)tl >> 32)) >> 4);
+    return mulh<3>(y, half_omega);
+}
+
+template <int K>
+struct FxIn {
+    double j[6 * K];
+    double w[K];
+    double lu, lv;
+};
+
+// Ring planes, int4 each: (c_u, c_v), (a_u, a_v), (p_u, p_v) whole units, (k_u,
+// k_v, p's fractions), state (one row more: the next strip's first row), and the
+// second smoothness coefficient pair when the axes' weights differ.
+constexpr int kPC = 0, kPA = 1, kPP = 2, kPK = 3, kPS = 4, kPD = 5;
+
+// Folds one pixel's coefficients (core/level_solver.py:229-255, 309-364).  The
+// weights come divided by wsum = 2 (wx + wy), so with the tensor's cross terms
+// doubled and sums S over the channels
+//   d = 1 + S W psi J11,  c = (2 w / wsum) D,  a 2^k = -(S W psi 2 J12) D,
+//   p = (2 lap / wsum - S W psi 2 J13) D,  D = (omega / 2) / d.
+// The quadratic form E and the sums are float64 (11 K + 2 operations less the
+// power); the power, the reciprocals and the products with D are integers.
+template <int K, bool ISO>
+__device__ __forceinline__ void fx_fold(const FxArgs& A, const FxPow* pw, int pk, const FxIn<K>& in, long long su,
+                                        long long sv, double* wp_io, int wp_plane, int4* slot, int plane, int q, int kmax,
+                                        int& bad)
+{
+    const bool tick = (pk & kPkTick) != 0;
+    double den[2] = {1.0, 1.0}, a12 = 0.0, c3[2] = {0.0, 0.0};
+    double a = 0.0, b = 0.0;
+    if (tick) {
+        a = fx_to_double(su, q);
+        b = fx_to_double(sv, q);
+    }
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+        const double j11 = in.j[0 * K + k], j22 = in.j[1 * K + k], j33 = in.j[2 * K + k];
+        const double j12 = in.j[3 * K + k], j13 = in.j[4 * K + k], j23 = in.j[5 * K + k];
+        double wp = in.w[k];
+        if (tick) {
+            double t = __fma_rn(j11, a, j13);
+            t = __fma_rn(j12, b, t);
+            const double v = __fma_rn(j22, b, j23);
+            double E = __fma_rn(t, a, __fma_rn(v, b, j33));
+            if (__double_as_longlong(E) < __double_as_longlong(0.00001)) E = 0.00001;
+            wp = fx_wpow(wp, E, pw[k], bad);
+        }
+        if (pk & kPkStore) wp_io[k * wp_plane] = wp;
+        den[0] = __fma_rn(wp, j11, den[0]);
+        den[1] = __fma_rn(wp, j22, den[1]);
+        a12 = __fma_rn(wp, j12, a12);
+        c3[0] = __fma_rn(wp, j13, c3[0]);
+        c3[1] = __fma_rn(wp, j23, c3[1]);
+    }
+    // c < 1/2 for one coefficient over four neighbours, < 1 for one per axis
+    int4 vc, va, vp, vk, vd;
+    int* oc = &vc.x;
+    int* oa = &va.x;
+    int* op = &vp.x;
+    int* ok = &vk.x;
+    int* od = &vd.x;
+    const long long m12 = mantissa61(a12);
+    const int e12 = exponent_of(a12);
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+        int ex;
+        const long long D = fx_half_omega_over(den[i], A.half_omega, ex, bad);
+        int2 x = limbs(mulh<3>(D, A.ca) >> min(2 + ex, 63));
+        oc[2 * i] = x.x;
+        oc[2 * i + 1] = x.y;
+        if (!ISO) {
+            x = limbs(mulh<3>(D, A.cb) >> min(2 + ex, 63));
+            od[2 * i] = x.x;
+            od[2 * i + 1] = x.y;
+        }
+        // |a12| D = v 2^(z - 62) with v < 2^62
+        const int z = e12 - 1084 - ex + 62;
+        const int k = max(0, z);
+        bad |= k > kmax;
+        const long long v = mulh<2>(m12, D) >> min(2 + max(0, -z), 63);
+        x = limbs(__double2hiint(a12) < 0 ? v : -v);
+        oa[2 * i] = x.x;
+        oa[2 * i + 1] = x.y;
+        ok[i] = k & 31;
+        const double bb = __fma_rn(A.lap_scale, i ? in.lv : in.lu, -c3[i]);
+        const int n = 1084 + ex - q - exponent_of(bb);
+        bad |= n < 1;
+        long long whole;
+        split_units(mulh<2>(mantissa61(bb), D), max(n, 1), __double2hiint(bb) < 0, whole, ok[2 + i]);
+        // 2^29 units are added so that the update's result is already offset for its split into limbs
+        whole += 1 << 29;
+        op[2 * i] = (int)whole;
+        op[2 * i + 1] = (int)(whole >> 32);
+    }
+    slot[kPC * plane] = vc;
+    slot[kPA * plane] = va;
+    slot[kPP * plane] = vp;
+    slot[kPK * plane] = vk;
+    if (!ISO) slot[kPD * plane] = vd;
+}
+
+// 32 x 32 -> 64 bits.  As an instruction of its own: the fused multiply-add with
+// a 64-bit addend issues at 25 lanes per clock against 63 (measured), and a
+// chain of them waits 12.5 clocks a link against 9 for a product and a sum.
+__device__ __forceinline__ long long mulx(int a, int b)
+{
+    long long r;
+    asm("mul.wide.s32 %0, %1, %2;" : "=l"(r) : "r"(a), "r"(b));
+    return r;
+}
+
+// One component's update; p and the result are offset by 2^29, f holds p's
+// fraction plus half a unit.
+template <bool ISO>
+__device__ __forceinline__ long long fx_point(int oh, int ol, int ch, int cl, int dh, int dl, int ah, int al, int k, int f,
+                                              long long p, int own_h, int own_l, int oth_h, int oth_l, int s_h, int s_l,
+                                              int t_h, int t_l)
+{
+    long long M = f + mulx(oh, own_l) + mulx(ol, own_h);
+    long long H = p + mulx(oh, own_h);
+    if (!ISO) {
+        M += mulx(dh, t_l) + mulx(dl, t_h);
+        H += mulx(dh, t_h);
+    }
+    M += mulx(ch, s_l) + mulx(cl, s_h);
+    H += mulx(ch, s_h);
+    const long long MA = mulx(ah, oth_l) + mulx(al, oth_h);
+    return H + (mulx(ah, oth_h) << k) + (((M >> k) + MA) >> (30 - k));
+}
+
+__device__ __forceinline__ int4 sel4(bool c, int4 a, int4 b)
+{
+    return make_int4(c ? a.x : b.x, c ? a.y : b.y, c ? a.z : b.z, c ? a.w : b.w);
+}
+__device__ __forceinline__ long long join(int h, int l) { return ((long long)h << 30) + l; }
+
+constexpr int kFxTabBytes = 64 * 16 + 256 * 8 + 256 * 4;
+
+// Shared memory of a CTA of M strips: ring int4[planes][kFxRing][32 M] with the
+// state plane's halo int4[kFxRing] | iteration buffers int4[G][3][32 M + 2] |
+// mbarriers: full[M][kFxRing], empty[M][kFxRing], edge[2 parities] | the power table where there is room.
+template <int M, bool ISO>
+struct FxSmem {
+    static constexpr int rows = 32 * M;
+    static constexpr int plane = kFxRing * (rows + 1);  // int4 per ring plane (the halo row only used by the state)
+    static constexpr int planes = ISO ? 5 : 6;
+    static constexpr int buf = rows + 2;
+    static constexpr size_t bytes =
+        ((size_t)planes * plane + (size_t)kGMax * 3 * buf) * sizeof(int4) + (size_t)(2 * M * kFxRing + 2) * 8;
+    static constexpr bool table = M < 4;  // room for a power table
+    static constexpr size_t bytes_all = bytes + (table ? kFxTabBytes : 0);
+};
+
+// The border copies around pixel (r, c): its value before the last iteration
+// (set_boundary_2d, core/level_solver.py:45-66).
+__device__ __noinline__ void fx_ring(double* odu, double* odv, int rs, int r, int c, int h, int w, int4 own, int q)
+{
+    if (c != 0 && c != w - 1 && r != 0 && r != h - 1) return;
+    const double bu = fx_to_double(join(own.x, own.y), q), bv = fx_to_double(join(own.z, own.w), q);
+    for (int y = r == 0 ? -1 : r; y <= (r == h - 1 ? h : r); ++y)
+        for (int x = c == 0 ? -1 : c; x <= (c == w - 1 ? w : c); ++x)
+            if (y != r || x != c) {
+                odu[(long long)y * rs + x] = bu;
+                odv[(long long)y * rs + x] = bv;
+            }
+}
+
+__host__ __device__ __forceinline__ void place_fx(const void* tab, FxPow* P)
+{
+    P->A = static_cast<const longlong2*>(tab);
+    P->B = reinterpret_cast<const long long*>(P->A + 64);
+    P->R = reinterpret_cast<const unsigned*>(P->B + 256);
+}
+
+// Steps a row spends in a pass.  After a single iteration one step more, so that
+// the step before a row's first pixel of the next pass (which takes that
+// pixel's value as its right neighbour) is free.
+__device__ __forceinline__ int fx_span(int w, int pk)
+{
+    const int n = pk >> 8;
+    return w + (n > 1 ? 2 * (n - 1) : 1);
+}
+
+// A row's place in the chain of passes at local time tau.
+struct Cursor {
+    int p, start, end, pk;
+    __device__ __forceinline__ void init(const FxTable& T, int w)
+    {
+        p = 0;
+        start = 0;
+        pk = T.pk[0];
+        end = fx_span(w, pk);
+    }
+    __device__ __forceinline__ void advance(const FxTable& T, int w, int tau)
+    {
+        if (tau >= end && p < T.n - 1) {
+            ++p;
+            start = end;
+            pk = T.pk[p];
+            end = start + fx_span(w, pk);
+        }
+    }
+};
+
+template <int K, bool ISO, int M, int NU, int FC>
+__global__ void __launch_bounds__(32 * (M * (NU + FC) + 1)) k_sor_fx(FxArgs A, FxTable T)
+{
+    using SM = FxSmem<M, ISO>;
+    constexpr int G = kGMax;
+    constexpr int S = kFxRing;
+    constexpr int ROWS = SM::rows, PL = SM::plane, SR = ROWS + 1, BUF = SM::buf;
+    extern __shared__ __align__(16) unsigned char fx_sm[];
+    int4* ring = reinterpret_cast<int4*>(fx_sm);
+    int4* bufs = ring + SM::planes * PL;
+    unsigned long long* bars = reinterpret_cast<unsigned long long*>(bufs + G * 3 * BUF);
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+    const int nc = A.nc;
+    const int cta = nc > 1 ? (int)(blockIdx.x % nc) : 0;
+    const int f = nc > 1 ? (int)(blockIdx.x / nc) : (int)blockIdx.x;
+    if (A.second && !fx_recompute(A.fs.marks[f])) return;  // the same for every CTA of a cluster
+    // warps: M NU for the update (strip, iterations), one that waits for them, M FC for the fold
+    constexpr int WU = M * NU;
+    const int strip = (warp < WU ? warp : warp - WU - 1) % M;
+    const int row = strip * 32 + lane;  // in the CTA
+    const int r = cta * ROWS + row;     // in the level
+    const DiagGeom g = A.g;
+    const int P = g.P, h = g.h, w = g.w;
+    const int pl = g.D * P;
+    const bool row_ok = r < h;
+    const bool above = cta > 0, below = cta + 1 < nc;  // other CTAs of the frame
+    auto full_bar = [&](int st, int slot) { return smem_addr(bars + st * S + slot); };
+    auto empty_bar = [&](int st, int slot) { return smem_addr(bars + M * S + st * S + slot); };
+    auto edge_bar = [&](int par) { return smem_addr(bars + 2 * M * S + par); };
+    // bytes a step's edge rows bring: every iteration's from above, all but the last one's from below
+    const unsigned edge_bytes = (above ? G * sizeof(int4) : 0) + (below ? (G - 1) * sizeof(int4) : 0);
+    // the power's table in shared memory when the channels share one: a fold's three look-ups
+    // are dependent loads, about 700 clocks each from L2
+    bool one = SM::table;
+    for (int k = 1; k < K; ++k) one = one && A.pw[k].A == A.pw[0].A;
+    int4* tab = reinterpret_cast<int4*>(bars + 2 * M * S + 2);
+    if (one)
+        for (int i = t; i < kFxTabBytes / 16; i += blockDim.x) tab[i] = reinterpret_cast<const int4*>(A.pw[0].A)[i];
+    if (t == 0) {
+        for (int i = 0; i < 2 * M * S + 2; ++i) mbar_init(smem_addr(bars + i), 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        if (nc > 1)
+            for (int par = 0; par < 2; ++par) mbar_expect(edge_bar(par), edge_bytes);
+    }
+    auto sync_all = [&]() {
+        if (nc > 1)
+            cooperative_groups::this_cluster().sync();
+        else
+            __syncthreads();
+    };
+    sync_all();
+
+    // the frame's format
+    int reach = A.reach;
+    if (reach < 0) {
+        reach = fx_recompute(A.fs.prev_marks[f]) ? A.fs.prev_reach2[f] : A.fs.prev_reach[f];
+        reach = min(max(reach + 1, kFxReachMin), kFxReachMax);
+    }
+    const int kmax = A.kmax + (A.second ? kFxWider : 0);
+    const int lim = A.lim - (A.second ? kFxWider : 0);
+    const int q = lim - reach - (A.second ? kFxWider : 0);
+
+    double* odu = A.out_du + f * A.out_fs;
+    double* odv = A.out_dv + f * A.out_fs;
+    int total = 0;
+    for (int p = 0; p < T.n; ++p) total += fx_span(w, T.pk[p]);
+    const int nsteps = total + h - 1;
+    bool dead = false;
+    int bad = 0, big = 0, nonzero = 0, top = 0;
+    Cursor cur;
+    cur.init(T, w);
+
+    if (warp > WU) {
+        // ------------------------------------------------------------ fold
+        const int fj = (warp - WU - 1) / M;
+        FxPow pw[K];
+#pragma unroll
+        for (int k = 0; k < K; ++k) {
+            pw[k] = A.pw[k];
+            if (one) place_fx(tab, &pw[k]);
+        }
+        const double* Jr = A.J + f * A.J_fs + r;
+        const double* Wr = A.W + f * A.W_fs + r;
+        const double* lapr = A.lap + f * A.lap_fs + r;
+        double* wpr = A.wp + f * A.wp_fs + r;
+        const long long* dur = A.du + f * A.st_fs + r;
+        const long long* dvr = A.dv + f * A.st_fs + r;
+        // the first row's state also goes to the CTA above, as the row below its last one
+        const bool sends = above && row == 0;
+        unsigned halo = smem_addr(ring + kPS * PL + ROWS), halo_bar = full_bar(M - 1, 0);
+        if (sends) {
+            asm("mapa.shared::cluster.u32 %0, %0, %1;" : "+r"(halo) : "r"(cta - 1));
+            asm("mapa.shared::cluster.u32 %0, %0, %1;" : "+r"(halo_bar) : "r"(cta - 1));
+        }
+        const bool gets = below && strip == M - 1;
+        // a pixel's pass-start state is stored w steps before it enters again: with w steps
+        // to spare over this warp's lead it is fetched one fold ahead, like J and W
+        const bool early = w >= FC + kFxAhead;
+        auto fetch = [&](int c, int pk, FxIn<K>& in) {
+            if (row_ok && (unsigned)c < (unsigned)w) {
+                const int o = (r + c) * P;
+#pragma unroll
+                for (int i = 0; i < 6 * K; ++i) in.j[i] = __ldg(Jr + i * pl + o);
+                const double* wsrc = (pk & kPkCoef) ? wpr : ((pk & kPkTick) ? Wr + K * pl : Wr);
+#pragma unroll
+                for (int k = 0; k < K; ++k) in.w[k] = wsrc[k * pl + o];
+                in.lu = __ldg(lapr + o);
+                in.lv = __ldg(lapr + pl + o);
+            }
+        };
+        auto fetch_state = [&](int c, int pk, long long& su, long long& sv) {
+            su = sv = 0;
+            if (row_ok && (unsigned)c < (unsigned)w && !(pk & kPkZero)) {
+                const int o = (r + c) * P;
+                su = dur[o];
+                sv = dvr[o];
+            }
+        };
+        FxIn<K> in;
+        long long su = 0, sv = 0;
+        cur.advance(T, w, fj - r);
+        fetch(fj - r - cur.start, cur.pk, in);
+        for (int s = fj; s < nsteps; s += FC) {
+            const int slot = (unsigned)s % S;
+            // the update has finished step s - kFxAhead: the slot is free, and the states stored up to then can be read
+            if (s >= kFxAhead) mbar_wait(empty_bar(strip, slot), ((unsigned)(s - kFxAhead) / S) & 1, dead);
+            const int c = s - r - cur.start, pk = cur.pk;
+            if (!early) fetch_state(c, pk, su, sv);
+            const FxIn<K> now = in;
+            const long long nu = su, nv = sv;
+            cur.advance(T, w, s + FC - r);
+            fetch(s + FC - r - cur.start, cur.pk, in);
+            if (early) fetch_state(s + FC - r - cur.start, cur.pk, su, sv);
+            int4* sl = ring + slot * SR + row;
+            const int2 lu = limbs(nu), lv = limbs(nv);
+            sl[kPS * PL] = make_int4(lu.x, lu.y, lv.x, lv.y);
+            st_async_if(sends, halo + slot * SR * 16, make_int4(lu.x, lu.y, lv.x, lv.y), halo_bar + slot * 8);
+            if (row_ok && (unsigned)c < (unsigned)w)
+                fx_fold<K, ISO>(A, pw, pk, now, nu, nv, wpr + (r + c) * P, pl, sl, PL, q, kmax, bad);
+            __syncwarp();
+            if (lane == 0) {
+                if (gets)
+                    mbar_arrive_expect(full_bar(strip, slot), sizeof(int4));
+                else
+                    mbar_arrive(full_bar(strip, slot));
+            }
+        }
+    } else if (warp == WU) {
+        // ------------------------------------------------------------ wait
+        // What a step needs from other warps and CTAs is awaited here, beside the update of the
+        // step before: the fold's slots and the neighbouring CTAs' edge rows.
+        auto wait_full = [&](int s) {
+            if (s < nsteps)
+                for (int st = 0; st < M; ++st) mbar_wait(full_bar(st, (unsigned)s % S), ((unsigned)s / S) & 1, dead);
+        };
+        wait_full(0);
+        wait_full(1);
+        asm volatile("bar.sync 1, %0;" ::"n"(32 * (WU + 1)) : "memory");
+        for (int s = 0; s < nsteps; ++s) {
+            wait_full(s + 2);
+            if (nc > 1 && s + 1 < nsteps) {
+                mbar_wait(edge_bar(s & 1), ((unsigned)s >> 1) & 1, dead);
+                if (lane == 0) mbar_expect(edge_bar(s & 1), edge_bytes);
+            }
+            asm volatile("bar.sync 1, %0;" ::"n"(32 * (WU + 1)) : "memory");
+            // step s is done by every iteration: the slot of the pixel that entered 2 (G - 1) steps ago is free
+            if (lane < M) mbar_arrive(empty_bar(lane, (unsigned)(s + kFxAhead) % S));
+        }
+    } else {
+        // ---------------------------------------------------------- update
+        constexpr int NG = (G + NU - 1) / NU;  // iterations of this warp: g0, g0 + NU, ...
+        const int g0 = warp / M;
+        const int oh = A.oh, ol = A.ol;
+        const bool first_row = r == 0, last_row = r == h - 1;
+        // edge rows to the neighbouring CTAs: the last row's values go below, the first row's above
+        const bool send_dn = below && row == ROWS - 1, send_up = above && row == 0;
+        unsigned ebuf = smem_addr(bufs + (send_dn ? 0 : ROWS + 1)), ebar = edge_bar(0);
+        if (send_dn || send_up) {
+            const int peer = send_dn ? cta + 1 : cta - 1;
+            asm("mapa.shared::cluster.u32 %0, %0, %1;" : "+r"(ebuf) : "r"(peer));
+            asm("mapa.shared::cluster.u32 %0, %0, %1;" : "+r"(ebar) : "r"(peer));
+        }
+        const int limw = 1 << (lim - 32);
+        int4 lf[NG], own[NG];  // the values left of the current pixel, and the pixel's own
+        int4 C[NG], Ac[NG], Pc[NG], Kc[NG], D[NG];  // coefficients of the current step
+        int4* myring = ring + row;
+        int co[NG];            // ring offset of iteration i's pixel
+#pragma unroll
+        for (int i = 0; i < NG; ++i) {
+            lf[i] = own[i] = make_int4(0, 0, 0, 0);
+            co[i] = (unsigned)(-2 * (g0 + i * NU)) % S * SR;
+        }
+        auto next_slot = [&](int o) { return o == (S - 1) * SR ? 0 : o + SR; };
+        auto fetch_coef = [&]() {
+#pragma unroll
+            for (int i = 0; i < NG; ++i) {
+                const int4* rg = myring + co[i];
+                C[i] = rg[kPC * PL];
+                Ac[i] = rg[kPA * PL];
+                Pc[i] = rg[kPP * PL];
+                Kc[i] = rg[kPK * PL];
+                if (!ISO) D[i] = rg[kPD * PL];
+                co[i] = next_slot(co[i]);
+            }
+        };
+        int so = 0, so1 = SR;           // state slots of steps s and s + 1
+        int b0 = 0, b1 = 2 * BUF, b2 = BUF;  // the buffers of steps s, s - 1, s - 2
+        asm volatile("bar.sync 1, %0;" ::"n"(32 * (WU + 1)) : "memory");
+        if (g0 == 0) own[0] = myring[kPS * PL];
+        fetch_coef();
+        for (int s = 0; s < nsteps; ++s) {
+            cur.advance(T, w, s - r);
+            const int Gp = cur.pk >> 8;
+            const int d0 = s - cur.start;  // the diagonal of iteration 0's pixel
+            const int c0 = d0 - r;
+#pragma unroll
+            for (int i = 0; i < NG; ++i) {
+                const int gi = g0 + i * NU;
+                if (gi >= G) break;
+                const int c = c0 - 2 * gi;
+                // border copies: the neighbour outside is the pixel's own value before the update
+                const int4* base = gi == 0 ? myring + kPS * PL : bufs + (gi - 1) * 3 * BUF + row + 1;
+                const int4* before = base + (gi == 0 ? so : b2);
+                const int4* prev = base + (gi == 0 ? so1 : b1);
+                int4* mybuf = bufs + gi * 3 * BUF + row + 1;
+                const int4 rt = *(c == w - 1 ? before : prev);
+                const int4 dn = *(last_row ? before : prev + 1);
+                const int4 up = *(first_row ? before : mybuf + b1 - 1);
+                const int4 ow = own[i];
+                const int4 le = sel4(c == 0, ow, lf[i]);
+                const int4 Ci = C[i], Ai = Ac[i], Pi = Pc[i], Ki = Kc[i], Di = ISO ? make_int4(0, 0, 0, 0) : D[i];
+                int4 su, sv;  // sums over the neighbours: (h, l) of the rows', then of the columns'
+                if (ISO) {
+                    su = make_int4(up.x + dn.x + le.x + rt.x, up.y + dn.y + le.y + rt.y, 0, 0);
+                    sv = make_int4(up.z + dn.z + le.z + rt.z, up.w + dn.w + le.w + rt.w, 0, 0);
+                } else {
+                    su = make_int4(up.x + dn.x, up.y + dn.y, le.x + rt.x, le.y + rt.y);
+                    sv = make_int4(up.z + dn.z, up.w + dn.w, le.z + rt.z, le.w + rt.w);
+                }
+                const long long pu = ((long long)Pi.y << 32) | (unsigned)Pi.x;
+                const long long pv = ((long long)Pi.w << 32) | (unsigned)Pi.z;
+                const long long U = fx_point<ISO>(oh, ol, Ci.x, Ci.y, Di.x, Di.y, Ai.x, Ai.y, Ki.x, Ki.z, pu, ow.x, ow.y, ow.z,
+                                                  ow.w, su.x, su.y, su.z, su.w);
+                int4 n;
+                n.x = (int)(U >> 30);
+                n.y = (int)((unsigned)U & 0x3fffffffu) - (1 << 29);
+                const long long V = fx_point<ISO>(oh, ol, Ci.z, Ci.w, Di.z, Di.w, Ai.z, Ai.w, Ki.y, Ki.w, pv, ow.z, ow.w, n.x,
+                                                  n.y, sv.x, sv.y, sv.z, sv.w);
+                n.z = (int)(V >> 30);
+                n.w = (int)((unsigned)V & 0x3fffffffu) - (1 << 29);
+                mybuf[b0] = n;
+                st_async_if((send_dn || (send_up && gi + 1 < G)) && s + 1 < nsteps, ebuf + (gi * 3 * BUF + b0) * 16, n,
+                            ebar + (s & 1) * 8);
+                const int uh = (int)(U >> 32), vh = (int)(V >> 32);
+                const bool valid = gi < Gp && row_ok && (unsigned)c < (unsigned)w;
+                top |= valid ? (uh ^ (uh >> 31)) | (vh ^ (vh >> 31)) : 0;
+                const bool last = valid && gi == Gp - 1;
+                long long* ou = reinterpret_cast<long long*>(A.du) + f * A.st_fs + r + (long long)(d0 - 2 * gi) * P;
+                long long* ov = reinterpret_cast<long long*>(A.dv) + f * A.st_fs + r + (long long)(d0 - 2 * gi) * P;
+                st_global_if(last, ou, U - (1 << 29));
+                st_global_if(last, ov, V - (1 << 29));
+                if (A.ring && last && cur.p == T.n - 1) fx_ring(odu, odv, A.out_rs, r, c, h, w, ow, q);
+                lf[i] = n;
+                own[i] = rt;
+            }
+            fetch_coef();
+            asm volatile("bar.sync 1, %0;" ::"n"(32 * (WU + 1)) : "memory");
+            so = so1;
+            so1 = next_slot(so1);
+            const int b = b2;
+            b2 = b1;
+            b1 = b0;
+            b0 = b;
+        }
+        bad |= top >= limw;
+    }
+    // the level's result, by all warps: states as float64, row-major
+    __syncthreads();
+    if (row_ok && warp != WU) {
+        const long long* sdu = A.du + f * A.st_fs + r;
+        const long long* sdv = A.dv + f * A.st_fs + r;
+        for (int c = warp < WU ? warp / M : NU + (warp - WU - 1) / M; c < w; c += NU + FC) {
+            const long long nu = sdu[(r + c) * P], nv = sdv[(r + c) * P];
+            const long long mag = (nu < 0 ? ~nu : nu) | (nv < 0 ? ~nv : nv);
+            big |= mag >= (1ll << 42);
+            nonzero |= (nu | nv) != 0;
+            const long long o = (long long)r * A.out_rs + c;
+            odu[o] = fx_to_double(nu, q);
+            odv[o] = fx_to_double(nv, q);
+        }
+    }
+    const int m = (bad || dead ? 1 : 0) | (big ? 2 : 0) | (nonzero ? 4 : 0);
+    const int mm = __reduce_or_sync(~0u, m);
+    const int tt = __reduce_or_sync(~0u, top);
+    int* marks = A.second ? A.fs.marks2 : A.fs.marks;
+    int* out_reach = A.second ? A.fs.reach2 : A.fs.reach;
+    if (lane == 0 && mm) atomicOr(marks + f, mm);
+    // the largest |du|, |dv| of any iteration is below 2^(64 - clz(tt) - q) px; floor at 0
+    if (lane == 0 && warp < WU) atomicMax(out_reach + f, max(0, 64 - __clz(tt) - q));
+    sync_all();  // no CTA leaves while another may still write into its shared memory
+}
+
+template <int K, bool ISO, int M, int NU, int FC>
+cudaError_t run_fx(const FxArgs& A, const FxTable& T, int n_frames, cudaStream_t st)
+{
+    constexpr size_t smem = FxSmem<M, ISO>::bytes_all;
+    auto kern = k_sor_fx<K, ISO, M, NU, FC>;
+    cudaError_t e = ensure_max_dyn_smem((const void*)kern, (int)smem);
+    if (e != cudaSuccess) return e;
+    if (A.nc > 8 && (e = ensure_nonportable_clusters((const void*)kern)) != cudaSuccess) return e;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(n_frames * A.nc));
+    cfg.blockDim = dim3(32 * (M * (NU + FC) + 1));
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = (unsigned)A.nc;
+    at[0].val.clusterDim.y = 1;
+    at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = A.nc > 1 ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, kern, A, T);
+}
+
+template <int K, bool ISO>
+cudaError_t run_fx_m(const FxArgs& A, const FxTable& T, int m, int n_frames, cudaStream_t st)
+{
+    if (m == 1) return run_fx<K, ISO, 1, 5, 8>(A, T, n_frames, st);
+    if (m == 2) return run_fx<K, ISO, 2, 1, 4>(A, T, n_frames, st);
+    return run_fx<K, ISO, 4, 1, 2>(A, T, n_frames, st);
+}
+
+template <int K>
+cudaError_t run_fx_k(const FxArgs& A, const FxTable& T, int m, int n_frames, cudaStream_t st)
+{
+    return A.ca == A.cb ? run_fx_m<K, true>(A, T, m, n_frames, st) : run_fx_m<K, false>(A, T, m, n_frames, st);
+}
+
+}  // namespace
+
+size_t fx_pow_bytes() { return kFxTabBytes; }
+
+bool make_fx_pow(double b, void* host, FxPow* P)
+{
+    if (!(b >= -1.0 && b <= 1.0)) return false;
+    longlong2* A = static_cast<longlong2*>(host);
+    long long* B = reinterpret_cast<long long*>(A + 64);
+    unsigned* R = reinterpret_cast<unsigned*>(B + 256);
+    const long double lb = b;
+    for (int e = 0; e < 64; ++e) {
+        const long double y = (e + kPowEMin) * lb;
+        const long double fl = std::floor(y);
+        A[e].x = (long long)std::rint(exp2l(y - fl) * 2305843009213693952.0L);  // 2^61
+        A[e].y = (long long)fl;
+    }
+    for (int j = 0; j < 256; ++j) {
+        R[j] = (unsigned)std::rint(65536.0 / (1.0 + (2.0 * j + 1.0) / 512.0));
+        B[j] = (long long)std::rint(exp2l(lb * (16.0L - log2l((long double)R[j]))) * 1152921504606846976.0L);  // 2^60
+    }
+    long double c = lb, cn[7];
+    for (int n = 2; n <= 6; ++n) cn[n] = c = c * (lb - (n - 1)) / n;
+    P->c1 = (long long)std::rint(lb * 1152921504606846976.0L);
+    P->c2 = (long long)std::rint(cn[2] * 1152921504606846976.0L);
+    P->c3 = (int)std::rint(cn[3] * 1073741824.0L);
+    P->c4 = (int)std::rint(cn[4] * 1073741824.0L);
+    P->c5 = (int)std::rint(cn[5] * 1073741824.0L);
+    P->c6 = (int)std::rint(cn[6] * 1073741824.0L);
+    return true;
+}
+
+void place_fx_pow(void* dev, FxPow* P) { place_fx(dev, P); }
+
+bool sor_fx_supports(int K, const DiagGeom& g, int n_passes, double omega)
+{
+    // w: a pixel's state has to be stored before the fold that reads it, up to kFxAhead steps
+    // ahead of the update; omega in [1, 2) keeps |1 - omega| < 1 and c < 1/2
+    return K >= 1 && K <= 4 && (g.P & 31) == 0 && g.w >= kFxAhead + 1 && n_passes >= 1 && n_passes <= kMaxChain &&
+           g.P / 32 <= kFxMaxStrips && omega >= 1.0 && omega < 2.0 &&
+           (long long)g.D * g.P * (6 * K + 2) < 0x7fffffffLL;
+}
+
+cudaError_t launch_sor_fx(const double* J, long long J_fs, const double* W, long long W_fs, const double* lap,
+                          long long lap_fs, double* wp, long long wp_fs, double* du, double* dv, long long st_fs,
+                          int n_frames, int K, DiagGeom g, const ChainPass* passes, int n_passes, double wx, double wy,
+                          double omega, cudaStream_t st, double* out_du, double* out_dv, long long out_fs, int out_rs,
+                          int ring, int rows, const FxPow* pows, int reach, int second, const FxState& fs)
+{
+    if (!sor_fx_supports(K, g, n_passes, omega) || n_frames < 1 || !out_du || !out_dv || !fs.marks)
+        return cudaErrorInvalidValue;
+    const int strips = g.P / 32;
+    int m = rows >= 128 ? 4 : (rows >= 64 ? 2 : 1);
+    while ((strips + m - 1) / m > kFxMaxCluster) m *= 2;
+    FxTable T;
+    T.n = n_passes;
+    for (int p = 0; p < n_passes; ++p) {
+        const ChainPass& c = passes[p];
+        if (c.G < 1 || c.G > kGMax || c.mode < -1 || c.mode > 3) return cudaErrorInvalidValue;
+        const bool coef_in = c.mode < 0, store = c.mode >= 0 && c.store_coef;
+        T.pk[p] = (c.G << 8) | (store ? kPkStore : 0) | (coef_in ? kPkCoef : 0) |
+                  (!coef_in && (c.mode & 2) ? kPkTick : 0) | (!coef_in && (c.mode & 1) ? kPkZero : 0);
+    }
+    for (int p = n_passes; p < kMaxChain; ++p) T.pk[p] = 1 << 8;
+    FxArgs A;
+    A.J = J;
+    A.J_fs = J_fs;
+    A.W = W;
+    A.W_fs = W_fs;
+    A.lap = lap;
+    A.lap_fs = lap_fs;
+    A.wp = wp;
+    A.wp_fs = wp_fs;
+    A.du = reinterpret_cast<long long*>(du);
+    A.dv = reinterpret_cast<long long*>(dv);
+    A.st_fs = st_fs;
+    A.out_du = out_du;
+    A.out_dv = out_dv;
+    A.out_fs = out_fs;
+    A.out_rs = out_rs;
+    A.ring = ring;
+    A.g = g;
+    // the row neighbours (above and below) carry the y weight
+    const double wsum = ((wx + wx) + wy) + wy, two61 = 2305843009213693952.0;
+    A.lap_scale = 2.0 / wsum;
+    A.half_omega = (long long)std::rint(0.5 * omega * two61);
+    A.ca = (long long)std::rint(2.0 * wy / wsum * two61);
+    A.cb = (long long)std::rint(2.0 * wx / wsum * two61);
+    // 1 - omega as float64 holds it, in limbs
+    const long long om = (long long)std::rint((1.0 - omega) * 1152921504606846976.0);
+    A.oh = (int)((om + (1 << 29)) >> 30);
+    A.ol = (int)(om - ((long long)A.oh << 30));
+    for (int k = 0; k < 4; ++k) A.pw[k] = k < K ? pows[k] : FxPow();
+    A.lim = kFxLim;
+    A.kmax = kFxKmax;
+    A.reach = reach;
+    A.second = second;
+    A.fs = fs;
+    A.nc = (strips + m - 1) / m;
+    switch (K) {
+        case 1: return run_fx_k<1>(A, T, m, n_frames, st);
+        case 2: return run_fx_k<2>(A, T, m, n_frames, st);
+        case 3: return run_fx_k<3>(A, T, m, n_frames, st);
+        default: return run_fx_k<4>(A, T, m, n_frames, st);
+    }
+}
+
+}  // namespace frg
