@@ -278,9 +278,7 @@ struct LevelPlan {
     double* ref64 = nullptr;    // (K, h, w) reference level in float64, for its tensor
     double* refd64 = nullptr;   // (4, K, h, w) its derivatives gx1, gy1, fxx1, fyy1 (launch_x_ref_derivs)
     bool chain64 = false;       // fp64 plan: this level runs the float64 chained SOR
-    int rows64 = 0;             // its rows per CTA strip (64, 128, 256); 0: chosen per call from the batch size
-    bool fx = false;            // its updates run in fixed point (launch_sor_fx)
-    double* wdiagfx = nullptr;  // wdiag64 divided by 2 (wx + wy), for that form
+    int rows64 = 0;             // its rows per CTA (64, 128, 256) as asked for; 0: 32, or what the level's height needs
     int sor_G = 0;        // fused SOR iterations per pass (0: the most the ring allows)
     int sor_threads = 0;  // fused SOR threads per CTA (0: the level's rows, P)
     int sor_variant = 0;  // fused SOR kernel: 0 diagonal ring in shared memory, 1 rows with the state in registers
@@ -388,8 +386,6 @@ struct frg_plan {
     double* xacc[2] = {nullptr, nullptr};  // (T, 2, h*w)
     double a_data64[kMaxK] = {0};
     PowTab64 pow64[kMaxK];  // the float64 chained SOR's power table per channel (shared by equal exponents)
-    FxPow fxpow[kMaxK];     // the same for its fixed-point form
-    int* marks = nullptr;   // (levels, 4, T): the fixed-point form's per-frame words (FxState)
     // final cubic upsampling when min_level > 0 (tables per output column / row)
     int32_t* up_sx = nullptr;
     float* up_wx = nullptr;
@@ -401,7 +397,6 @@ struct frg_plan {
     // FP64 plans with a_smooth = 1, gradient or gray-value constancy and no GNC: the
     // levels the float64 chained SOR serves run it on diagonal-major float64 buffers
     bool dpath = false;
-    int n_sms = 0;            // multiprocessors of the plan's device
     double* dJ = nullptr;     // (T, 6, K, D*P)
     double* dlap = nullptr;   // (T, 2, D*P)
     double* dcoef = nullptr;  // (T, 5, D*P)
@@ -453,28 +448,6 @@ int make_pow_tables(frg_plan* pl, int channels)
     return FRG_OK;
 }
 
-// The fixed-point SOR's power tables, one per distinct exponent; only for exponents it serves.
-int make_fx_tables(frg_plan* pl, int channels)
-{
-    std::vector<char> tab(fx_pow_bytes());
-    for (int k = 0; k < channels; ++k) {
-        const double b = pl->a_data64[k] - 1.0;
-        int same = -1;
-        for (int q = 0; q < k && same < 0; ++q)
-            if (pl->a_data64[q] - 1.0 == b) same = q;
-        if (same >= 0) {
-            pl->fxpow[k] = pl->fxpow[same];
-            continue;
-        }
-        if (!make_fx_pow(b, tab.data(), &pl->fxpow[k])) return fail(FRG_EINVAL, "a_data - 1 must lie in [-1, 1]");
-        char* dt = nullptr;
-        if (int rc = dev_alloc(pl, &dt, tab.size())) return rc;
-        FRG_CUDA(cudaMemcpy(dt, tab.data(), tab.size(), cudaMemcpyHostToDevice));
-        place_fx_pow(dt, &pl->fxpow[k]);
-    }
-    return FRG_OK;
-}
-
 // Whether the fixed-point SOR serves every channel's power.
 bool fx_exponents_ok(int K, const double* a_data)
 {
@@ -483,25 +456,9 @@ bool fx_exponents_ok(int K, const double* a_data)
     return true;
 }
 
-// The fixed-point form's first guess of a level's |du|, |dv|, for levels without a
-// coarser one to go by: below 2^4 px (the second launch reaches 2^10).
-constexpr int kFxReachFirst = 4;
-
-// Per-frame words of one level, 4 n_frames from `base`; prev: the same of the coarser level.
-FxState fx_state(int* base, int* prev, int n)
-{
-    FxState s;
-    s.marks = base;
-    s.marks2 = base + n;
-    s.reach = base + 2 * n;
-    s.reach2 = base + 3 * n;
-    if (prev) {
-        s.prev_marks = prev;
-        s.prev_reach = prev + 2 * n;
-        s.prev_reach2 = prev + 3 * n;
-    }
-    return s;
-}
+// The fixed-point form's first guess of a single level's |du|, |dv|: below 2^4 px
+// (its second launch reaches 2^7).
+constexpr int kFxReach = 4;
 
 int upload_tables(frg_plan* pl, const HostTables& t, int n_out_x, const HostTables& ty, int n_out_y,
                   DevTables* d)
@@ -748,13 +705,6 @@ int frg_plan_create(const frg_params* params, int height, int width, int channel
     pl->dpath = pl->xpath && params->a_smooth == 1.0 && params->gnc_stages == 0;
     const int n_passes = fill_passes(params->iterations, params->update_lag, kGMax, nullptr, 0);
     size_t max_dp64 = 0;
-    {
-        int dev = 0;
-        if (cudaGetDevice(&dev) != cudaSuccess ||
-            cudaDeviceGetAttribute(&pl->n_sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
-            pl->n_sms = 1;
-    }
-
     // schedule: core/optical_flow.py:494-518
     const int m = height, n = width;
     const double eta = params->eta;
@@ -815,11 +765,6 @@ int frg_plan_create(const frg_params* params, int height, int width, int channel
                 return rc;
             }
             max_dp64 = std::max(max_dp64, (size_t)L.g.D * L.g.P);
-            L.fx = sor_fx_supports(channels, L.g, n_passes, params->omega) && fx_exponents_ok(channels, params->a_data);
-            if (L.fx && (rc = dev_alloc(pl, &L.wdiagfx, (size_t)2 * channels * L.g.D * L.g.P))) {
-                frg_plan_destroy(pl);
-                return rc;
-            }
         }
         max_dp = std::max(max_dp, (size_t)L.g.D * L.g.P);
         max_hw = std::max(max_hw, (size_t)L.h * L.w);
@@ -881,10 +826,7 @@ int frg_plan_create(const frg_params* params, int height, int width, int channel
             return rc;
         }
         for (int k = 0; k < channels; ++k) pl->a_data64[k] = params->a_data[k];
-        bool any_fx = false;
-        for (const LevelPlan& L : pl->levels) any_fx = any_fx || L.fx;
-        if ((max_dp64 > 0 && (rc = make_pow_tables(pl, channels))) ||
-            (any_fx && ((rc = make_fx_tables(pl, channels)) || (rc = dev_alloc(pl, &pl->marks, pl->levels.size() * 4 * T))))) {
+        if (max_dp64 > 0 && (rc = make_pow_tables(pl, channels))) {
             frg_plan_destroy(pl);
             return rc;
         }
@@ -1091,11 +1033,6 @@ int frg_set_reference(frg_plan* pl, const float* fixed, const float* weight, voi
                                            L.img.wy, L.img.P, st));
             if (L.chain64) {
                 FRG_LAUNCH(launch_x_pad_to_diag(L.wpad64, K, L.h, L.w, L.g, L.wdiag64, st, pl->a_data64));
-                if (L.fx) {
-                    const double wx = L.alpha_x / (L.h_col * L.h_col), wy = L.alpha_y / (L.h_row * L.h_row);
-                    FRG_LAUNCH(launch_x_pad_to_diag(L.wpad64, K, L.h, L.w, L.g, L.wdiagfx, st, pl->a_data64,
-                                                    1.0 / (((wx + wx) + wy) + wy)));
-                }
                 FRG_LAUNCH(launch_x_to_double(L.ref, (long long)K * hw, L.ref64, st));
                 FRG_LAUNCH(launch_x_ref_derivs(L.ref64, K, L.h, L.w, L.h_row, L.h_col, L.refd64, st));
             }
@@ -1330,8 +1267,6 @@ int run_xpath(frg_plan* pl, int T, const float* moving, const float* uv_init, do
     const long long fsz = (long long)H * W * K;
     int cur = 0;
     const LevelPlan* prev = nullptr;
-    if (pl->marks && !pl->solver_fn)
-        FRG_CUDA(cudaMemsetAsync(pl->marks, 0, sizeof(int) * pl->levels.size() * 4 * pl->max_T, st));
     for (size_t li = 0; li < pl->levels.size(); ++li) {
         const LevelPlan& L = pl->levels[li];
         const int h = L.h, w = L.w;
@@ -1397,20 +1332,10 @@ int run_xpath(frg_plan* pl, int T, const float* moving, const float* uv_init, do
                 int rc = record_event(&pl->prof, st);
                 if (rc) return rc;
             }
-            const int rows = L.rows64 ? L.rows64 : sor_chain64_default_rows(L.g, T, pl->n_sms);
-            // the fixed-point form first, in two formats; the float64 one then computes the frames both marked
-            const bool coarser = L.fx && prev && prev->fx;
-            int* words = L.fx ? pl->marks + li * 4 * pl->max_T : nullptr;
-            const FxState fs = fx_state(words, coarser ? words - 4 * pl->max_T : nullptr, pl->max_T);
-            for (int second = 0; L.fx && second < 2; ++second)
-                FRG_LAUNCH(launch_sor_fx(pl->dJ, 6LL * K * dp, L.wdiagfx, 0, pl->dlap, 2 * dp, pl->dcoef, 5 * dp, pl->ddu,
-                                         pl->ddv, dp, T, K, L.g, cp, np, wx, wy, pl->p.omega, st,
-                                         pl->xdu + (w + 2) + 1, pl->xdv + (w + 2) + 1, mn, w + 2, 0, L.rows64,
-                                         pl->fxpow, coarser ? -1 : kFxReachFirst, second, fs));
             FRG_LAUNCH(launch_sor_chain64(pl->dJ, 6LL * K * dp, L.wdiag64, 0, pl->dlap, 2 * dp, pl->dcoef, 5 * dp,
                                           pl->ddu, pl->ddv, dp, T, K, L.g, cp, np, pl->a_data64, wx, wy, pl->p.omega,
-                                          st, pl->xdu + (w + 2) + 1, pl->xdv + (w + 2) + 1, mn, w + 2, rows,
-                                          pl->pow64, L.fx ? fs.marks2 : nullptr));
+                                          st, pl->xdu + (w + 2) + 1, pl->xdv + (w + 2) + 1, mn, w + 2, L.rows64,
+                                          pl->pow64));
             if (timed) {
                 int rc = record_event(&pl->prof, st);
                 if (rc) return rc;
@@ -1551,8 +1476,10 @@ int frg_level_solve(int m, int n, int K, const float* J, const float* weight, co
 namespace {
 
 // compute_flow through the chained SOR: a_smooth = 1, no GNC, the levels
-// launch_sor_chain64 serves.  Same form as a pyramid level's solve; the level
-// may hold the whole displacement.
+// launch_sor_chain64 serves.  Fixed point first (one level alone may differ from
+// float64 in the last bits), float64 for what lies outside its ranges.  410 x 410 x
+// 2, 50 iterations, host arrays in and out: 7.9 ms; launch_x_sor, which takes every
+// other level, 540 ms.
 int seam_chain64(int h, int w, int K, const DiagGeom& g, const double* J, const double* weight, const double* u,
                  const double* v, double alpha_x, double alpha_y, const Pass* ps, int np, const double* a_data,
                  double hx, double hy, double omega, double* du, double* dv, cudaStream_t st)
@@ -1562,14 +1489,11 @@ int seam_chain64(int h, int w, int K, const DiagGeom& g, const double* J, const 
     ChainPass cp[kMaxChain];
     chain_passes(ps, np, cp);
     const bool fx = sor_fx_supports(K, g, np, omega) && fx_exponents_ok(K, a_data);
-    int dev = 0, n_sms = 1;
-    FRG_CUDA(cudaGetDevice(&dev));
-    FRG_CUDA(cudaDeviceGetAttribute(&n_sms, cudaDevAttrMultiProcessorCount, dev));
     const long long dp = (long long)g.D * g.P;
     const size_t tab = fx_pow_bytes();
     const size_t doubles = (size_t)(6 * K + 4 * K + 2 + 5 + 2) * dp;
     char* scratch = nullptr;
-    FRG_CUDA(cudaMallocAsync((void**)&scratch, doubles * sizeof(double) + K * tab + 4 * sizeof(int), st));
+    FRG_CUDA(cudaMallocAsync((void**)&scratch, doubles * sizeof(double) + K * tab + 2 * sizeof(int), st));
     double* Jd = (double*)scratch;
     double* Wd = Jd + 6LL * K * dp;
     double* Wfx = Wd + 2LL * K * dp;
@@ -1579,7 +1503,6 @@ int seam_chain64(int h, int w, int K, const DiagGeom& g, const double* J, const 
     double* sdv = sdu + dp;
     char* tabs = (char*)(sdv + dp);
     int* marks = (int*)(tabs + K * tab);
-    const FxState fs = fx_state(marks, nullptr, 1);
     auto run = [&]() -> int {
         FRG_LAUNCH(launch_x_seam_to_diag(J, weight, u, v, K, h, w, g, wx, wy, a_data, Jd, Wd, Wfx, lap, st));
         double* odu = du + (w + 2) + 1;
@@ -1593,14 +1516,14 @@ int seam_chain64(int h, int w, int K, const DiagGeom& g, const double* J, const 
             }
             // from pageable memory: returns once the tables are staged
             FRG_CUDA(cudaMemcpyAsync(tabs, host.data(), host.size(), cudaMemcpyHostToDevice, st));
-            FRG_CUDA(cudaMemsetAsync(marks, 0, 4 * sizeof(int), st));
+            FRG_CUDA(cudaMemsetAsync(marks, 0, 2 * sizeof(int), st));
             for (int second = 0; second < 2; ++second)
                 FRG_LAUNCH(launch_sor_fx(Jd, 0, Wfx, 0, lap, 0, coef, 0, sdu, sdv, 0, 1, K, g, cp, np, wx, wy, omega, st,
-                                         odu, odv, 0, w + 2, 1, 0, pows, kFxReachFirst, second, fs));
+                                         odu, odv, 0, w + 2, 1, pows, kFxReach, second, marks, marks + 1));
         }
         FRG_LAUNCH(launch_sor_chain64(Jd, 0, Wd, 0, lap, 0, coef, 0, sdu, sdv, 0, 1, K, g, cp, np, a_data, wx, wy, omega,
-                                      st, odu, odv, 0, w + 2, sor_chain64_default_rows(g, 1, n_sms), nullptr,
-                                      fx ? fs.marks2 : nullptr, 1));
+                                      st, odu, odv, 0, w + 2, 0, nullptr,
+                                      fx ? marks + 1 : nullptr, 1));
         return FRG_OK;
     };
     const int rc = run();
@@ -1631,7 +1554,10 @@ int frg_level_solve_f64(int m, int n, int K, const double* J, const double* weig
     if (!smooth && gnc_beta < 0.0) {
         Pass ps[kMaxChain];
         const int np = fill_passes(iterations, update_lag, kGMax, ps, kMaxChain);
-        if (sor_chain64_supports(K, g, np))
+        // not while the stream is captured: the chained form uploads tables from the call's own memory
+        cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+        FRG_CUDA(cudaStreamIsCapturing(st, &cap));
+        if (cap == cudaStreamCaptureStatusNone && sor_chain64_supports(K, g, np))
             return seam_chain64(h, w, K, g, J, weight, u, v, alpha_x, alpha_y, ps, np, a_data, hx, hy, omega, du, dv, st);
     }
     double* scratch = nullptr;

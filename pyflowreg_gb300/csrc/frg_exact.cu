@@ -1031,7 +1031,7 @@ struct ChannelScale {
 };
 
 __global__ void kx_pad_to_diag(const double* __restrict__ src, int K, int h, int w, DiagGeom g, double* __restrict__ dst,
-                               ChannelScale sc, int scaled, double common)
+                               ChannelScale sc, int scaled)
 {
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
     const int r = blockIdx.y;
@@ -1039,20 +1039,20 @@ __global__ void kx_pad_to_diag(const double* __restrict__ src, int K, int h, int
     if (c >= w || k >= K) return;
     const long long n = w + 2, mn = (long long)(h + 2) * n;
     const long long plane = (long long)g.D * g.P, di = diag_index(g, r, c);
-    const double v = dmul(src[k * mn + (long long)(r + 1) * n + c + 1], common);
+    const double v = src[k * mn + (long long)(r + 1) * n + c + 1];
     dst[k * plane + di] = v;
     if (scaled) dst[(K + k) * plane + di] = dmul(v, sc.s[k]);
 }
 
 cudaError_t launch_x_pad_to_diag(const double* src, int K, int h, int w, DiagGeom g, double* dst, cudaStream_t st,
-                                 const double* scale, double common)
+                                 const double* scale)
 {
     if (K < 1 || K > kMaxK) return cudaErrorInvalidValue;
     ChannelScale sc = {};
     if (scale)
         for (int k = 0; k < K; ++k) sc.s[k] = scale[k];
     dim3 blk(128), grd((w + 127) / 128, h, K);
-    kx_pad_to_diag<<<grd, blk, 0, st>>>(src, K, h, w, g, dst, sc, scale ? 1 : 0, common);
+    kx_pad_to_diag<<<grd, blk, 0, st>>>(src, K, h, w, g, dst, sc, scale ? 1 : 0);
     return cudaGetLastError();
 }
 

@@ -135,20 +135,19 @@ struct PowTab64 {
 // Host: fills tab (kPowTabN entries) and the series constants of *pt for
 // exponent b (pt->t untouched); false, with nothing written, when |b| > 1.
 bool make_pow_table(double b, double2* tab, PowTab64* pt);
-// The chained SOR in float64 (frg_sor64.cu, k_sor_chain64): the schedule of
+// The chained SOR in float64 (frg_sor64.cu, k_sor_split64): the schedule of
 // launch_sor_chain with float64 state, coefficients and arithmetic (the parity
 // precision).  J [6][K][D*P] (J11, J22, J33 + 1e-5, 2 J12, 2 J13, 2 J23), W
 // [2][K][D*P] (W, then W * a_data), lap [2][D*P], coef [5][D*P] and the state
 // du, dv [D*P] are diagonal-major doubles; the final pass writes du, dv
-// at out + r * out_rs + c.  Levels of at most 2048 (padded) rows (over 256 as
-// clusters of row strips), K <= 4, w >= 3, at most kMaxChain passes of G <= kGMax.
-// rows: the most rows per CTA (64, 128 or 256; 0 = 256), the level split into at
-// most 8 strips; every split gives the same bits.  pows: the power table of
-// each channel's exponent a_data[k] - 1 (null, or a null table: the general
+// at out + r * out_rs + c.  Levels of at most 2048 (padded) rows in clusters of at
+// most 16 CTAs, K <= 4, w >= 3, at most kMaxChain passes of G <= kGMax.  rows:
+// rows per CTA (0: 32, 64 over 512 rows, 128 over 1024; 64, 128 and 256 ask for at
+// least 64, 128 and 128); every split gives the same bits.  pows: the power table
+// of each channel's exponent a_data[k] - 1 (null, or a null table: the general
 // power).
 bool sor_chain64_supports(int K, const DiagGeom& g, int n_passes);
 bool sor_chain64_rows_ok(const DiagGeom& g, int rows);
-int sor_chain64_default_rows(const DiagGeom& g, int n_frames, int n_sms);
 cudaError_t launch_sor_chain64(const double* J, long long J_fs, const double* W, long long W_fs, const double* lap,
                                long long lap_fs, double* coef, long long coef_fs, double* du, double* dv,
                                long long st_fs, int n_frames, int K, DiagGeom g, const ChainPass* passes,
@@ -164,11 +163,10 @@ cudaError_t launch_sor_chain64(const double* J, long long J_fs, const double* W,
 // a first launch for all frames, and a second one (second = 1) with a wider
 // number format for the frames the first one marked; a frame that the second
 // one marks too (fx_recompute(marks2[f])) is left to launch_sor_chain64.
-// W: the weights divided by wsum = 2 (wx + wy) (both planes).  wp [K][D*P] (weights times psi of passes that continue a group) and the state
-// du, dv [D*P] are workspaces of 64-bit words.  rows: rows per CTA (32, 64, 128;
-// 0 = 32), the level's strips in clusters of at most 16 CTAs; every split gives
-// the same bits.  reach: 2^reach px bounds the level's |du|, |dv|; -1: taken
-// from the frame's previous level.
+// W: the weights divided by wsum = 2 (wx + wy) (both planes).  wp [K][D*P] (weights
+// times psi of passes that continue a group) and the state du, dv [D*P] are
+// workspaces of 64-bit words.  32 rows per CTA, more where the level would need over
+// 16 CTAs.  reach: 2^reach px bounds the level's |du|, |dv|.
 struct FxPow {
     const longlong2* A = nullptr;     // [64] 2^(e b) = A.x 2^(A.y - 61), e from kPowEMin
     const long long* B = nullptr;     // [256] (2^16 / R)^b, 60 fraction bits
@@ -177,12 +175,6 @@ struct FxPow {
     int c3 = 0, c4 = 0, c5 = 0, c6 = 0;  // 30 fraction bits
 };
 __host__ __device__ inline bool fx_recompute(int mark) { return (mark & 1) || ((mark & 4) && !(mark & 2)); }
-// Per-frame words of a level: marks of both launches (marks2 starts at
-// marks) and the reach each one saw, and the previous level's.
-struct FxState {
-    int *marks = nullptr, *marks2 = nullptr, *reach = nullptr, *reach2 = nullptr;
-    const int *prev_marks = nullptr, *prev_reach = nullptr, *prev_reach2 = nullptr;
-};
 size_t fx_pow_bytes();
 // Host: fills `host` (fx_pow_bytes()) and the constants of *P for exponent b;
 // false when |b| > 1.  place_fx_pow: the table's place on the device.
@@ -193,7 +185,7 @@ cudaError_t launch_sor_fx(const double* J, long long J_fs, const double* W, long
                           long long lap_fs, double* wp, long long wp_fs, double* du, double* dv, long long st_fs,
                           int n_frames, int K, DiagGeom g, const ChainPass* passes, int n_passes, double wx, double wy,
                           double omega, cudaStream_t st, double* out_du, double* out_dv, long long out_fs, int out_rs,
-                          int ring, int rows, const FxPow* pows, int reach, int second, const FxState& fs);
+                          int ring, const FxPow* pows, int reach, int second, int* marks, int* marks2);
 // x^b elementwise by the float64 solver's power (frg_dpow.cuh), with the table
 // path for |b| <= 1; upload_dpow_tables must have run on the current device.
 cudaError_t launch_pow64(long long n, const double* x, double b, double* out, cudaStream_t st);
@@ -264,9 +256,9 @@ cudaError_t launch_x_seam_to_diag(const double* J, const double* wgt, const doub
                                   double* Wfx, double* lap, cudaStream_t st);
 // Padded (K, h + 2, w + 2) float64 planes to diagonal-major (K, D*P) at dst;
 // with scale (K host values), also each plane times scale[k] at dst + K*D*P
-// (the float64 chained SOR's weights W and W * a_data); both times `common`.
+// (the float64 chained SOR's weights W and W * a_data).
 cudaError_t launch_x_pad_to_diag(const double* src, int K, int h, int w, DiagGeom g, double* dst, cudaStream_t st,
-                                 const double* scale = nullptr, double common = 1.0);
+                                 const double* scale = nullptr);
 cudaError_t launch_x_hwk_to_planes(const double* src, int n_arrays, long long mn, int K, double* dst, cudaStream_t st);
 // cv2.resize INTER_CUBIC of planar planes (n_frames * n_planes, ih, iw) to
 // (oh, ow): width pass into tmp, height pass into the strided dst view.

@@ -3,34 +3,42 @@
 // compute_flow (core/level_solver.py:158-369) sweeps columns outer, rows
 // inner, in place, in float64.  Float32 arithmetic moves the flow by up to
 // ~0.7 px against it: the 1/32-pixel warp of the next level turns rounding
-// differences into different samples.  With every solver operation rounded to
-// 44 mantissa bits the flow still moves by 2e-3 px; at 48 bits by 1e-8 px.
-// So the parity path computes in float64, and on GB300, whose float64 pipe
-// issues at about 1/64 of the float32 rate, it is bound by float64
-// instructions: this kernel keeps the instruction count per update at the
-// minimum (14 float64 operations per pixel update, the coefficients folded
-// once per pass) and everything else off the float64 pipe.
+// differences into different samples, and even last-bit differences do so at
+// single pixels of a large batch.  So the pyramid keeps float64 and its
+// operations in one order, and on GB300, where one float64 instruction holds a
+// scheduler's float64 pipe for 64 clocks, it is bound by float64 instructions:
+// 14 per pixel update and about 47 (two channels) per fold of a pixel's
+// coefficients, once per pass of up to five updates.
 //
-// Schedule: that of k_sor_chain (frg_sor.cu).  Row r's local time is
-// tau = s - r; pass p occupies tau in [start_p, start_p + span_p), pixel (r, c)
-// of pipelined iteration gi is updated at tau = start_p + c + 2 gi, and every
-// neighbour value an update reads was produced one step earlier, so it stays
-// in registers (left, right, own) or comes from the neighbouring row through a
-// warp shuffle (up, down) or the two-parity exchange buffer (warp edges).
-// Each pixel's five coefficients (A12, BU, BV, omega/den_u, omega/den_v) are
-// folded once per pass when the pixel enters and wait in a shared-memory ring
-// of 2G - 1 slots until its last update of the pass.
+// Schedule (k_sor_chain's, frg_sor.cu).  Row r's local time is tau = s - r; pass p
+// occupies tau in [start_p, start_p + span_p), pixel (r, c) of pipelined
+// iteration gi is updated at tau = start_p + c + 2 gi, and every neighbour value
+// an update reads was produced one step earlier.
 //
-// One thread per row, at most 256, 128 or 64 rows per CTA (a launch choice:
-// the shorter strips fit three or six CTAs per SM, or spread a single frame
-// over more SMs); taller levels run as a thread-block cluster of row strips
-// whose edge rows exchange their values through distributed shared memory,
-// with a cluster barrier per step.
-#include "frg_internal.h"
+// A step's work is split over specialised warps.  One warp that updates all five
+// iterations of 32 rows and folds the entering pixels issues 117 dependent
+// float64 instructions per step, 7500 clocks, on one of the SM's four pipes.
+// Here every 32 rows have an update warp per iteration (NU = 5) and FC fold
+// warps, which run up to kFoldAhead steps ahead: fold warp j takes steps j, j +
+// FC, ..., and writes each entering pixel's five coefficients (A12, BU, BV,
+// omega/den_u, omega/den_v) and pass-start state into a ring of slots in shared
+// memory, so that all four pipes work on one strip and the folds' loads are off
+// the step.  An iteration writes its new values to a buffer of the last three
+// steps, from which the next iteration reads the right, lower and own values and
+// the row below the upper one; one barrier per step.  One more warp waits for
+// the folds and for the neighbouring CTAs while the others update.  A frame's
+// row strips are CTAs of a cluster and pass their edge rows by st.async with a
+// transaction barrier.  Any split gives the same bits.
+//
+// 512 x 512 x 2, all levels, GB300: one frame 187 -> 37 ms, 24 frames 208 -> 87,
+// 100 frames 423 -> 291, against one warp per 32 rows for everything (its strip
+// heights chosen from the batch size).  What is left is the pipe: 117
+// instructions at 64 to 76 clocks over four pipes, about 2000 clocks of a
+// measured 2300 per step.
 #include "frg_dpow.cuh"
+#include "frg_split.cuh"
 
-#include <cooperative_groups.h>
-
+#include <algorithm>
 #include <cmath>
 #include <cstring>
 #include <mutex>
@@ -141,9 +149,8 @@ cudaError_t launch_pow64(long long n, const double* x, double b, double* out, cu
 
 namespace {
 
-constexpr int kLane64 = 256;       // most rows (threads) per CTA
+constexpr int kLane64 = 256;       // most rows per CTA a caller may ask for
 constexpr int kG64 = kGMax;        // iterations pipelined per pass, as a template maximum
-constexpr int kSmem64 = 232448;    // 227 KB of dynamic shared memory per CTA
 constexpr int kMaxStrips64 = 16;   // cluster size (over 8: the non-portable opt-in)
 constexpr int kPortableStrips = 8;
 
@@ -169,17 +176,11 @@ struct Sor64Args {
     double omega, one_m_omega;
     double a_m1[kMaxK];  // a_data - 1
     PowTab64 pw[kMaxK];  // the power's table per channel (null table: the general power)
-    int nc;              // row strips (CTAs) per frame
+    int nc;              // CTAs per frame
+    int ahead;           // steps a fold may run ahead: at most the columns of a row less one
     const int* marks;    // frames to compute (fx_recompute); null: all
     int ring;            // the final pass also writes the border copies around the output
 };
-
-struct Chain64Table {
-    int n;
-    int pk[kMaxChain];  // G << 8 | store << 3 | coef << 2 | tick << 1 | zero
-};
-
-constexpr int kPkZero = 1, kPkTick = 2, kPkCoef = 4, kPkStore = 8;
 
 // The fold's inputs of one pixel (J, W, lap; or the stored coefficients),
 // loaded at the start of the step whose end folds them: a step of float64
@@ -189,12 +190,6 @@ struct FoldIn64 {
     double j[6 * K];
     double w[K];
     double lu, lv;
-};
-
-// Pass-start state, prefetched two steps ahead: du, dv of pixel (r, c) entering
-// the ring and of pixel (r + 1, c - 1) below its left neighbour.
-struct Pre64 {
-    double du, dv, nu, nv;
 };
 
 struct Coef64 {
@@ -240,11 +235,11 @@ __device__ __forceinline__ double omega_over(double omega, double den)
 // The tensor holds the cross terms doubled (2 J12, 2 J13, 2 J23, exact), as E
 // uses them; the sums over them are then twice the sums above, exactly, and
 // A12 = sum / 2, BU = fma(-1/2, sum, lap_u) give the same bits.
-template <int K, bool CO>
+template <int K>
 __device__ __forceinline__ Coef64 fold64(const Sor64Args& A, int pk, const FoldIn64<K>& r, double du, double dv)
 {
     Coef64 o;
-    if (CO && (pk & kPkCoef)) {
+    if (pk & kPkCoef) {
         o.A12 = r.j[0];
         o.BU = r.j[1];
         o.BV = r.j[2];
@@ -303,250 +298,269 @@ __device__ __forceinline__ double2 sor_point64(double2 c, double2 up, double2 dn
     return make_double2(dun, dvn);
 }
 
-// Shared memory: CA double2[S][NT] (A12, BU) | CB double2[S][NT] (BV, iDu) |
-// CC double[S][NT] (iDv) | X double2[2][NW][2][G] | XE double2[2][2][G].
-size_t chain64_smem(int nt)
-{
-    constexpr int S = 2 * kG64 - 1;
-    return (size_t)S * nt * (2 * sizeof(double2) + sizeof(double)) +
-           (size_t)(2 * (nt / 32) * 2 * kG64 + 2 * 2 * kG64) * sizeof(double2);
-}
-
-// NTM: the most rows (threads) of one CTA, 256, 128 or 64.  The launch bounds
-// ask for 1, 3 or 6 CTAs per SM (at most 255 or 170 registers per thread), so
-// shorter strips keep 12 warps per SM where 256-row CTAs keep 8.
-template <int NT>
-struct StripBounds {
-    static constexpr int blocks = NT >= 256 ? 1 : (NT >= 128 ? 3 : 6);
+// Shared memory of a CTA of M strips of 32 rows: ring double2[3][kRingSlots][32 M + 1]
+// (A12, BU | BV, iDu | state, whose last row is the next strip's first) and
+// double[kRingSlots][32 M + 1] (iDv) | iteration buffers double2[G][3][32 M + 2] |
+// mbarriers: full[M][kRingSlots], empty[M][kRingSlots], edge[2 parities] | a word
+// for waits that ran out.
+template <int M>
+struct Split64Smem {
+    static constexpr int rows = 32 * M;
+    static constexpr int plane = kRingSlots * (rows + 1);
+    static constexpr int buf = rows + 2;
+    static constexpr size_t bytes = ((size_t)3 * plane + (size_t)kGMax * 3 * buf) * sizeof(double2) +
+                                    (size_t)plane * sizeof(double) + (size_t)(2 * M * kRingSlots + 2) * 8 + 16;
 };
 
-template <int K, bool CO, bool CL, int NTM>
-__global__ void __launch_bounds__(NTM, StripBounds<NTM>::blocks) k_sor_chain64(Sor64Args A, Chain64Table T)
+// The chained solver, one step of the wavefront divided among warps (see the
+// file's head).  MB: CTAs per SM that the registers are to allow.
+template <int K, int M, int NU, int FC, int MB>
+__global__ void __launch_bounds__(32 * SplitRoles<M, NU, FC>::warps, MB) k_sor_split64(Sor64Args A, PassTable T)
 {
+    using SM = Split64Smem<M>;
+    using Roles = SplitRoles<M, NU, FC>;
     constexpr int G = kG64;
-    constexpr int S = 2 * G - 1;
+    constexpr int S = kRingSlots;
+    constexpr int ROWS = SM::rows, PL = SM::plane, SR = ROWS + 1, BUF = SM::buf, WU = Roles::WU;
     extern __shared__ __align__(16) double sm64[];
+    double2* ring = reinterpret_cast<double2*>(sm64);  // planes kA, kB, kS
+    constexpr int kA = 0, kB = PL, kS = 2 * PL;
+    double2* bufs = ring + 3 * PL;
+    double* ringd = reinterpret_cast<double*>(bufs + G * 3 * BUF);
+    unsigned long long* bars = reinterpret_cast<unsigned long long*>(ringd + PL);
+    int* gave_up = reinterpret_cast<int*>(bars + 2 * M * S + 2);
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+    const int nc = A.nc;
+    const int cta = nc > 1 ? (int)(blockIdx.x % nc) : 0;
+    const int f = nc > 1 ? (int)(blockIdx.x / nc) : (int)blockIdx.x;
+    if (A.marks && !fx_recompute(A.marks[f])) return;  // the same for every CTA of a cluster
+    const bool update = warp < WU;
+    const int strip = (update ? warp : Roles::fold(warp)) % M;
+    const int row = strip * 32 + lane;  // in the CTA
+    const int r = cta * ROWS + row;     // in the level
     const DiagGeom g = A.g;
     const int P = g.P, h = g.h, w = g.w;
-    const int NT = blockDim.x, t = threadIdx.x, lane = t & 31, warp = t >> 5, NW = NT >> 5;
-    const int nc = CL ? A.nc : 1;
-    const int strip = CL ? (int)(blockIdx.x % nc) : 0;
-    const int f = CL ? (int)(blockIdx.x / nc) : (int)blockIdx.x;
-    const int r = strip * NT + t;  // the level row of this thread
-    if (A.marks && !fx_recompute(A.marks[f])) return;  // the same for every CTA of a cluster
-    double2* CA = reinterpret_cast<double2*>(sm64);
-    double2* CB = CA + S * NT;
-    double* CC = reinterpret_cast<double*>(CB + S * NT);
-    double2* X = reinterpret_cast<double2*>(CC + S * NT);
-    double2* XE = X + 2 * NW * 2 * G;
     const int pl = g.D * P;
-    const double* Jr = A.J + f * A.J_fs + r;
-    const double* Wr = A.W + f * A.W_fs + r;
-    const double* lapr = A.lap + f * A.lap_fs + r;
-    double* coefr = A.coef + f * A.coef_fs + r;
-    double* dur = A.du + f * A.st_fs + r;
-    double* dvr = A.dv + f * A.st_fs + r;
-    double* odu = A.out_du ? A.out_du + f * A.out_fs : nullptr;
-    double* odv = A.out_dv ? A.out_dv + f * A.out_fs : nullptr;
-    const double omm = A.one_m_omega, wa = A.wa, wb = A.wb;
     const bool row_ok = r < h;
-    const bool has_below = r + 1 < h;
-    const int last = T.n - 1;
-    auto span = [&](int pk) {
-        const int G_p = pk >> 8;
-        return w + (G_p > 1 ? 2 * (G_p - 1) : 1);
-    };
-
-    // pass-start state of the pixel entering at column c of a pass with flags pk,
-    // and of the pixel below its left neighbour
-    auto fetch_state = [&](int c, int pk, Pre64& p) {
-        const bool zero = (pk & kPkZero) != 0;
-        const int o = (r + c) * P;
-        if (row_ok && c >= 0 && c < w) {
-            p.du = zero ? 0.0 : dur[o];
-            p.dv = zero ? 0.0 : dvr[o];
-        }
-        if (has_below && c >= 1 && c <= w) {
-            p.nu = zero ? 0.0 : dur[o + 1];
-            p.nv = zero ? 0.0 : dvr[o + 1];
-        }
-    };
-    // fold inputs of the pixel at column c of a pass with flags pk
-    auto fetch_fold = [&](int c, int pk, FoldIn64<K>& f) {
-        const int o = (r + c) * P;
-        if (row_ok && c >= 0 && c < w) {
-            if (CO && (pk & kPkCoef)) {
-#pragma unroll
-                for (int q = 0; q < 5; ++q) f.j[q] = coefr[q * pl + o];
-            } else {
-#pragma unroll
-                for (int q = 0; q < 6 * K; ++q) f.j[q] = Jr[q * pl + o];
-                const double* wsrc = (pk & kPkTick) ? Wr + K * pl : Wr;  // W * a_data on a tick
-#pragma unroll
-                for (int k = 0; k < K; ++k) f.w[k] = wsrc[k * pl + o];
-                f.lu = lapr[o];
-                f.lv = lapr[pl + o];
-            }
-        }
-    };
-    auto fold_into = [&](int c, int pk, const FoldIn64<K>& f, const Pre64& p, int slot) {
-        if (row_ok && c >= 0 && c < w) {
-            const Coef64 cf = fold64<K, CO>(A, pk, f, p.du, p.dv);
-            if (CO && (pk & kPkStore)) {
-                const int o = (r + c) * P;
-                coefr[o] = cf.A12;
-                coefr[pl + o] = cf.BU;
-                coefr[2 * pl + o] = cf.BV;
-                coefr[3 * pl + o] = cf.iDu;
-                coefr[4 * pl + o] = cf.iDv;
-            }
-            CA[slot * NT + t] = make_double2(cf.A12, cf.BU);
-            CB[slot * NT + t] = make_double2(cf.BV, cf.iDu);
-            CC[slot * NT + t] = cf.iDv;
-        }
-    };
-    auto xs = [&](int par, int wp, int dir, int gi) -> double2& { return X[((par * NW + wp) * 2 + dir) * G + gi]; };
-    auto step_barrier = [&]() {
-        if constexpr (CL)
+    const bool above = cta > 0, below = cta + 1 < nc;  // other CTAs of the frame
+    auto full_bar = [&](int st, int slot) { return smem_addr(bars + st * S + slot); };
+    auto empty_bar = [&](int st, int slot) { return smem_addr(bars + M * S + st * S + slot); };
+    auto edge_bar = [&](int par) { return smem_addr(bars + 2 * M * S + par); };
+    // bytes a step's edge rows bring: every iteration's from above, all but the last one's from below
+    const unsigned edge_bytes = (above ? G * sizeof(double2) : 0) + (below ? (G - 1) * sizeof(double2) : 0);
+    if (t == 0) {
+        *gave_up = 0;
+        for (int i = 0; i < 2 * M * S + 2; ++i) mbar_init(smem_addr(bars + i), 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        if (nc > 1)
+            for (int par = 0; par < 2; ++par) mbar_expect(edge_bar(par), edge_bytes);
+    }
+    auto sync_all = [&]() {
+        if (nc > 1)
             cooperative_groups::this_cluster().sync();
         else
             __syncthreads();
     };
-    if constexpr (CL) step_barrier();  // every CTA of the cluster is running before any remote write
+    sync_all();
 
-    int cp = 0, cstart = 0;
-    int pk_cur = T.pk[0];
-    int pk_nxt = last > 0 ? T.pk[1] : 0;
-    int cend = span(pk_cur);
-    Pre64 pre[2];
-    fetch_state(-r, pk_cur, pre[0]);
-    fetch_state(1 - r, pk_cur, pre[1]);
-    {
-        FoldIn64<K> f0;
-        fetch_fold(-r, pk_cur, f0);
-        fold_into(-r, pk_cur, f0, pre[0], 0);
-    }
-    double2 V0[G], V1[G], V2[G];
-#pragma unroll
-    for (int gi = 0; gi < G; ++gi) V0[gi] = V1[gi] = V2[gi] = make_double2(0.0, 0.0);
-
+    double* odu = A.out_du + f * A.out_fs;
+    double* odv = A.out_dv + f * A.out_fs;
     int total = 0;
-    for (int p = 0; p < T.n; ++p) total += span(T.pk[p]);
+    for (int p = 0; p < T.n; ++p) total += pass_span(w, T.pk[p]);
     const int nsteps = total + h - 1;
-    int slot0 = 0;  // s % S
-    for (int s0 = 0; s0 < nsteps; s0 += 2) {
-#pragma unroll
-        for (int q = 0; q < 2; ++q) {
-            const int s = s0 + q;
-            if (s < nsteps) {
-                Pre64& cur = pre[q];      // the pixel entering at step s
-                Pre64& nxt = pre[q ^ 1];  // the pixel entering at step s + 1
-                const int slot1 = slot0 + 1 == S ? 0 : slot0 + 1;
-                const int tau = s - r;
-                if (tau >= cend && cp < last) {
-                    ++cp;
-                    cstart = cend;
-                    pk_cur = pk_nxt;
-                    pk_nxt = cp < last ? T.pk[cp + 1] : 0;
-                    cend = cstart + span(pk_cur);
+    bool dead = false;
+    Cursor cur;
+    cur.init(T, w);
+
+    if (!update && warp != Roles::wait && warp != Roles::idle) {
+        // ------------------------------------------------------------ fold
+        const int fj = Roles::fold(warp) / M;
+        const double* Jr = A.J + f * A.J_fs + r;
+        const double* Wr = A.W + f * A.W_fs + r;
+        const double* lapr = A.lap + f * A.lap_fs + r;
+        double* coefr = A.coef + f * A.coef_fs + r;
+        const double* dur = A.du + f * A.st_fs + r;
+        const double* dvr = A.dv + f * A.st_fs + r;
+        // the first row's state also goes to the CTA above, as the row below its last one
+        const bool sends = above && row == 0;
+        unsigned halo = smem_addr(ring + kS + ROWS), halo_bar = full_bar(M - 1, 0);
+        if (sends) {
+            asm("mapa.shared::cluster.u32 %0, %0, %1;" : "+r"(halo) : "r"(cta - 1));
+            asm("mapa.shared::cluster.u32 %0, %0, %1;" : "+r"(halo_bar) : "r"(cta - 1));
+        }
+        const bool gets = below && strip == M - 1;
+        for (int s = fj; s < nsteps; s += FC) {
+            const int slot = (unsigned)s % S;
+            // the update has finished step s - ahead: the slot is free, and the states stored up to then can be read
+            if (s >= A.ahead) mbar_wait(empty_bar(strip, slot), ((unsigned)(s - A.ahead) / S) & 1, dead);
+            cur.advance(T, w, s - r);
+            const int c = s - r - cur.start, pk = cur.pk, o = (r + c) * P;
+            const bool in_level = row_ok && (unsigned)c < (unsigned)w;
+            FoldIn64<K> in;
+            double su = 0.0, sv = 0.0;
+            if (in_level) {
+                if (!(pk & kPkZero)) {
+                    su = dur[o];
+                    sv = dvr[o];
                 }
-                const bool more = cp < last;
-                const bool e_nx = more && tau + 2 >= cend, f_nx = more && tau + 1 >= cend;
-                const int Gp = pk_cur >> 8;
-                const bool final_out = !more && odu != nullptr;
-                const int c0 = tau - cstart;
-                const int c_f = f_nx ? tau + 1 - cend : c0 + 1;  // the pixel folded at the end of this step
-                const int pk_f = f_nx ? pk_nxt : pk_cur;
-                FoldIn64<K> fin;
-                fetch_fold(c_f, pk_f, fin);
-                const double2 ps0 = make_double2(cur.du, cur.dv);
-                const double2 ps1 = make_double2(nxt.du, nxt.dv);
-                const double2 dn1 = make_double2(nxt.nu, nxt.nv);
-                fetch_state(e_nx ? tau + 2 - cend : c0 + 2, e_nx ? pk_nxt : pk_cur, cur);
-                const int pin = (s + 1) & 1;  // parity written at step s - 1
+                if (pk & kPkCoef) {
 #pragma unroll
-                for (int gj = 0; gj < G; ++gj) {
-                    const int gi = G - 1 - gj;  // the independent updates first, the newest column last
-                    double2 up, dn;
-                    up.x = __shfl_up_sync(0xffffffffu, V1[gi].x, 1);
-                    up.y = __shfl_up_sync(0xffffffffu, V1[gi].y, 1);
-                    if (lane == 0 && warp > 0) up = xs(pin, warp - 1, 0, gi);
-                    if (CL && t == 0 && strip > 0) up = XE[(pin * 2 + 0) * G + gi];
-                    if (gi == 0) {
-                        dn = dn1;
-                    } else {
-                        dn.x = __shfl_down_sync(0xffffffffu, V1[gi - 1].x, 1);
-                        dn.y = __shfl_down_sync(0xffffffffu, V1[gi - 1].y, 1);
-                        if (lane == 31 && warp < NW - 1) dn = xs(pin, warp + 1, 1, gi - 1);
-                        if (CL && t == NT - 1 && strip < nc - 1) dn = XE[(pin * 2 + 1) * G + gi - 1];
-                    }
-                    const int c = c0 - 2 * gi;
-                    if (gi < Gp && row_ok && c >= 0 && c < w) {
-                        const double2 own = gi == 0 ? ps0 : V2[gi - 1];
-                        const double2 lf = c > 0 ? V1[gi] : own;
-                        const double2 rt = c < w - 1 ? (gi == 0 ? ps1 : V1[gi - 1]) : own;
-                        const double2 u_ = r > 0 ? up : own;
-                        const double2 d_ = r < h - 1 ? dn : own;
-                        int sl = slot0 - 2 * gi;
-                        if (sl < 0) sl += S;
-                        V0[gi] = sor_point64(own, u_, d_, lf, rt, CA[sl * NT + t], CB[sl * NT + t], CC[sl * NT + t],
-                                             wa, wb, omm);
-                        if (gi == Gp - 1) {
-                            if (final_out) {
-                                odu[(long long)r * A.out_rs + c] = V0[gi].x;
-                                odv[(long long)r * A.out_rs + c] = V0[gi].y;
-                                if (A.ring && (c == 0 || c == w - 1 || r == 0 || r == h - 1)) {
-                                    const long long o = (long long)r * A.out_rs + c;
-                                    for (int yr = r == 0 ? -1 : 0; yr <= (r == h - 1 ? 1 : 0); ++yr)
-                                        for (int xc = c == 0 ? -1 : 0; xc <= (c == w - 1 ? 1 : 0); ++xc)
-                                            if (yr | xc) {
-                                                odu[o + (long long)yr * A.out_rs + xc] = own.x;
-                                                odv[o + (long long)yr * A.out_rs + xc] = own.y;
-                                            }
-                                }
-                            } else {
-                                dur[(r + c) * P] = V0[gi].x;
-                                dvr[(r + c) * P] = V0[gi].y;
-                            }
+                    for (int q = 0; q < 5; ++q) in.j[q] = coefr[q * pl + o];
+                } else {
+#pragma unroll
+                    for (int q = 0; q < 6 * K; ++q) in.j[q] = __ldg(Jr + q * pl + o);
+                    const double* wsrc = (pk & kPkTick) ? Wr + K * pl : Wr;  // W * a_data on a tick
+#pragma unroll
+                    for (int k = 0; k < K; ++k) in.w[k] = __ldg(wsrc + k * pl + o);
+                    in.lu = __ldg(lapr + o);
+                    in.lv = __ldg(lapr + pl + o);
+                }
+            }
+            const int ro = slot * SR + row;
+            const double2 st = make_double2(su, sv);
+            ring[kS + ro] = st;
+            st_async_if(sends, halo + slot * SR * 16, *reinterpret_cast<const int4*>(&st), halo_bar + slot * 8);
+            if (in_level) {
+                const Coef64 cf = fold64<K>(A, pk, in, su, sv);
+                if (pk & kPkStore) {
+                    coefr[o] = cf.A12;
+                    coefr[pl + o] = cf.BU;
+                    coefr[2 * pl + o] = cf.BV;
+                    coefr[3 * pl + o] = cf.iDu;
+                    coefr[4 * pl + o] = cf.iDv;
+                }
+                ring[kA + ro] = make_double2(cf.A12, cf.BU);
+                ring[kB + ro] = make_double2(cf.BV, cf.iDu);
+                ringd[ro] = cf.iDv;
+            }
+            __syncwarp();
+            if (lane == 0) {
+                if (gets)
+                    mbar_arrive_expect(full_bar(strip, slot), sizeof(double2));
+                else
+                    mbar_arrive(full_bar(strip, slot));
+            }
+        }
+    } else if (warp == Roles::wait) {
+        // ------------------------------------------------------------ wait
+        // What a step needs from other warps and CTAs is awaited here, beside the update of the
+        // step before: the fold's slots and the neighbouring CTAs' edge rows.
+        auto wait_full = [&](int s) {
+            if (s < nsteps)
+                for (int st = 0; st < M; ++st) mbar_wait(full_bar(st, (unsigned)s % S), ((unsigned)s / S) & 1, dead);
+        };
+        wait_full(0);
+        wait_full(1);
+        asm volatile("bar.sync 1, %0;" ::"n"(32 * (WU + 1)) : "memory");
+        for (int s = 0; s < nsteps; ++s) {
+            wait_full(s + 2);
+            if (nc > 1 && s + 1 < nsteps) {
+                mbar_wait(edge_bar(s & 1), ((unsigned)s >> 1) & 1, dead);
+                if (lane == 0) mbar_expect(edge_bar(s & 1), edge_bytes);
+            }
+            asm volatile("bar.sync 1, %0;" ::"n"(32 * (WU + 1)) : "memory");
+            // step s is done by every iteration: the slot of the pixel that entered 2 (G - 1) steps ago is free
+            if (lane < M) mbar_arrive(empty_bar(lane, (unsigned)(s + A.ahead) % S));
+        }
+    } else if (update) {
+        // ---------------------------------------------------------- update
+        constexpr int NG = (G + NU - 1) / NU;  // iterations of this warp: g0, g0 + NU, ...
+        const int g0 = warp / M;
+        const double omm = A.one_m_omega, wa = A.wa, wb = A.wb;
+        const bool first_row = r == 0, last_row = r == h - 1;
+        // edge rows to the neighbouring CTAs: the last row's values go below, the first row's above
+        const bool send_dn = below && row == ROWS - 1, send_up = above && row == 0;
+        unsigned ebuf = smem_addr(bufs + (send_dn ? 0 : ROWS + 1)), ebar = edge_bar(0);
+        if (send_dn || send_up) {
+            const int peer = send_dn ? cta + 1 : cta - 1;
+            asm("mapa.shared::cluster.u32 %0, %0, %1;" : "+r"(ebuf) : "r"(peer));
+            asm("mapa.shared::cluster.u32 %0, %0, %1;" : "+r"(ebar) : "r"(peer));
+        }
+        double2 lf[NG], own[NG];  // the values left of the current pixel, and the pixel's own
+        double2* myring = ring + row;
+        int co[NG];               // ring offset of iteration i's pixel
+#pragma unroll
+        for (int i = 0; i < NG; ++i) {
+            lf[i] = own[i] = make_double2(0.0, 0.0);
+            co[i] = (unsigned)(-2 * (g0 + i * NU)) % S * SR;
+        }
+        auto next_slot = [&](int o) { return o == (S - 1) * SR ? 0 : o + SR; };
+        int so = 0, so1 = SR;                // state slots of steps s and s + 1
+        int b0 = 0, b1 = 2 * BUF, b2 = BUF;  // the buffers of steps s, s - 1, s - 2
+        double* sdu = A.du + f * A.st_fs + r;
+        double* sdv = A.dv + f * A.st_fs + r;
+        asm volatile("bar.sync 1, %0;" ::"n"(32 * (WU + 1)) : "memory");
+        if (g0 == 0) own[0] = myring[kS];
+        for (int s = 0; s < nsteps; ++s) {
+            cur.advance(T, w, s - r);
+            const int Gp = cur.pk >> 8;
+            const int d0 = s - cur.start;  // the diagonal of iteration 0's pixel
+#pragma unroll
+            for (int i = 0; i < NG; ++i) {
+                const int gi = g0 + i * NU;
+                if (gi >= G) break;
+                const int c = d0 - r - 2 * gi;
+                // where the iteration before has its values: of this pixel (before), and what it wrote
+                // in the last step: the right neighbour, and in the next row the lower one (prev)
+                const double2* base = gi == 0 ? myring + kS : bufs + (gi - 1) * 3 * BUF + row + 1;
+                const double2* before = base + (gi == 0 ? so : b2);
+                const double2* prev = base + (gi == 0 ? so1 : b1);
+                double2* mybuf = bufs + gi * 3 * BUF + row + 1;
+                // border copies: the neighbour outside is the pixel's own value before the update
+                const double2 rt = *(c == w - 1 ? before : prev);
+                double2 n = lf[i];
+                const bool valid = gi < Gp && row_ok && (unsigned)c < (unsigned)w;
+                if (valid) {
+                    const double2 dn = *(last_row ? before : prev + 1);
+                    const double2 up = *(first_row ? before : mybuf + b1 - 1);
+                    const double2 ow = own[i];
+                    n = sor_point64(ow, up, dn, c == 0 ? ow : lf[i], rt, myring[kA + co[i]], myring[kB + co[i]],
+                                    ringd[row + co[i]], wa, wb, omm);
+                    if (gi == Gp - 1) {
+                        if (cur.p < T.n - 1) {
+                            sdu[(d0 - 2 * gi) * P] = n.x;
+                            sdv[(d0 - 2 * gi) * P] = n.y;
+                        } else {
+                            const long long o = (long long)r * A.out_rs + c;
+                            odu[o] = n.x;
+                            odv[o] = n.y;
+                            if (A.ring && (c == 0 || c == w - 1 || r == 0 || r == h - 1))
+                                for (int yr = r == 0 ? -1 : 0; yr <= (r == h - 1 ? 1 : 0); ++yr)
+                                    for (int xc = c == 0 ? -1 : 0; xc <= (c == w - 1 ? 1 : 0); ++xc)
+                                        if (yr | xc) {
+                                            odu[o + (long long)yr * A.out_rs + xc] = ow.x;
+                                            odv[o + (long long)yr * A.out_rs + xc] = ow.y;
+                                        }
                         }
                     }
                 }
-                fold_into(c_f, pk_f, fin, nxt, slot1);
-                const int pout = s & 1;
-                if (lane == 31) {
-#pragma unroll
-                    for (int gi = 0; gi < G; ++gi) xs(pout, warp, 0, gi) = V0[gi];
-                }
-                if (lane == 0) {
-#pragma unroll
-                    for (int gi = 0; gi + 1 < G; ++gi) xs(pout, warp, 1, gi) = V0[gi];
-                }
-                if constexpr (CL) {
-                    if (t == NT - 1 && strip < nc - 1) {
-                        double2* dst = cooperative_groups::this_cluster().map_shared_rank(XE, strip + 1);
-#pragma unroll
-                        for (int gi = 0; gi < G; ++gi) dst[(pout * 2 + 0) * G + gi] = V0[gi];
-                    }
-                    if (t == 0 && strip > 0) {
-                        double2* dst = cooperative_groups::this_cluster().map_shared_rank(XE, strip - 1);
-#pragma unroll
-                        for (int gi = 0; gi + 1 < G; ++gi) dst[(pout * 2 + 1) * G + gi] = V0[gi];
-                    }
-                }
-#pragma unroll
-                for (int gi = 0; gi < G; ++gi) {
-                    V2[gi] = V1[gi];
-                    V1[gi] = V0[gi];
-                }
-                slot0 = slot1;
+                mybuf[b0] = n;
+                st_async_if((send_dn || (send_up && gi + 1 < G)) && s + 1 < nsteps, ebuf + (gi * 3 * BUF + b0) * 16,
+                            *reinterpret_cast<const int4*>(&n), ebar + (s & 1) * 8);
+                lf[i] = n;
+                own[i] = rt;
+                co[i] = next_slot(co[i]);
             }
-            step_barrier();
+            asm volatile("bar.sync 1, %0;" ::"n"(32 * (WU + 1)) : "memory");
+            so = so1;
+            so1 = next_slot(so1);
+            const int b = b2;
+            b2 = b1;
+            b1 = b0;
+            b0 = b;
         }
     }
+    if (dead) *gave_up = 1;
+    __syncthreads();
+    if (*gave_up && row_ok && update)  // a wait ran out: the rows' result is void
+        for (int c = warp / M; c < w; c += NU) {
+            const long long o = (long long)r * A.out_rs + c;
+            odu[o] = odv[o] = __longlong_as_double(0x7ff8000000000000ll);
+        }
+    sync_all();  // no CTA leaves while another may still write into its shared memory
 }
 
-// Row strips of a level with at most `rows` rows per CTA (256, 128 or 64): one
-// CTA when the level fits, else nc CTAs of nt rows (a cluster when nc > 1).
+// Row strips of a level with at most `rows` rows per CTA (256, 128 or 64).
 void split64(const DiagGeom& g, int rows, int* nc, int* nt)
 {
     const int n = (g.P + rows - 1) / rows;
@@ -554,52 +568,43 @@ void split64(const DiagGeom& g, int rows, int* nc, int* nt)
     *nt = ((g.P + n - 1) / n + 31) / 32 * 32;
 }
 
-template <int K, bool CO, bool CL, int NTM>
-cudaError_t run_chain64_t(const Sor64Args& A, const Chain64Table& T, int n_frames, int nt, cudaStream_t st)
+template <int K, int M, int NU, int FC, int MB>
+cudaError_t run_split64(Sor64Args A, const PassTable& T, int n_frames, cudaStream_t st)
 {
-    const size_t smem = chain64_smem(nt);
-    const cudaError_t e = ensure_max_dyn_smem((const void*)k_sor_chain64<K, CO, CL, NTM>, kSmem64);
+    constexpr size_t smem = Split64Smem<M>::bytes;
+    A.ahead = std::min(kFoldAhead, A.g.w - 1);
+    A.nc = (A.g.P / 32 + M - 1) / M;
+    if (A.nc > kMaxSplitCluster || (long long)n_frames * A.nc > 0x7fffffffLL) return cudaErrorInvalidValue;
+    auto kern = k_sor_split64<K, M, NU, FC, MB>;
+    cudaError_t e = ensure_max_dyn_smem((const void*)kern, (int)smem);
     if (e != cudaSuccess) return e;
-    if constexpr (!CL) {
-        k_sor_chain64<K, CO, false, NTM><<<n_frames, nt, smem, st>>>(A, T);
-        return cudaGetLastError();
-    } else {
-        if (A.nc > kPortableStrips) {
-            const cudaError_t e2 = ensure_nonportable_clusters((const void*)k_sor_chain64<K, CO, true, NTM>);
-            if (e2 != cudaSuccess) return e2;
-        }
-        cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3((unsigned)(n_frames * A.nc));
-        cfg.blockDim = dim3((unsigned)nt);
-        cfg.dynamicSmemBytes = smem;
-        cfg.stream = st;
-        cudaLaunchAttribute at[1];
-        at[0].id = cudaLaunchAttributeClusterDimension;
-        at[0].val.clusterDim.x = (unsigned)A.nc;
-        at[0].val.clusterDim.y = 1;
-        at[0].val.clusterDim.z = 1;
-        cfg.attrs = at;
-        cfg.numAttrs = 1;
-        return cudaLaunchKernelEx(&cfg, k_sor_chain64<K, CO, true, NTM>, A, T);
-    }
+    if (A.nc > kPortableStrips && (e = ensure_nonportable_clusters((const void*)kern)) != cudaSuccess) return e;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(n_frames * A.nc));
+    cfg.blockDim = dim3(32 * SplitRoles<M, NU, FC>::warps);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = (unsigned)A.nc;
+    at[0].val.clusterDim.y = 1;
+    at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = A.nc > 1 ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, kern, A, T);
 }
 
-template <int K, int NTM>
-cudaError_t run_chain64_n(const Sor64Args& A, const Chain64Table& T, bool co, int n_frames, int nt, cudaStream_t st)
-{
-    if (A.nc == 1)
-        return co ? run_chain64_t<K, true, false, NTM>(A, T, n_frames, nt, st)
-                  : run_chain64_t<K, false, false, NTM>(A, T, n_frames, nt, st);
-    return co ? run_chain64_t<K, true, true, NTM>(A, T, n_frames, nt, st)
-              : run_chain64_t<K, false, true, NTM>(A, T, n_frames, nt, st);
-}
-
+// Warps per 32 rows by what the launch has to fill: at most one CTA per SM, all
+// registers; more, two CTAs per SM (100 frames 291 ms against 364).  Levels over
+// 512 and 1024 rows need 64 and 128 rows per CTA.  Other counts of update and
+// fold warps measured within 3 % or worse.
 template <int K>
-cudaError_t run_chain64(const Sor64Args& A, const Chain64Table& T, bool co, int n_frames, int nt, cudaStream_t st)
+cudaError_t run_split64_m(const Sor64Args& A, const PassTable& T, int m, int n_frames, int n_sms, cudaStream_t st)
 {
-    if (nt <= 64) return run_chain64_n<K, 64>(A, T, co, n_frames, nt, st);
-    if (nt <= 128) return run_chain64_n<K, 128>(A, T, co, n_frames, nt, st);
-    return run_chain64_n<K, 256>(A, T, co, n_frames, nt, st);
+    if (m == 4) return run_split64<K, 4, 3, 3, 1>(A, T, n_frames, st);
+    if (m == 2) return run_split64<K, 2, 5, 6, 1>(A, T, n_frames, st);
+    if ((long long)n_frames * (A.g.P / 32) <= n_sms) return run_split64<K, 1, 5, 6, 1>(A, T, n_frames, st);
+    return run_split64<K, 1, 5, 6, 2>(A, T, n_frames, st);
 }
 
 }  // namespace
@@ -609,24 +614,7 @@ bool sor_chain64_rows_ok(const DiagGeom& g, int rows)
     if (rows != 64 && rows != 128 && rows != kLane64) return false;
     int nc, nt;
     split64(g, rows, &nc, &nt);
-    return nc <= kMaxStrips64 && chain64_smem(nt) <= (size_t)kSmem64;
-}
-
-int sor_chain64_default_rows(const DiagGeom& g, int n_frames, int n_sms)
-{
-    // levels over 512 rows: 128-row strips (three CTAs per SM) while the cluster
-    // stays within 16 CTAs
-    if (g.P > 512 && sor_chain64_rows_ok(g, 128)) return 128;
-    // the tallest strips that still give every SM work; shorter strips where a
-    // batch of few frames would leave SMs idle (one frame per call: 8 strips)
-    for (int rows = kLane64; rows >= 64; rows /= 2) {
-        if (!sor_chain64_rows_ok(g, rows)) break;
-        const long long ctas = (long long)n_frames * ((g.P + rows - 1) / rows);
-        if (ctas >= n_sms) return rows;
-    }
-    for (int rows = 64; rows <= kLane64; rows *= 2)
-        if (sor_chain64_rows_ok(g, rows)) return rows;
-    return kLane64;
+    return nc <= kMaxStrips64;
 }
 
 bool sor_chain64_supports(int K, const DiagGeom& g, int n_passes)
@@ -637,7 +625,7 @@ bool sor_chain64_supports(int K, const DiagGeom& g, int n_passes)
     // 32-bit offsets within a frame: the largest plane index read is (6K + 2) planes of D * P
     const long long plane = (long long)g.D * g.P;
     // the tallest strips must fit a portable cluster: the fallback of a refused larger cluster
-    return nc <= kPortableStrips && plane * (6 * K + 2) < 0x7fffffffLL && chain64_smem(nt) <= (size_t)kSmem64;
+    return nc <= kPortableStrips && plane * (6 * K + 2) < 0x7fffffffLL;
 }
 
 cudaError_t launch_sor_chain64(const double* J, long long J_fs, const double* W, long long W_fs, const double* lap,
@@ -648,21 +636,19 @@ cudaError_t launch_sor_chain64(const double* J, long long J_fs, const double* W,
                                int rows, const PowTab64* pows, const int* marks, int ring)
 {
     if (!sor_chain64_supports(K, g, n_passes) || n_frames < 1) return cudaErrorInvalidValue;
-    if (rows == 0) rows = kLane64;
-    if (!sor_chain64_rows_ok(g, rows)) return cudaErrorInvalidValue;
-    int nc = 0, nt = 0;
-    split64(g, rows, &nc, &nt);
-    if ((long long)n_frames * nc > 0x7fffffffLL) return cudaErrorInvalidValue;
-    Chain64Table T;
+    if (rows != 0 && !sor_chain64_rows_ok(g, rows)) return cudaErrorInvalidValue;
+    int dev = 0, n_sms = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&n_sms, cudaDevAttrMultiProcessorCount, dev);
+    if (e != cudaSuccess) return e;
+    PassTable T;
     T.n = n_passes;
-    bool co = false;
     for (int p = 0; p < n_passes; ++p) {
         const ChainPass& q = passes[p];
         if (q.G < 1 || q.G > kG64 || q.mode < -1 || q.mode > 3) return cudaErrorInvalidValue;
         const bool coef_in = q.mode < 0, store = q.mode >= 0 && q.store_coef;
         T.pk[p] = (q.G << 8) | (store ? kPkStore : 0) | (coef_in ? kPkCoef : 0) |
                   (!coef_in && (q.mode & 2) ? kPkTick : 0) | (!coef_in && (q.mode & 1) ? kPkZero : 0);
-        co = co || coef_in || store;
     }
     for (int p = n_passes; p < kMaxChain; ++p) T.pk[p] = 1 << 8;
     Sor64Args A;
@@ -693,24 +679,16 @@ cudaError_t launch_sor_chain64(const double* J, long long J_fs, const double* W,
         A.a_m1[k] = k < K ? a_data[k] - 1.0 : 0.0;
         A.pw[k] = pows && k < K ? pows[k] : PowTab64();
     }
-    auto launch = [&](int nc_, int nt_) {
-        A.nc = nc_;
-        switch (K) {
-            case 1: return run_chain64<1>(A, T, co, n_frames, nt_, st);
-            case 2: return run_chain64<2>(A, T, co, n_frames, nt_, st);
-            case 3: return run_chain64<3>(A, T, co, n_frames, nt_, st);
-            default: return run_chain64<4>(A, T, co, n_frames, nt_, st);
-        }
-    };
-    cudaError_t e = launch(nc, nt);
-    if (e != cudaSuccess && nc > kPortableStrips) {
-        // a device that cannot schedule a cluster this large refuses the launch (nothing ran, the
-        // error is not sticky): the tallest strips give the same bits with at most 8 CTAs
-        cudaGetLastError();
-        split64(g, kLane64, &nc, &nt);
-        e = launch(nc, nt);
+    // rows per CTA: 32 unless the cluster would pass 16 CTAs; a caller's choice of more is taken
+    const int strips = g.P / 32;
+    int m = strips <= kMaxSplitCluster ? 1 : (strips <= 2 * kMaxSplitCluster ? 2 : 4);
+    if (rows >= 64) m = std::max(m, rows >= 128 ? 4 : 2);
+    switch (K) {
+        case 1: return run_split64_m<1>(A, T, m, n_frames, n_sms, st);
+        case 2: return run_split64_m<2>(A, T, m, n_frames, n_sms, st);
+        case 3: return run_split64_m<3>(A, T, m, n_frames, n_sms, st);
+        default: return run_split64_m<4>(A, T, m, n_frames, n_sms, st);
     }
-    return e;
 }
 
 }  // namespace frg

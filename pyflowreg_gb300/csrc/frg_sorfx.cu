@@ -1,5 +1,8 @@
-// Exact-order chained SOR of the float64 path with the updates in 64-bit
-// fixed point.
+// Exact-order chained SOR of a single level (the level_solver seam) with the
+// updates in 64-bit fixed point, as exact as float64 but not its bits.  The
+// pyramid keeps k_sor_split64: there a last-bit difference moves psi by up to
+// 1e-7 where the residual cancels, and among the 1e8 pixels of a batch some 1/32
+// px warp sample of the next level comes out another one.
 //
 // compute_flow (core/level_solver.py:158-369) sweeps columns outer, rows inner,
 // in place, in float64.  On GB300 one float64 instruction holds a scheduler's
@@ -27,21 +30,20 @@
 //
 // Range.  States are held below 2^lim units, |a 2^k| below 2^kmax and p below
 // 2^62 units, with lim + kmax = 63: then the sum of the true terms stays below
-// 2^64 - 2^lim, so a sum that wraps cannot land in the range of a state.  A
-// frame's unit follows its size: q = lim - reach, where 2^reach px bounds the
-// largest |du|, |dv| that the frame reached on the coarser level, with a bit to
-// spare.  A coefficient or a state outside its range, or anything not finite,
+// 2^64 - 2^lim, so a sum that wraps cannot land in the range of a state.  The
+// unit follows from the caller's bound 2^reach px of |du|, |dv|: q = lim - reach.
+// A coefficient or a state outside its range, or anything not finite,
 // marks the frame, and so does a level whose result is nowhere above 2^42 units
 // but not zero (so small that a float64 state would hold more bits).  Marked
 // frames are solved again by a second launch with a wider format, and what that
-// one marks by k_sor_chain64.
+// one marks by k_sor_split64.
 //
-// Schedule: that of k_sor_chain64 (row r's local time is tau = s - r; pixel
+// Schedule: that of k_sor_split64 (row r's local time is tau = s - r; pixel
 // (r, c) of pipelined iteration gi of a pass is updated at tau = start + c +
 // 2 gi), with the work split over specialised warps.  Every 32 rows have NU
 // update warps, which share the five pipelined iterations, and FC fold warps,
 // which run ahead of them: fold warp j takes steps j, j + FC, ..., and writes
-// each entering pixel's coefficients and pass-start state into a ring of kFxRing
+// each entering pixel's coefficients and pass-start state into a ring of kRingSlots
 // slots in shared memory (mbarriers both ways).  The folds' float64
 // instructions and loads are off the update's critical path, and the float64
 // pipes of all four schedulers work on one row strip.  An update's neighbours
@@ -50,9 +52,7 @@
 // and own values and the row below the upper one; one barrier per step.  A
 // frame's strips in other CTAs of its cluster get the edge rows through
 // distributed shared memory (st.async with a transaction barrier).
-#include "frg_internal.h"
-
-#include <cooperative_groups.h>
+#include "frg_split.cuh"
 
 #include <algorithm>
 #include <cmath>
@@ -61,15 +61,8 @@ namespace frg {
 
 namespace {
 
-constexpr int kFxRing = 16;          // ring slots: a pixel's coefficients are read for 2 (G - 1) + 1 = 9 steps
-constexpr int kFxUse = 2 * (kGMax - 1);
-constexpr int kFxAhead = kFxRing - kFxUse;  // steps a fold may run ahead of the update
-constexpr int kFxMaxStrips = 64;
-constexpr int kFxMaxCluster = 16;
 constexpr int kFxKmax = 4, kFxLim = 63 - kFxKmax;  // |omega A12 / den| stays below 16 but for rare pixels of coarse levels
 constexpr int kFxWider = 3;          // bits by which the second launch widens both
-constexpr int kFxReachMin = 1, kFxReachMax = 10;
-constexpr unsigned kFxSpin = 500000u;       // bound of every wait, in tries of at most 2 us; a wait that runs out marks the frame
 
 struct FxArgs {
     const double* J;
@@ -93,81 +86,12 @@ struct FxArgs {
     long long half_omega, ca, cb;  // omega / 2, 2 wa / wsum, 2 wb / wsum: 61 fraction bits
     int oh, ol;          // 1 - omega
     FxPow pw[4];
-    FxState fs;
-    int lim, kmax, reach;  // reach < 0: from the frame's previous level
+    int *marks, *marks2;   // [n_frames] of the first and the second launch
+    int lim, kmax, reach;
+    int ahead;           // steps a fold may run ahead: at most the columns of a row less one
     int second;          // second launch: frames the first one marked, format wider by kFxWider bits
     int nc;              // CTAs per frame
 };
-
-struct FxTable {
-    int n;
-    int pk[kMaxChain];  // G << 8 | store << 3 | coef << 2 | tick << 1 | zero
-};
-
-constexpr int kPkZero = 1, kPkTick = 2, kPkCoef = 4, kPkStore = 8;
-
-__device__ __forceinline__ unsigned smem_addr(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
-
-__device__ __forceinline__ void mbar_init(unsigned mb, unsigned count)
-{
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(mb), "r"(count) : "memory");
-}
-
-__device__ __forceinline__ void mbar_arrive(unsigned mb)
-{
-    asm volatile("{\n\t.reg .b64 t;\n\tmbarrier.arrive.release.cta.shared::cta.b64 t, [%0];\n\t}" ::"r"(mb) : "memory");
-}
-
-__device__ __forceinline__ void mbar_expect(unsigned mb, unsigned bytes)
-{
-    asm volatile("{\n\t.reg .b64 t;\n\tmbarrier.arrive.expect_tx.relaxed.cta.shared::cta.b64 t, [%0], %1;\n\t}" ::"r"(mb),
-                 "r"(bytes)
-                 : "memory");
-}
-
-__device__ __forceinline__ void mbar_arrive_expect(unsigned mb, unsigned bytes)
-{
-    asm volatile("{\n\t.reg .b64 t;\n\tmbarrier.arrive.expect_tx.release.cta.shared::cta.b64 t, [%0], %1;\n\t}" ::"r"(mb),
-                 "r"(bytes)
-                 : "memory");
-}
-
-// 16 bytes into another CTA's shared memory, counted by a barrier there.  A
-// predicated instruction: a branch around it costs the step about 50 clocks.
-__device__ __forceinline__ void st_async_if(bool p, unsigned addr, int4 v, unsigned mb)
-{
-    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.s32 p, %6, 0;\n\t"
-                 "@p st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v4.b32 [%0], {%1, %2, %3, %4}, [%5];\n\t}" ::"r"(addr),
-                 "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w), "r"(mb), "r"((int)p)
-                 : "memory");
-}
-
-__device__ __forceinline__ void st_global_if(bool p, long long* a, long long v)
-{
-    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.s32 p, %2, 0;\n\t@p st.global.b64 [%0], %1;\n\t}" ::"l"(a), "l"(v), "r"((int)p)
-                 : "memory");
-}
-
-__device__ __forceinline__ bool mbar_test(unsigned mb, unsigned parity)
-{
-    unsigned ok;
-    asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2, 2000;\n\t"
-                 "selp.u32 %0, 1, 0, p;\n\t}"
-                 : "=r"(ok)
-                 : "r"(mb), "r"(parity)
-                 : "memory");
-    return ok != 0;
-}
-
-// Waits for the phase with this parity to complete.  After one wait has run
-// out no further one is made (the frame is marked and recomputed).
-__device__ __forceinline__ void mbar_wait(unsigned mb, unsigned parity, bool& dead)
-{
-    if (dead) return;
-    for (unsigned i = 0; i < kFxSpin; ++i)
-        if (mbar_test(mb, parity)) return;
-    dead = true;
-}
 
 __device__ __forceinline__ long long mulw(int a, int b) { return (long long)a * b; }
 
@@ -421,18 +345,18 @@ __device__ __forceinline__ long long join(int h, int l) { return ((long long)h <
 
 constexpr int kFxTabBytes = 64 * 16 + 256 * 8 + 256 * 4;
 
-// Shared memory of a CTA of M strips: ring int4[planes][kFxRing][32 M] with the
-// state plane's halo int4[kFxRing] | iteration buffers int4[G][3][32 M + 2] |
-// mbarriers: full[M][kFxRing], empty[M][kFxRing], edge[2 parities] | the power table where there is room.
+// Shared memory of a CTA of M strips: ring int4[planes][kRingSlots][32 M] with the
+// state plane's halo int4[kRingSlots] | iteration buffers int4[G][3][32 M + 2] |
+// mbarriers: full[M][kRingSlots], empty[M][kRingSlots], edge[2 parities] | the power table where there is room.
 template <int M, bool ISO>
 struct FxSmem {
     static constexpr int rows = 32 * M;
-    static constexpr int plane = kFxRing * (rows + 1);  // int4 per ring plane (the halo row only used by the state)
+    static constexpr int plane = kRingSlots * (rows + 1);  // int4 per ring plane (the halo row only used by the state)
     static constexpr int planes = ISO ? 5 : 6;
     static constexpr int buf = rows + 2;
     static constexpr size_t bytes =
-        ((size_t)planes * plane + (size_t)kGMax * 3 * buf) * sizeof(int4) + (size_t)(2 * M * kFxRing + 2) * 8;
-    static constexpr bool table = M < 4;  // room for a power table
+        ((size_t)planes * plane + (size_t)kGMax * 3 * buf) * sizeof(int4) + (size_t)(2 * M * kRingSlots + 2) * 8;
+    static constexpr bool table = bytes + kFxTabBytes <= 232448;  // room for a power table
     static constexpr size_t bytes_all = bytes + (table ? kFxTabBytes : 0);
 };
 
@@ -457,42 +381,15 @@ __host__ __device__ __forceinline__ void place_fx(const void* tab, FxPow* P)
     P->R = reinterpret_cast<const unsigned*>(P->B + 256);
 }
 
-// Steps a row spends in a pass.  After a single iteration one step more, so that
-// the step before a row's first pixel of the next pass (which takes that
-// pixel's value as its right neighbour) is free.
-__device__ __forceinline__ int fx_span(int w, int pk)
-{
-    const int n = pk >> 8;
-    return w + (n > 1 ? 2 * (n - 1) : 1);
-}
-
-// A row's place in the chain of passes at local time tau.
-struct Cursor {
-    int p, start, end, pk;
-    __device__ __forceinline__ void init(const FxTable& T, int w)
-    {
-        p = 0;
-        start = 0;
-        pk = T.pk[0];
-        end = fx_span(w, pk);
-    }
-    __device__ __forceinline__ void advance(const FxTable& T, int w, int tau)
-    {
-        if (tau >= end && p < T.n - 1) {
-            ++p;
-            start = end;
-            pk = T.pk[p];
-            end = start + fx_span(w, pk);
-        }
-    }
-};
-
-template <int K, bool ISO, int M, int NU, int FC>
-__global__ void __launch_bounds__(32 * (M * (NU + FC) + 1)) k_sor_fx(FxArgs A, FxTable T)
+// MB: CTAs per SM that the registers are to allow.  A fold's loads are not
+// fetched ahead: the registers for that would cost the second CTA of an SM, and
+// folds wait less than they run ahead.
+template <int K, bool ISO, int M, int NU, int FC, int MB>
+__global__ void __launch_bounds__(32 * SplitRoles<M, NU, FC>::warps, MB) k_sor_fx(FxArgs A, PassTable T)
 {
     using SM = FxSmem<M, ISO>;
     constexpr int G = kGMax;
-    constexpr int S = kFxRing;
+    constexpr int S = kRingSlots;
     constexpr int ROWS = SM::rows, PL = SM::plane, SR = ROWS + 1, BUF = SM::buf;
     extern __shared__ __align__(16) unsigned char fx_sm[];
     int4* ring = reinterpret_cast<int4*>(fx_sm);
@@ -502,10 +399,11 @@ __global__ void __launch_bounds__(32 * (M * (NU + FC) + 1)) k_sor_fx(FxArgs A, F
     const int nc = A.nc;
     const int cta = nc > 1 ? (int)(blockIdx.x % nc) : 0;
     const int f = nc > 1 ? (int)(blockIdx.x / nc) : (int)blockIdx.x;
-    if (A.second && !fx_recompute(A.fs.marks[f])) return;  // the same for every CTA of a cluster
-    // warps: M NU for the update (strip, iterations), one that waits for them, M FC for the fold
-    constexpr int WU = M * NU;
-    const int strip = (warp < WU ? warp : warp - WU - 1) % M;
+    if (A.second && !fx_recompute(A.marks[f])) return;  // the same for every CTA of a cluster
+    using Roles = SplitRoles<M, NU, FC>;
+    constexpr int WU = Roles::WU;
+    const bool update = warp < WU;
+    const int strip = (update ? warp : Roles::fold(warp)) % M;
     const int row = strip * 32 + lane;  // in the CTA
     const int r = cta * ROWS + row;     // in the level
     const DiagGeom g = A.g;
@@ -539,29 +437,24 @@ __global__ void __launch_bounds__(32 * (M * (NU + FC) + 1)) k_sor_fx(FxArgs A, F
     };
     sync_all();
 
-    // the frame's format
-    int reach = A.reach;
-    if (reach < 0) {
-        reach = fx_recompute(A.fs.prev_marks[f]) ? A.fs.prev_reach2[f] : A.fs.prev_reach[f];
-        reach = min(max(reach + 1, kFxReachMin), kFxReachMax);
-    }
+    // the number format
     const int kmax = A.kmax + (A.second ? kFxWider : 0);
     const int lim = A.lim - (A.second ? kFxWider : 0);
-    const int q = lim - reach - (A.second ? kFxWider : 0);
+    const int q = lim - A.reach - (A.second ? kFxWider : 0);
 
     double* odu = A.out_du + f * A.out_fs;
     double* odv = A.out_dv + f * A.out_fs;
     int total = 0;
-    for (int p = 0; p < T.n; ++p) total += fx_span(w, T.pk[p]);
+    for (int p = 0; p < T.n; ++p) total += pass_span(w, T.pk[p]);
     const int nsteps = total + h - 1;
     bool dead = false;
     int bad = 0, big = 0, nonzero = 0, top = 0;
     Cursor cur;
     cur.init(T, w);
 
-    if (warp > WU) {
+    if (!update && warp != Roles::wait && warp != Roles::idle) {
         // ------------------------------------------------------------ fold
-        const int fj = (warp - WU - 1) / M;
+        const int fj = Roles::fold(warp) / M;
         FxPow pw[K];
 #pragma unroll
         for (int k = 0; k < K; ++k) {
@@ -582,12 +475,20 @@ __global__ void __launch_bounds__(32 * (M * (NU + FC) + 1)) k_sor_fx(FxArgs A, F
             asm("mapa.shared::cluster.u32 %0, %0, %1;" : "+r"(halo_bar) : "r"(cta - 1));
         }
         const bool gets = below && strip == M - 1;
-        // a pixel's pass-start state is stored w steps before it enters again: with w steps
-        // to spare over this warp's lead it is fetched one fold ahead, like J and W
-        const bool early = w >= FC + kFxAhead;
-        auto fetch = [&](int c, int pk, FxIn<K>& in) {
-            if (row_ok && (unsigned)c < (unsigned)w) {
-                const int o = (r + c) * P;
+        for (int s = fj; s < nsteps; s += FC) {
+            const int slot = (unsigned)s % S;
+            // the update has finished step s - ahead: the slot is free, and the states stored up to then can be read
+            if (s >= A.ahead) mbar_wait(empty_bar(strip, slot), ((unsigned)(s - A.ahead) / S) & 1, dead);
+            cur.advance(T, w, s - r);
+            const int c = s - r - cur.start, pk = cur.pk, o = (r + c) * P;
+            const bool in_level = row_ok && (unsigned)c < (unsigned)w;
+            FxIn<K> in;
+            long long su = 0, sv = 0;
+            if (in_level) {
+                if (!(pk & kPkZero)) {
+                    su = dur[o];
+                    sv = dvr[o];
+                }
 #pragma unroll
                 for (int i = 0; i < 6 * K; ++i) in.j[i] = __ldg(Jr + i * pl + o);
                 const double* wsrc = (pk & kPkCoef) ? wpr : ((pk & kPkTick) ? Wr + K * pl : Wr);
@@ -596,36 +497,11 @@ __global__ void __launch_bounds__(32 * (M * (NU + FC) + 1)) k_sor_fx(FxArgs A, F
                 in.lu = __ldg(lapr + o);
                 in.lv = __ldg(lapr + pl + o);
             }
-        };
-        auto fetch_state = [&](int c, int pk, long long& su, long long& sv) {
-            su = sv = 0;
-            if (row_ok && (unsigned)c < (unsigned)w && !(pk & kPkZero)) {
-                const int o = (r + c) * P;
-                su = dur[o];
-                sv = dvr[o];
-            }
-        };
-        FxIn<K> in;
-        long long su = 0, sv = 0;
-        cur.advance(T, w, fj - r);
-        fetch(fj - r - cur.start, cur.pk, in);
-        for (int s = fj; s < nsteps; s += FC) {
-            const int slot = (unsigned)s % S;
-            // the update has finished step s - kFxAhead: the slot is free, and the states stored up to then can be read
-            if (s >= kFxAhead) mbar_wait(empty_bar(strip, slot), ((unsigned)(s - kFxAhead) / S) & 1, dead);
-            const int c = s - r - cur.start, pk = cur.pk;
-            if (!early) fetch_state(c, pk, su, sv);
-            const FxIn<K> now = in;
-            const long long nu = su, nv = sv;
-            cur.advance(T, w, s + FC - r);
-            fetch(s + FC - r - cur.start, cur.pk, in);
-            if (early) fetch_state(s + FC - r - cur.start, cur.pk, su, sv);
             int4* sl = ring + slot * SR + row;
-            const int2 lu = limbs(nu), lv = limbs(nv);
+            const int2 lu = limbs(su), lv = limbs(sv);
             sl[kPS * PL] = make_int4(lu.x, lu.y, lv.x, lv.y);
             st_async_if(sends, halo + slot * SR * 16, make_int4(lu.x, lu.y, lv.x, lv.y), halo_bar + slot * 8);
-            if (row_ok && (unsigned)c < (unsigned)w)
-                fx_fold<K, ISO>(A, pw, pk, now, nu, nv, wpr + (r + c) * P, pl, sl, PL, q, kmax, bad);
+            if (in_level) fx_fold<K, ISO>(A, pw, pk, in, su, sv, wpr + o, pl, sl, PL, q, kmax, bad);
             __syncwarp();
             if (lane == 0) {
                 if (gets)
@@ -634,7 +510,7 @@ __global__ void __launch_bounds__(32 * (M * (NU + FC) + 1)) k_sor_fx(FxArgs A, F
                     mbar_arrive(full_bar(strip, slot));
             }
         }
-    } else if (warp == WU) {
+    } else if (warp == Roles::wait) {
         // ------------------------------------------------------------ wait
         // What a step needs from other warps and CTAs is awaited here, beside the update of the
         // step before: the fold's slots and the neighbouring CTAs' edge rows.
@@ -653,9 +529,9 @@ __global__ void __launch_bounds__(32 * (M * (NU + FC) + 1)) k_sor_fx(FxArgs A, F
             }
             asm volatile("bar.sync 1, %0;" ::"n"(32 * (WU + 1)) : "memory");
             // step s is done by every iteration: the slot of the pixel that entered 2 (G - 1) steps ago is free
-            if (lane < M) mbar_arrive(empty_bar(lane, (unsigned)(s + kFxAhead) % S));
+            if (lane < M) mbar_arrive(empty_bar(lane, (unsigned)(s + A.ahead) % S));
         }
-    } else {
+    } else if (update) {
         // ---------------------------------------------------------- update
         constexpr int NG = (G + NU - 1) / NU;  // iterations of this warp: g0, g0 + NU, ...
         const int g0 = warp / M;
@@ -694,6 +570,8 @@ __global__ void __launch_bounds__(32 * (M * (NU + FC) + 1)) k_sor_fx(FxArgs A, F
         };
         int so = 0, so1 = SR;           // state slots of steps s and s + 1
         int b0 = 0, b1 = 2 * BUF, b2 = BUF;  // the buffers of steps s, s - 1, s - 2
+        long long* sdu = A.du + f * A.st_fs + r;
+        long long* sdv = A.dv + f * A.st_fs + r;
         asm volatile("bar.sync 1, %0;" ::"n"(32 * (WU + 1)) : "memory");
         if (g0 == 0) own[0] = myring[kPS * PL];
         fetch_coef();
@@ -744,11 +622,14 @@ __global__ void __launch_bounds__(32 * (M * (NU + FC) + 1)) k_sor_fx(FxArgs A, F
                 const bool valid = gi < Gp && row_ok && (unsigned)c < (unsigned)w;
                 top |= valid ? (uh ^ (uh >> 31)) | (vh ^ (vh >> 31)) : 0;
                 const bool last = valid && gi == Gp - 1;
-                long long* ou = reinterpret_cast<long long*>(A.du) + f * A.st_fs + r + (long long)(d0 - 2 * gi) * P;
-                long long* ov = reinterpret_cast<long long*>(A.dv) + f * A.st_fs + r + (long long)(d0 - 2 * gi) * P;
-                st_global_if(last, ou, U - (1 << 29));
-                st_global_if(last, ov, V - (1 << 29));
-                if (A.ring && last && cur.p == T.n - 1) fx_ring(odu, odv, A.out_rs, r, c, h, w, ow, q);
+                if (__any_sync(~0u, last)) {
+                    const int o = (d0 - 2 * gi) * P;
+                    if (last) {
+                        sdu[o] = U - (1 << 29);
+                        sdv[o] = V - (1 << 29);
+                        if (A.ring && cur.p == T.n - 1) fx_ring(odu, odv, A.out_rs, r, c, h, w, ow, q);
+                    }
+                }
                 lf[i] = n;
                 own[i] = rt;
             }
@@ -765,10 +646,10 @@ __global__ void __launch_bounds__(32 * (M * (NU + FC) + 1)) k_sor_fx(FxArgs A, F
     }
     // the level's result, by all warps: states as float64, row-major
     __syncthreads();
-    if (row_ok && warp != WU) {
+    if (row_ok && (update || (warp != Roles::wait && warp != Roles::idle))) {
         const long long* sdu = A.du + f * A.st_fs + r;
         const long long* sdv = A.dv + f * A.st_fs + r;
-        for (int c = warp < WU ? warp / M : NU + (warp - WU - 1) / M; c < w; c += NU + FC) {
+        for (int c = update ? warp / M : NU + Roles::fold(warp) / M; c < w; c += NU + FC) {
             const long long nu = sdu[(r + c) * P], nv = sdv[(r + c) * P];
             const long long mag = (nu < 0 ? ~nu : nu) | (nv < 0 ? ~nv : nv);
             big |= mag >= (1ll << 42);
@@ -780,26 +661,24 @@ __global__ void __launch_bounds__(32 * (M * (NU + FC) + 1)) k_sor_fx(FxArgs A, F
     }
     const int m = (bad || dead ? 1 : 0) | (big ? 2 : 0) | (nonzero ? 4 : 0);
     const int mm = __reduce_or_sync(~0u, m);
-    const int tt = __reduce_or_sync(~0u, top);
-    int* marks = A.second ? A.fs.marks2 : A.fs.marks;
-    int* out_reach = A.second ? A.fs.reach2 : A.fs.reach;
-    if (lane == 0 && mm) atomicOr(marks + f, mm);
-    // the largest |du|, |dv| of any iteration is below 2^(64 - clz(tt) - q) px; floor at 0
-    if (lane == 0 && warp < WU) atomicMax(out_reach + f, max(0, 64 - __clz(tt) - q));
+    if (lane == 0 && mm) atomicOr((A.second ? A.marks2 : A.marks) + f, mm);
     sync_all();  // no CTA leaves while another may still write into its shared memory
 }
 
-template <int K, bool ISO, int M, int NU, int FC>
-cudaError_t run_fx(const FxArgs& A, const FxTable& T, int n_frames, cudaStream_t st)
+template <int K, bool ISO, int M, int NU, int FC, int MB>
+cudaError_t run_fx(FxArgs A, const PassTable& T, int n_frames, cudaStream_t st)
 {
     constexpr size_t smem = FxSmem<M, ISO>::bytes_all;
-    auto kern = k_sor_fx<K, ISO, M, NU, FC>;
+    A.ahead = std::min(kFoldAhead, A.g.w - 1);
+    A.nc = (A.g.P / 32 + M - 1) / M;
+    if (A.nc > kMaxSplitCluster) return cudaErrorInvalidValue;
+    auto kern = k_sor_fx<K, ISO, M, NU, FC, MB>;
     cudaError_t e = ensure_max_dyn_smem((const void*)kern, (int)smem);
     if (e != cudaSuccess) return e;
     if (A.nc > 8 && (e = ensure_nonportable_clusters((const void*)kern)) != cudaSuccess) return e;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)(n_frames * A.nc));
-    cfg.blockDim = dim3(32 * (M * (NU + FC) + 1));
+    cfg.blockDim = dim3(32 * SplitRoles<M, NU, FC>::warps);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
     cudaLaunchAttribute at[1];
@@ -812,16 +691,19 @@ cudaError_t run_fx(const FxArgs& A, const FxTable& T, int n_frames, cudaStream_t
     return cudaLaunchKernelEx(&cfg, kern, A, T);
 }
 
+// 32 rows per CTA, five update and eight fold warps each with all registers, up to
+// the 512 rows that a cluster of 16 CTAs covers (the level of 410 x 410 x 2 in
+// seam_chain64).  Levels over 512 and 1024 rows need 64 and 128 rows per CTA.
 template <int K, bool ISO>
-cudaError_t run_fx_m(const FxArgs& A, const FxTable& T, int m, int n_frames, cudaStream_t st)
+cudaError_t run_fx_m(const FxArgs& A, const PassTable& T, int m, int n_frames, cudaStream_t st)
 {
-    if (m == 1) return run_fx<K, ISO, 1, 5, 8>(A, T, n_frames, st);
-    if (m == 2) return run_fx<K, ISO, 2, 1, 4>(A, T, n_frames, st);
-    return run_fx<K, ISO, 4, 1, 2>(A, T, n_frames, st);
+    if (m == 4) return run_fx<K, ISO, 4, 3, 3, 1>(A, T, n_frames, st);
+    if (m == 2) return run_fx<K, ISO, 2, 5, 6, 1>(A, T, n_frames, st);
+    return run_fx<K, ISO, 1, 5, 8, 1>(A, T, n_frames, st);
 }
 
 template <int K>
-cudaError_t run_fx_k(const FxArgs& A, const FxTable& T, int m, int n_frames, cudaStream_t st)
+cudaError_t run_fx_k(const FxArgs& A, const PassTable& T, int m, int n_frames, cudaStream_t st)
 {
     return A.ca == A.cb ? run_fx_m<K, true>(A, T, m, n_frames, st) : run_fx_m<K, false>(A, T, m, n_frames, st);
 }
@@ -862,10 +744,10 @@ void place_fx_pow(void* dev, FxPow* P) { place_fx(dev, P); }
 
 bool sor_fx_supports(int K, const DiagGeom& g, int n_passes, double omega)
 {
-    // w: a pixel's state has to be stored before the fold that reads it, up to kFxAhead steps
-    // ahead of the update; omega in [1, 2) keeps |1 - omega| < 1 and c < 1/2
-    return K >= 1 && K <= 4 && (g.P & 31) == 0 && g.w >= kFxAhead + 1 && n_passes >= 1 && n_passes <= kMaxChain &&
-           g.P / 32 <= kFxMaxStrips && omega >= 1.0 && omega < 2.0 &&
+    // three columns or more, so that a state is stored before a fold (at least two steps ahead of
+    // the update) reads it; omega in [1, 2) keeps |1 - omega| < 1 and c < 1/2
+    return K >= 1 && K <= 4 && (g.P & 31) == 0 && g.w >= 3 && n_passes >= 1 && n_passes <= kMaxChain &&
+           g.P / 32 <= kMaxSplitStrips && omega >= 1.0 && omega < 2.0 &&
            (long long)g.D * g.P * (6 * K + 2) < 0x7fffffffLL;
 }
 
@@ -873,14 +755,14 @@ cudaError_t launch_sor_fx(const double* J, long long J_fs, const double* W, long
                           long long lap_fs, double* wp, long long wp_fs, double* du, double* dv, long long st_fs,
                           int n_frames, int K, DiagGeom g, const ChainPass* passes, int n_passes, double wx, double wy,
                           double omega, cudaStream_t st, double* out_du, double* out_dv, long long out_fs, int out_rs,
-                          int ring, int rows, const FxPow* pows, int reach, int second, const FxState& fs)
+                          int ring, const FxPow* pows, int reach, int second, int* marks, int* marks2)
 {
-    if (!sor_fx_supports(K, g, n_passes, omega) || n_frames < 1 || !out_du || !out_dv || !fs.marks)
+    if (!sor_fx_supports(K, g, n_passes, omega) || n_frames < 1 || !out_du || !out_dv || !marks || !marks2)
         return cudaErrorInvalidValue;
+    // rows per CTA: 32, the most CTAs per frame, unless the cluster would pass 16 CTAs
     const int strips = g.P / 32;
-    int m = rows >= 128 ? 4 : (rows >= 64 ? 2 : 1);
-    while ((strips + m - 1) / m > kFxMaxCluster) m *= 2;
-    FxTable T;
+    const int m = strips <= kMaxSplitCluster ? 1 : (strips <= 2 * kMaxSplitCluster ? 2 : 4);
+    PassTable T;
     T.n = n_passes;
     for (int p = 0; p < n_passes; ++p) {
         const ChainPass& c = passes[p];
@@ -923,8 +805,8 @@ cudaError_t launch_sor_fx(const double* J, long long J_fs, const double* W, long
     A.kmax = kFxKmax;
     A.reach = reach;
     A.second = second;
-    A.fs = fs;
-    A.nc = (strips + m - 1) / m;
+    A.marks = marks;
+    A.marks2 = marks2;
     switch (K) {
         case 1: return run_fx_k<1>(A, T, m, n_frames, st);
         case 2: return run_fx_k<2>(A, T, m, n_frames, st);

@@ -1,0 +1,135 @@
+// What the split forms of the chained float64 SOR share (k_sor_split64,
+// k_sor_fx): the work of 32 rows is divided among update warps (one per
+// pipelined iteration), fold warps that run ahead of them and one warp that waits
+// for both and for the neighbouring CTAs; rings, barriers and the place of a row
+// in the chain of passes.
+//
+// Every wait is bounded: a wait that runs out is given up, and so is every later
+// one of that warp, so that the kernel ends; the caller of mbar_wait reports it.
+#pragma once
+
+#include "frg_internal.h"
+
+#include <cooperative_groups.h>
+
+namespace frg {
+
+namespace {
+
+constexpr int kRingSlots = 16;          // ring slots: a pixel's coefficients are read for 2 (G - 1) + 1 = 9 steps
+constexpr int kRingUse = 2 * (kGMax - 1);
+constexpr int kFoldAhead = kRingSlots - kRingUse;  // most steps a fold may run ahead of the update
+constexpr int kMaxSplitStrips = 64;
+constexpr int kMaxSplitCluster = 16;
+constexpr unsigned kMaxTries = 500000u;  // tries of a wait, of at most 2 us each
+
+struct PassTable {
+    int n;
+    int pk[kMaxChain];  // G << 8 | store << 3 | coef << 2 | tick << 1 | zero
+};
+
+constexpr int kPkZero = 1, kPkTick = 2, kPkCoef = 4, kPkStore = 8;
+
+__device__ __forceinline__ unsigned smem_addr(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
+
+__device__ __forceinline__ void mbar_init(unsigned mb, unsigned count)
+{
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(mb), "r"(count) : "memory");
+}
+
+__device__ __forceinline__ void mbar_arrive(unsigned mb)
+{
+    asm volatile("{\n\t.reg .b64 t;\n\tmbarrier.arrive.release.cta.shared::cta.b64 t, [%0];\n\t}" ::"r"(mb) : "memory");
+}
+
+__device__ __forceinline__ void mbar_expect(unsigned mb, unsigned bytes)
+{
+    asm volatile("{\n\t.reg .b64 t;\n\tmbarrier.arrive.expect_tx.relaxed.cta.shared::cta.b64 t, [%0], %1;\n\t}" ::"r"(mb),
+                 "r"(bytes)
+                 : "memory");
+}
+
+__device__ __forceinline__ void mbar_arrive_expect(unsigned mb, unsigned bytes)
+{
+    asm volatile("{\n\t.reg .b64 t;\n\tmbarrier.arrive.expect_tx.release.cta.shared::cta.b64 t, [%0], %1;\n\t}" ::"r"(mb),
+                 "r"(bytes)
+                 : "memory");
+}
+
+// 16 bytes into another CTA's shared memory, counted by a barrier there.  A
+// predicated instruction: a branch around it costs the step about 50 clocks.
+__device__ __forceinline__ void st_async_if(bool p, unsigned addr, int4 v, unsigned mb)
+{
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.s32 p, %6, 0;\n\t"
+                 "@p st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v4.b32 [%0], {%1, %2, %3, %4}, [%5];\n\t}" ::"r"(addr),
+                 "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w), "r"(mb), "r"((int)p)
+                 : "memory");
+}
+
+__device__ __forceinline__ bool mbar_test(unsigned mb, unsigned parity)
+{
+    unsigned ok;
+    asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2, 2000;\n\t"
+                 "selp.u32 %0, 1, 0, p;\n\t}"
+                 : "=r"(ok)
+                 : "r"(mb), "r"(parity)
+                 : "memory");
+    return ok != 0;
+}
+
+// Waits for the phase with this parity to complete.  After one wait has run
+// out no further one is made (the frame is marked and recomputed).
+__device__ __forceinline__ void mbar_wait(unsigned mb, unsigned parity, bool& dead)
+{
+    if (dead) return;
+    for (unsigned i = 0; i < kMaxTries; ++i)
+        if (mbar_test(mb, parity)) return;
+    dead = true;
+}
+
+// Steps a row spends in a pass.  After a single iteration one step more, so that
+// the step before a row's first pixel of the next pass (which takes that
+// pixel's value as its right neighbour) is free.
+__device__ __forceinline__ int pass_span(int w, int pk)
+{
+    const int n = pk >> 8;
+    return w + (n > 1 ? 2 * (n - 1) : 1);
+}
+
+// Which warp does what.  Warp i runs on scheduler i % 4, and with five update
+// warps two share one: that scheduler gets the waiting warp besides and no fold
+// (one idle warp fills its place when there are more than six).
+template <int M, int NU, int FC>
+struct SplitRoles {
+    static constexpr int WU = M * NU;
+    static constexpr bool spread = M == 1 && NU == 5;
+    static constexpr int wait = spread ? 8 : WU;
+    static constexpr int idle = spread && FC > 6 ? 12 : -1;
+    static constexpr int warps = WU + 1 + M * FC + (idle >= 0 ? 1 : 0);
+    __device__ static int fold(int warp) { return spread ? warp - (warp < 8 ? 5 : (warp < 12 ? 6 : 7)) : warp - WU - 1; }
+};
+
+// A row's place in the chain of passes at local time tau.
+struct Cursor {
+    int p, start, end, pk;
+    __device__ __forceinline__ void init(const PassTable& T, int w)
+    {
+        p = 0;
+        start = 0;
+        pk = T.pk[0];
+        end = pass_span(w, pk);
+    }
+    __device__ __forceinline__ void advance(const PassTable& T, int w, int tau)
+    {
+        if (tau >= end && p < T.n - 1) {
+            ++p;
+            start = end;
+            pk = T.pk[p];
+            end = start + pass_span(w, pk);
+        }
+    }
+};
+
+}  // namespace
+
+}  // namespace frg
