@@ -1023,11 +1023,11 @@ int frg_set_reference(frg_plan* pl, const float* fixed, const float* weight, voi
     if (pl->xpath) {
         for (LevelPlan& L : pl->levels) {
             const long long hw = (long long)L.h * L.w, mn = (long long)(L.h + 2) * (L.w + 2);
-            FRG_LAUNCH(launch_x_resize_h_f(fixed, 0, 1, (long long)W * K, K, 1, K, H, pl->tmp, L.w, L.img.ix,
+            FRG_LAUNCH(launch_x_resize_h_f(fixed, 0, 1, (long long)W * K, K, 1, K, H, W, pl->tmp, L.w, L.img.ix,
                                            L.img.wx, L.img.P, st));
             FRG_LAUNCH(launch_x_resize_v_f(pl->tmp, 1, K, H, L.w, L.ref, 0, hw, L.w, L.h, 0, L.img.iy, L.img.wy,
                                            L.img.P, st));
-            FRG_LAUNCH(launch_x_resize_h_f(wsrc, 0, 1, (long long)W * K, K, 1, K, H, pl->tmp, L.w, L.img.ix,
+            FRG_LAUNCH(launch_x_resize_h_f(wsrc, 0, 1, (long long)W * K, K, 1, K, H, W, pl->tmp, L.w, L.img.ix,
                                            L.img.wx, L.img.P, st));
             FRG_LAUNCH(launch_x_resize_v_d(pl->tmp, 1, K, H, L.w, L.wpad64, 0, mn, L.w + 2, L.h, 2, L.img.iy,
                                            L.img.wy, L.img.P, st));
@@ -1185,16 +1185,16 @@ int run_xpath_gnc(frg_plan* pl, int T, const float* moving, const float* uv_init
             const LevelPlan& L = pl->levels[li];
             const int h = L.h, w = L.w;
             const long long hw = (long long)h * w, mn = (long long)(h + 2) * (w + 2);
-            FRG_LAUNCH(launch_x_resize_h_f(moving, fsz, 1, (long long)W * K, K, T, K, H, pl->tmp, w, L.img.ix,
+            FRG_LAUNCH(launch_x_resize_h_f(moving, fsz, 1, (long long)W * K, K, T, K, H, W, pl->tmp, w, L.img.ix,
                                            L.img.wx, L.img.P, st));
             FRG_LAUNCH(launch_x_resize_v_f(pl->tmp, T, K, H, w, pl->f2, K * hw, hw, w, h, 0, L.img.iy, L.img.wy,
                                            L.img.P, st));
             if (L.top) {
                 if (stage > 0) {
-                    FRG_LAUNCH(launch_x_resize_h_d(flow_out, (long long)H * W * 2, 1, (long long)W * 2, 2, T, 2, H,
+                    FRG_LAUNCH(launch_x_resize_h_d(flow_out, (long long)H * W * 2, 1, (long long)W * 2, 2, T, 2, H, W,
                                                    pl->tmp, w, L.flow.ix, L.flow.wx, L.flow.P, st));
                 } else if (uv_init) {
-                    FRG_LAUNCH(launch_x_resize_h_f(uv_init, 0, 1, (long long)W * 2, 2, T, 2, H, pl->tmp, w, L.flow.ix,
+                    FRG_LAUNCH(launch_x_resize_h_f(uv_init, 0, 1, (long long)W * 2, 2, T, 2, H, W, pl->tmp, w, L.flow.ix,
                                                    L.flow.wx, L.flow.P, st));
                 } else {
                     FRG_CUDA(cudaMemsetAsync(pl->xuv, 0, sizeof(double) * T * 2 * mn, st));
@@ -1204,7 +1204,7 @@ int run_xpath_gnc(frg_plan* pl, int T, const float* moving, const float* uv_init
                                                    L.flow.wy, L.flow.P, st));
             } else {
                 const long long phw = (long long)prev->h * prev->w;
-                FRG_LAUNCH(launch_x_resize_h_d(pl->xacc[cur], 2 * phw, phw, prev->w, 1, T, 2, prev->h, pl->tmp, w,
+                FRG_LAUNCH(launch_x_resize_h_d(pl->xacc[cur], 2 * phw, phw, prev->w, 1, T, 2, prev->h, prev->w, pl->tmp, w,
                                                L.flow.ix, L.flow.wx, L.flow.P, st));
                 FRG_LAUNCH(launch_x_resize_v_d(pl->tmp, T, 2, prev->h, w, pl->xuv, 2 * mn, mn, w + 2, h, 1,
                                                L.flow.iy, L.flow.wy, L.flow.P, st));
@@ -1272,7 +1272,7 @@ int run_xpath(frg_plan* pl, int T, const float* moving, const float* uv_init, do
         const int h = L.h, w = L.w;
         const long long hw = (long long)h * w, mn = (long long)(h + 2) * (w + 2);
         // moving level images (numba typing of the resize)
-        FRG_LAUNCH(launch_x_resize_h_f(moving, fsz, 1, (long long)W * K, K, T, K, H, pl->tmp, w, L.img.ix, L.img.wx,
+        FRG_LAUNCH(launch_x_resize_h_f(moving, fsz, 1, (long long)W * K, K, T, K, H, W, pl->tmp, w, L.img.ix, L.img.wx,
                                        L.img.P, st));
         FRG_LAUNCH(launch_x_resize_v_f(pl->tmp, T, K, H, w, pl->f2, K * hw, hw, w, h, 0, L.img.iy, L.img.wy, L.img.P,
                                        st));
@@ -1281,7 +1281,7 @@ int run_xpath(frg_plan* pl, int T, const float* moving, const float* uv_init, do
         if (L.top) {
             uv_fs = 0;
             if (uv_init) {
-                FRG_LAUNCH(launch_x_resize_h_f(uv_init, 0, 1, (long long)W * 2, 2, 1, 2, H, pl->tmp, w, L.flow.ix,
+                FRG_LAUNCH(launch_x_resize_h_f(uv_init, 0, 1, (long long)W * 2, 2, 1, 2, H, W, pl->tmp, w, L.flow.ix,
                                                L.flow.wx, L.flow.P, st));
                 FRG_LAUNCH(launch_x_resize_v_d(pl->tmp, 1, 2, H, w, pl->xuv, 0, mn, w + 2, h, 1, L.flow.iy, L.flow.wy,
                                                L.flow.P, st));
@@ -1291,7 +1291,7 @@ int run_xpath(frg_plan* pl, int T, const float* moving, const float* uv_init, do
         } else {
             uv_fs = 2 * mn;
             const long long phw = (long long)prev->h * prev->w;
-            FRG_LAUNCH(launch_x_resize_h_d(pl->xacc[cur], 2 * phw, phw, prev->w, 1, T, 2, prev->h, pl->tmp, w,
+            FRG_LAUNCH(launch_x_resize_h_d(pl->xacc[cur], 2 * phw, phw, prev->w, 1, T, 2, prev->h, prev->w, pl->tmp, w,
                                            L.flow.ix, L.flow.wx, L.flow.P, st));
             FRG_LAUNCH(launch_x_resize_v_d(pl->tmp, T, 2, prev->h, w, pl->xuv, 2 * mn, mn, w + 2, h, 1, L.flow.iy,
                                            L.flow.wy, L.flow.P, st));

@@ -9,6 +9,7 @@
 // reference's own rounding when it computes in the reference's precision.
 // Layout: row-major planes, the level arrays with their one-pixel ring
 // (m = h + 2 rows, n = w + 2 columns), like the reference's numpy arrays.
+#include "frg_dfsum.cuh"
 #include "frg_internal.h"
 #include "frg_select.cuh"
 
@@ -22,26 +23,64 @@ __device__ __forceinline__ double dsub(double a, double b) { return __dsub_rn(a,
 __device__ __forceinline__ double dmul(double a, double b) { return __dmul_rn(a, b); }
 __device__ __forceinline__ double ddiv(double a, double b) { return __ddiv_rn(a, b); }
 
-// float -> double on the integer pipe: the conversion instruction runs on the
-// float64 pipe (GB300: 1/64 of the float32 rate), while a normal float's bits
-// map to the double's by a re-biased exponent and a shifted fraction.  Exact;
-// zeros likewise; subnormals, infinities and NaN take the conversion.
-__device__ __forceinline__ double f2d(float f)
-{
-    const unsigned b = __float_as_uint(f);
-    const unsigned e = (b >> 23) & 0xffu;
-    if (e == 0u || e == 0xffu) {
-        if ((b << 1) == 0u) return __hiloint2double((int)(b & 0x80000000u), 0);
-        return (double)f;
-    }
-    const unsigned hi = (b & 0x80000000u) | ((e + 896u) << 20) | ((b >> 3) & 0xfffffu);
-    return __hiloint2double((int)hi, (int)(b << 29));
-}
-
 // ---------------------------------------------------------------------------
 // Resize with numba typing (util/resize_util.py:116-141): float32 input and
 // products, float64 accumulator, float32 result (stored as float or double).
 // ---------------------------------------------------------------------------
+// Horizontal pass.  A block holds RW rows of one plane in shared memory, columns
+// first (pitch RW + 1: no bank conflicts either way), so that a warp's lanes take
+// RW rows of the same 32 / RW output columns: the taps are conflict-free at every
+// scale and the tap table is read once per warp.  The outputs go through shared
+// memory to be stored row by row.  What bounds it is the float64 additions of the
+// general form (64 issue slots each), which DfSum keeps off that pipe.
+constexpr int kRxCols = 64;  // output columns per store tile
+
+template <typename Tin, int RW>
+__global__ void __launch_bounds__(256) kx_resize_h_rows(const Tin* __restrict__ src, long long fs, long long ps, long long rs,
+                                                        long long cs, int n_planes, int ih, int iw, float* __restrict__ dst,
+                                                        int ow, const int32_t* __restrict__ ix,
+                                                        const float* __restrict__ wx, int P, float err)
+{
+    constexpr int pitch = RW + 1, XW = 32 / RW, XB = 8 * XW;  // columns per warp and per block at a time
+    extern __shared__ float sx[];
+    float* tile = sx + (size_t)iw * pitch;  // [RW][kRxCols + 1]
+    const int y0 = blockIdx.x * RW;
+    const int fp = blockIdx.y;
+    const int f = fp / n_planes, pl = fp - f * n_planes;
+    const int nr = min(RW, ih - y0);
+    const Tin* base = src + f * fs + pl * ps + (long long)y0 * rs;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    for (int q = warp; q < nr; q += 8) {
+        const Tin* row = base + (long long)q * rs;
+#pragma unroll 4
+        for (int x = lane; x < iw; x += 32) sx[x * pitch + q] = (float)row[(long long)x * cs];
+    }
+    __syncthreads();
+    const int r = lane % RW;
+    float* out = dst + ((long long)fp * ih + y0) * ow;
+    for (int xt = 0; xt < ow; xt += kRxCols) {
+        const int nx = min(kRxCols, ow - xt);
+        for (int xi = warp * XW + lane / RW; xi < nx && r < nr; xi += XB) {
+            const int32_t* ixr = ix + (long long)(xt + xi) * P;
+            const float* wxr = wx + (long long)(xt + xi) * P;
+            DfSum acc;
+            for (int p = 0; p < P; ++p) acc.add(__fmul_rn(sx[__ldg(ixr + p) * pitch + r], __ldg(wxr + p)));
+            float v;
+            if (!acc.value(err, &v)) {
+                double s = 0.0;
+                for (int p = 0; p < P; ++p) s = dadd(s, f2d(__fmul_rn(sx[ixr[p] * pitch + r], wxr[p])));
+                v = (float)s;
+            }
+            tile[r * (kRxCols + 1) + xi] = v;
+        }
+        __syncthreads();
+        for (int q = warp; q < nr; q += 8)
+            for (int x = lane; x < nx; x += 32) out[(long long)q * ow + xt + x] = tile[q * (kRxCols + 1) + x];
+        __syncthreads();
+    }
+}
+
+// The general form, for rows too long for shared memory.
 template <typename Tin>
 __global__ void kx_resize_h(const Tin* __restrict__ src, long long fs, long long ps, long long rs, long long cs,
                             int n_planes, int ih, float* __restrict__ dst, int ow, const int32_t* __restrict__ ix,
@@ -63,47 +102,102 @@ __global__ void kx_resize_h(const Tin* __restrict__ src, long long fs, long long
 
 // ring: 0 none, 1 edge-replicated ring (add_boundary), 2 zero ring
 // (cv2.copyMakeBorder BORDER_CONSTANT 0, core/optical_flow.py:565-568).
+// Four output rows per thread: their sums are independent, which covers the
+// latency of the loads and of the dependent additions.
+constexpr int kRvx = 4;
+
 template <typename Tout>
 __global__ void kx_resize_v(const float* __restrict__ src, int n_planes, int ih, int ow, Tout* __restrict__ dst,
                             long long fs, long long ps, long long rs, int oh, int ring,
-                            const int32_t* __restrict__ iy, const float* __restrict__ wy, int P)
+                            const int32_t* __restrict__ iy, const float* __restrict__ wy, int P, float err)
 {
     const int pad = ring ? 1 : 0;
     const int xo = blockIdx.x * blockDim.x + threadIdx.x;
-    const int yo = blockIdx.y;
     const int fp = blockIdx.z;
     if (xo >= ow + 2 * pad) return;
     const int f = fp / n_planes, pl = fp - f * n_planes;
-    Tout* out = dst + f * fs + pl * ps + (long long)yo * rs + xo;
-    const bool inside = xo >= pad && xo < ow + pad && yo >= pad && yo < oh + pad;
-    if (!inside && ring == 2) {
-        *out = (Tout)0;
-        return;
-    }
     const int x = xclamp(xo - pad, 0, ow - 1);
-    const int y = xclamp(yo - pad, 0, oh - 1);
     const float* col = src + (long long)fp * ih * ow + x;
-    double s = 0.0;
-    for (int p = 0; p < P; ++p)
-        s = dadd(s, f2d(__fmul_rn(col[(long long)iy[(long long)y * P + p] * ow], wy[(long long)y * P + p])));
-    *out = (Tout)(float)s;
+    const int32_t* iyr[kRvx];
+    const float* wyr[kRvx];
+#pragma unroll
+    for (int q = 0; q < kRvx; ++q) {
+        const int y = xclamp((int)blockIdx.y * kRvx + q - pad, 0, oh - 1);
+        iyr[q] = iy + (long long)y * P;
+        wyr[q] = wy + (long long)y * P;
+    }
+    DfSum acc[kRvx];
+    for (int p = 0; p < P; ++p) {
+#pragma unroll
+        for (int q = 0; q < kRvx; ++q)
+            acc[q].add(__fmul_rn(__ldg(col + (long long)__ldg(iyr[q] + p) * ow), __ldg(wyr[q] + p)));
+    }
+#pragma unroll
+    for (int q = 0; q < kRvx; ++q) {
+        const int yo = blockIdx.y * kRvx + q;
+        if (yo >= oh + 2 * pad) break;
+        float v;
+        if (!acc[q].value(err, &v)) {
+            double s = 0.0;
+            for (int p = 0; p < P; ++p) s = dadd(s, f2d(__fmul_rn(col[(long long)iyr[q][p] * ow], wyr[q][p])));
+            v = (float)s;
+        }
+        const bool inside = xo >= pad && xo < ow + pad && yo >= pad && yo < oh + pad;
+        dst[f * fs + pl * ps + (long long)yo * rs + xo] = !inside && ring == 2 ? (Tout)0 : (Tout)v;
+    }
 }
 
-cudaError_t launch_x_resize_h_f(const float* src, long long fs, long long ps, long long rs, long long cs,
-                                int n_frames, int n_planes, int ih, float* dst, int ow, const int32_t* ix,
-                                const float* wx, int P, cudaStream_t st)
+// Rows per block by the shared memory they take: 32 while two blocks share an SM
+// (rows up to 817 columns), then 16 and 8 (up to 3357 and 6399), else rows read from
+// memory.  Everything but the solver on 100 frames of 512 x 512 x 2, this, the
+// vertical pass and kx_warp included: 54 ms before, 38 ms now.
+template <typename Tin>
+static cudaError_t launch_x_resize_h(const Tin* src, long long fs, long long ps, long long rs, long long cs, int n_frames,
+                                     int n_planes, int ih, int iw, float* dst, int ow, const int32_t* ix,
+                                     const float* wx, int P, cudaStream_t st)
 {
+    const auto bytes = [&](int rw) { return ((size_t)iw * (rw + 1) + (size_t)rw * (kRxCols + 1)) * sizeof(float); };
+    constexpr size_t most = 232448;
+    const auto run = [&](auto kern, int rw) -> cudaError_t {
+        const cudaError_t e = ensure_max_dyn_smem((const void*)kern, (int)most);
+        if (e != cudaSuccess) return e;
+        dim3 grd((ih + rw - 1) / rw, n_frames * n_planes);
+        kern<<<grd, 256, bytes(rw), st>>>(src, fs, ps, rs, cs, n_planes, ih, iw, dst, ow, ix, wx, P, kDfErr(P));
+        return cudaGetLastError();
+    };
+    if (n_frames * n_planes <= 65535) {
+        if (bytes(32) <= most / 2) return run(kx_resize_h_rows<Tin, 32>, 32);
+        if (bytes(16) <= most) return run(kx_resize_h_rows<Tin, 16>, 16);
+        if (bytes(8) <= most) return run(kx_resize_h_rows<Tin, 8>, 8);
+    }
     dim3 blk(128), grd((ow + 127) / 128, ih, n_frames * n_planes);
-    kx_resize_h<float><<<grd, blk, 0, st>>>(src, fs, ps, rs, cs, n_planes, ih, dst, ow, ix, wx, P);
+    kx_resize_h<Tin><<<grd, blk, 0, st>>>(src, fs, ps, rs, cs, n_planes, ih, dst, ow, ix, wx, P);
     return cudaGetLastError();
 }
 
-cudaError_t launch_x_resize_h_d(const double* src, long long fs, long long ps, long long rs, long long cs,
-                                int n_frames, int n_planes, int ih, float* dst, int ow, const int32_t* ix,
+cudaError_t launch_x_resize_h_f(const float* src, long long fs, long long ps, long long rs, long long cs,
+                                int n_frames, int n_planes, int ih, int iw, float* dst, int ow, const int32_t* ix,
                                 const float* wx, int P, cudaStream_t st)
 {
-    dim3 blk(128), grd((ow + 127) / 128, ih, n_frames * n_planes);
-    kx_resize_h<double><<<grd, blk, 0, st>>>(src, fs, ps, rs, cs, n_planes, ih, dst, ow, ix, wx, P);
+    return launch_x_resize_h<float>(src, fs, ps, rs, cs, n_frames, n_planes, ih, iw, dst, ow, ix, wx, P, st);
+}
+
+cudaError_t launch_x_resize_h_d(const double* src, long long fs, long long ps, long long rs, long long cs,
+                                int n_frames, int n_planes, int ih, int iw, float* dst, int ow, const int32_t* ix,
+                                const float* wx, int P, cudaStream_t st)
+{
+    return launch_x_resize_h<double>(src, fs, ps, rs, cs, n_frames, n_planes, ih, iw, dst, ow, ix, wx, P, st);
+}
+
+template <typename Tout>
+static cudaError_t launch_x_resize_v(const float* src, int n_frames, int n_planes, int ih, int ow, Tout* dst,
+                                     long long fs, long long ps, long long rs, int oh, int ring, const int32_t* iy,
+                                     const float* wy, int P, cudaStream_t st)
+{
+    const int owp = ow + (ring ? 2 : 0), ohp = oh + (ring ? 2 : 0);
+    const int bx = owp >= 96 ? 128 : (owp >= 48 ? 64 : 32);
+    dim3 blk(bx), grd((owp + bx - 1) / bx, (ohp + kRvx - 1) / kRvx, n_frames * n_planes);
+    kx_resize_v<Tout><<<grd, blk, 0, st>>>(src, n_planes, ih, ow, dst, fs, ps, rs, oh, ring, iy, wy, P, kDfErr(P));
     return cudaGetLastError();
 }
 
@@ -111,20 +205,14 @@ cudaError_t launch_x_resize_v_f(const float* src, int n_frames, int n_planes, in
                                 long long fs, long long ps, long long rs, int oh, int ring, const int32_t* iy,
                                 const float* wy, int P, cudaStream_t st)
 {
-    const int pad = ring ? 1 : 0;
-    dim3 blk(128), grd((ow + 2 * pad + 127) / 128, oh + 2 * pad, n_frames * n_planes);
-    kx_resize_v<float><<<grd, blk, 0, st>>>(src, n_planes, ih, ow, dst, fs, ps, rs, oh, ring, iy, wy, P);
-    return cudaGetLastError();
+    return launch_x_resize_v<float>(src, n_frames, n_planes, ih, ow, dst, fs, ps, rs, oh, ring, iy, wy, P, st);
 }
 
 cudaError_t launch_x_resize_v_d(const float* src, int n_frames, int n_planes, int ih, int ow, double* dst,
                                 long long fs, long long ps, long long rs, int oh, int ring, const int32_t* iy,
                                 const float* wy, int P, cudaStream_t st)
 {
-    const int pad = ring ? 1 : 0;
-    dim3 blk(128), grd((ow + 2 * pad + 127) / 128, oh + 2 * pad, n_frames * n_planes);
-    kx_resize_v<double><<<grd, blk, 0, st>>>(src, n_planes, ih, ow, dst, fs, ps, rs, oh, ring, iy, wy, P);
-    return cudaGetLastError();
+    return launch_x_resize_v<double>(src, n_frames, n_planes, ih, ow, dst, fs, ps, rs, oh, ring, iy, wy, P, st);
 }
 
 // ---------------------------------------------------------------------------
@@ -147,6 +235,24 @@ struct WarpScale {
     int pow2_col, pow2_row;
 };
 
+// float32(x + u / spacing).  The quotient is replaced by the product with the
+// reciprocal, within two units in the last place of it, unless the sum lies so
+// near the middle between two float32s that this could decide its rounding: 3
+// float64 operations instead of about 12.
+__device__ __forceinline__ float warp_map(int x, double u, double spacing, double per_spacing, int pow2)
+{
+    const double xd = f2d((float)x);
+    const double s = dadd(xd, dmul(u, per_spacing));
+    if (!pow2) {
+        const int hi = __double2hiint(s), e = (hi >> 20) & 0x7ff;
+        // the 29 bits a float32 drops, against their middle: a unit of s is at least a unit of the quotient when
+        // |s| is not far below |u / spacing| (x >= 0, so only for a sum near zero, e small)
+        const int drop = (__double2loint(s) & 0x1fffffff) - 0x10000000;
+        if (e < 1023 || e == 0x7ff || abs(drop) <= 64 + 64 * (x >> 4)) return (float)dadd(xd, ddiv(u, spacing));
+    }
+    return (float)s;
+}
+
 __global__ void kx_warp(const float* __restrict__ f2, const float* __restrict__ f1, const double* __restrict__ u,
                         const double* __restrict__ v, long long uv_fs, int K, int h, int w, WarpScale S,
                         float* __restrict__ out)
@@ -164,8 +270,8 @@ __global__ void kx_warp(const float* __restrict__ f2, const float* __restrict__ 
     const long long hw = (long long)h * w;
     const long long o = (long long)(y + 1) * n + (x + 1);
     const double uu = u[f * uv_fs + o], vv = v[f * uv_fs + o];
-    const float mx = (float)dadd((double)x, S.pow2_col ? dmul(uu, S.i_col) : ddiv(uu, S.h_col));
-    const float my = (float)dadd((double)y, S.pow2_row ? dmul(vv, S.i_row) : ddiv(vv, S.h_row));
+    const float mx = warp_map(x, uu, S.h_col, S.i_col, S.pow2_col);
+    const float my = warp_map(y, vv, S.h_row, S.i_row, S.pow2_row);
     const bool oob = (mx < 0.0f) || (mx >= (float)w) || (my < 0.0f) || (my >= (float)h);
     if (oob) {
         for (int k = 0; k < K; ++k)
@@ -176,29 +282,36 @@ __global__ void kx_warp(const float* __restrict__ f2, const float* __restrict__ 
     const float cy = fminf(fmaxf(my, 0.0f), (float)(h - 1));
     const int X = __float2int_rn(cx * 32.0f), Y = __float2int_rn(cy * 32.0f);
     const int ix = X >> 5, fx = X & 31, iy = Y >> 5, fy = Y & 31;
-    // the 16 weights (float products, exact in double) and the tap offsets, once for all channels
-    double w2[4][4];
+    // the 16 weights (float products) and the tap offsets, once for all channels
+    float w2[4][4];
     long long ro[4];
     int co[4];
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
         const float wyi = s_tab[fy * 4 + i];
 #pragma unroll
-        for (int j = 0; j < 4; ++j) w2[i][j] = f2d(__fmul_rn(wyi, s_tab[fx * 4 + j]));
+        for (int j = 0; j < 4; ++j) w2[i][j] = __fmul_rn(wyi, s_tab[fx * 4 + j]);
         ro[i] = (long long)xclamp(iy - 1 + i, 0, h - 1) * w;
         co[i] = xclamp(ix - 1 + i, 0, w - 1);
     }
     for (int k = 0; k < K; ++k) {
         const float* src = f2 + ((long long)f * K + k) * hw;
-        double acc = 0.0;
+        DfSum acc;
 #pragma unroll
         for (int i = 0; i < 4; ++i)
 #pragma unroll
-            for (int j = 0; j < 4; ++j)
-                // the product of two floats is exact in double, so the fused form rounds as
-                // dadd(acc, dmul(...)) does
-                acc = __fma_rn(f2d(src[ro[i] + co[j]]), w2[i][j], acc);
-        out[((long long)f * K + k) * hw + (long long)y * w + x] = (float)acc;
+            for (int j = 0; j < 4; ++j) acc.add_product(__ldg(src + ro[i] + co[j]), w2[i][j]);
+        float r;
+        if (!acc.value(kDfErr(32), &r)) {
+            double s = 0.0;
+            for (int i = 0; i < 4; ++i)
+                for (int j = 0; j < 4; ++j)
+                    // the product of two floats is exact in double, so the fused form rounds as
+                    // dadd(acc, dmul(...)) does
+                    s = __fma_rn(f2d(src[ro[i] + co[j]]), f2d(__fmul_rn(s_tab[fy * 4 + i], s_tab[fx * 4 + j])), s);
+            r = (float)s;
+        }
+        out[((long long)f * K + k) * hw + (long long)y * w + x] = r;
     }
 }
 

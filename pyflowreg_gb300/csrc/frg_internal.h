@@ -201,10 +201,10 @@ cudaError_t upload_cubic_table(const float* tab128, const float* lin64);
 // FP64 reference-order kernels (frg_exact.cu).
 cudaError_t upload_cubic_table_x(const float* tab128);
 cudaError_t launch_x_resize_h_f(const float* src, long long fs, long long ps, long long rs, long long cs,
-                                int n_frames, int n_planes, int ih, float* dst, int ow, const int32_t* ix,
+                                int n_frames, int n_planes, int ih, int iw, float* dst, int ow, const int32_t* ix,
                                 const float* wx, int P, cudaStream_t st);
 cudaError_t launch_x_resize_h_d(const double* src, long long fs, long long ps, long long rs, long long cs,
-                                int n_frames, int n_planes, int ih, float* dst, int ow, const int32_t* ix,
+                                int n_frames, int n_planes, int ih, int iw, float* dst, int ow, const int32_t* ix,
                                 const float* wx, int P, cudaStream_t st);
 cudaError_t launch_x_resize_v_f(const float* src, int n_frames, int n_planes, int ih, int ow, float* dst,
                                 long long fs, long long ps, long long rs, int oh, int ring, const int32_t* iy,
