@@ -1413,6 +1413,11 @@ int frg_imregister(int n_frames, int height, int width, int channels, const floa
     int rc = ensure_remap_tables();
     if (rc) return rc;
     const long long H = height, W = width, K = channels;
+    if (warp_hwk_supports(n_frames, channels, height, width)) {
+        FRG_LAUNCH(launch_warp_hwk(frames, reference, flow, n_frames, channels, height, width, cubic ? 1 : 0, out,
+                                   (cudaStream_t)stream));
+        return FRG_OK;
+    }
     View f2 = view(frames, H * W * K, 1, W * K, K);
     View f1 = view(reference, 0, 1, W * K, K);
     View u = view(flow, H * W * 2, 0, W * 2, 2);

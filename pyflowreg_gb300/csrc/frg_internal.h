@@ -54,6 +54,10 @@ cudaError_t launch_resize_v(const float* src, int n_frames, int n_planes, int ih
                             int oh, int pad, const int32_t* iy, const float* wy, int P, cudaStream_t st);
 cudaError_t launch_warp(View f2, View f1, View u, View v, int n_frames, int K, int h, int w,
                         float h_col, float h_row, int cubic, ViewW out, cudaStream_t st);
+// launch_warp for interleaved frames (T, h, w, K), flow (T, h, w, 2), unit spacing.
+bool warp_hwk_supports(int n_frames, int K, int h, int w);
+cudaError_t launch_warp_hwk(const float* f2, const float* f1, const float* flow, int n_frames, int K, int h, int w,
+                            int cubic, float* out, cudaStream_t st);
 cudaError_t launch_tensor(View f1, View f2, int n_frames, int K, int h, int w, float hy, float hx,
                           int gray, float* J, long long J_fs, DiagGeom g, cudaStream_t st);
 // launch_tensor plus the smoothness constant (launch_lap) from the same

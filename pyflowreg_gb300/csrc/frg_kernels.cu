@@ -320,6 +320,144 @@ __global__ void k_warp(View f2, View f1, View u, View v, int K, int h, int w, fl
     }
 }
 
+// The same for interleaved frames (T, h, w, K), flow (T, h, w, 2) and unit spacing
+// (the compensation warp), K <= 4: the channels of a tap are one load where they
+// are aligned (VEC), offsets within a frame are 32-bit, and a block covers 32 x 8
+// pixels, whose taps share rows.  The general form issues 16 K loads with 64-bit
+// addresses per pixel.  Same products and sums in the same order.  Bound by memory
+// and L1: 200 frames of 512 x 512 x 2, cubic, 1.14 ms before, 0.51 ms now.  Five and
+// more channels keep the general form.
+template <int K>
+struct Px {
+    float c[K];
+};
+
+template <int K, bool VEC>
+__device__ __forceinline__ Px<K> load_px(const float* __restrict__ p)
+{
+    Px<K> v;
+    if constexpr (VEC && K == 2) {
+        const float2 t = __ldg(reinterpret_cast<const float2*>(p));
+        v.c[0] = t.x;
+        v.c[1] = t.y;
+    } else if constexpr (VEC && K == 4) {
+        const float4 t = __ldg(reinterpret_cast<const float4*>(p));
+        v.c[0] = t.x;
+        v.c[1] = t.y;
+        v.c[2] = t.z;
+        v.c[3] = t.w;
+    } else {
+#pragma unroll
+        for (int k = 0; k < K; ++k) v.c[k] = __ldg(p + k);
+    }
+    return v;
+}
+
+template <int K, bool VEC>
+__device__ __forceinline__ void store_px(float* p, const Px<K>& v)
+{
+    if constexpr (VEC && K == 2) {
+        *reinterpret_cast<float2*>(p) = make_float2(v.c[0], v.c[1]);
+    } else if constexpr (VEC && K == 4) {
+        *reinterpret_cast<float4*>(p) = make_float4(v.c[0], v.c[1], v.c[2], v.c[3]);
+    } else {
+#pragma unroll
+        for (int k = 0; k < K; ++k) p[k] = v.c[k];
+    }
+}
+
+template <int K, bool VEC, bool CUBIC>
+__global__ void __launch_bounds__(256) k_warp_hwk(const float* __restrict__ f2, const float* __restrict__ f1,
+                                                  const float* __restrict__ flow, int h, int w, float* __restrict__ out)
+{
+    constexpr int N = CUBIC ? 4 : 2;
+    __shared__ float s_tab[32 * N];
+    const int tid = threadIdx.y * 32 + threadIdx.x;
+    for (int i = tid; i < 32 * N; i += 256) s_tab[i] = CUBIC ? c_cubic[i] : c_linear[i];
+    __syncthreads();
+    const int x = blockIdx.x * 32 + threadIdx.x, y = blockIdx.y * 8 + threadIdx.y;
+    if (x >= w || y >= h) return;
+    const long long fo = (long long)blockIdx.z * h * w;
+    const int o = y * w + x;
+    const float* wv = flow + (fo + o) * 2;
+    float uu, vv;
+    if constexpr (VEC) {
+        const float2 t = __ldg(reinterpret_cast<const float2*>(wv));
+        uu = t.x;
+        vv = t.y;
+    } else {
+        uu = __ldg(wv);
+        vv = __ldg(wv + 1);
+    }
+    const float mx = __fadd_rn((float)x, uu), my = __fadd_rn((float)y, vv);
+    float* po = out + (fo + o) * K;
+    if ((mx < 0.0f) || (mx >= (float)w) || (my < 0.0f) || (my >= (float)h)) {
+        store_px<K, VEC>(po, load_px<K, VEC>(f1 + (long long)o * K));
+        return;
+    }
+    const int X = __float2int_rn(fminf(fmaxf(mx, 0.0f), (float)(w - 1)) * 32.0f);
+    const int Y = __float2int_rn(fminf(fmaxf(my, 0.0f), (float)(h - 1)) * 32.0f);
+    const int ix = (X >> 5) - (CUBIC ? 1 : 0), fx = X & 31;
+    const int iy = (Y >> 5) - (CUBIC ? 1 : 0), fy = Y & 31;
+    const float* src = f2 + fo * K;
+    int co[N];
+    float wx[N];
+#pragma unroll
+    for (int j = 0; j < N; ++j) {
+        co[j] = clampi(ix + j, 0, w - 1) * K;
+        wx[j] = s_tab[fx * N + j];
+    }
+    Px<K> acc;
+#pragma unroll
+    for (int k = 0; k < K; ++k) acc.c[k] = 0.0f;
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+        const float wy = s_tab[fy * N + i];
+        const float* row = src + clampi(iy + i, 0, h - 1) * (w * K);
+#pragma unroll
+        for (int j = 0; j < N; ++j) {
+            const Px<K> v = load_px<K, VEC>(row + co[j]);
+            const float wt = __fmul_rn(wy, wx[j]);
+#pragma unroll
+            for (int k = 0; k < K; ++k) acc.c[k] = fmaf(v.c[k], wt, acc.c[k]);
+        }
+    }
+    store_px<K, VEC>(po, acc);
+}
+
+template <int K>
+static cudaError_t warp_hwk(const float* f2, const float* f1, const float* flow, int n_frames, int h, int w, int cubic,
+                            float* out, cudaStream_t st)
+{
+    const dim3 blk(32, 8), grd((w + 31) / 32, (h + 7) / 8, n_frames);
+    constexpr uintptr_t px = K == 4 ? 16 : 8;
+    const bool vec = (((uintptr_t)f2 | (uintptr_t)f1 | (uintptr_t)out) & (K % 2 ? 0 : px - 1)) == 0 && ((uintptr_t)flow & 7) == 0;
+    if (cubic)
+        vec ? k_warp_hwk<K, true, true><<<grd, blk, 0, st>>>(f2, f1, flow, h, w, out)
+            : k_warp_hwk<K, false, true><<<grd, blk, 0, st>>>(f2, f1, flow, h, w, out);
+    else
+        vec ? k_warp_hwk<K, true, false><<<grd, blk, 0, st>>>(f2, f1, flow, h, w, out)
+            : k_warp_hwk<K, false, false><<<grd, blk, 0, st>>>(f2, f1, flow, h, w, out);
+    return cudaGetLastError();
+}
+
+bool warp_hwk_supports(int n_frames, int K, int h, int w)
+{
+    return K >= 1 && K <= 4 && (long long)h * w * K < 0x7fffffffLL && (h + 7) / 8 <= 65535 && n_frames <= 65535;
+}
+
+cudaError_t launch_warp_hwk(const float* f2, const float* f1, const float* flow, int n_frames, int K, int h, int w,
+                            int cubic, float* out, cudaStream_t st)
+{
+    switch (K) {
+        case 1: return warp_hwk<1>(f2, f1, flow, n_frames, h, w, cubic, out, st);
+        case 2: return warp_hwk<2>(f2, f1, flow, n_frames, h, w, cubic, out, st);
+        case 3: return warp_hwk<3>(f2, f1, flow, n_frames, h, w, cubic, out, st);
+        case 4: return warp_hwk<4>(f2, f1, flow, n_frames, h, w, cubic, out, st);
+    }
+    return cudaErrorInvalidValue;
+}
+
 cudaError_t launch_warp(View f2, View f1, View u, View v, int n_frames, int K, int h, int w,
                         float h_col, float h_row, int cubic, ViewW out, cudaStream_t st)
 {
