@@ -515,6 +515,18 @@ __global__ void kd_tick(const T* __restrict__ J, const T* __restrict__ W, const 
     c[4 * hw] = B2 - ax * lxv - ay * lyv;
 }
 
+// One pixel of a red-black half-sweep: X and Y are the sums over its horizontal
+// and vertical neighbours, den the two denominators.
+template <typename T>
+__device__ __forceinline__ void rb_update(T duc, T dvc, T den_u, T den_v, T A12, T B1, T B2, T Xu, T Yu, T Xv, T Yv, T ax,
+                                          T ay, T omega, int gs, T& dun, T& dvn)
+{
+    const T nu = -(B1 + A12 * dvc) + ax * Xu + ay * Yu;
+    dun = ((T)1 - omega) * duc + omega * (nu / den_u);
+    const T nv = -(B2 + A12 * (gs ? dun : duc)) + ax * Xv + ay * Yv;
+    dvn = ((T)1 - omega) * dvc + omega * (nv / den_v);
+}
+
 // One red-black half-sweep in place (torch/core/level_solver.py:119-199):
 // pixels with (y + x) % 2 == color move.  gs = 0: du and dv of a moving pixel
 // both from the state before the half-sweep (the torch backend); gs = 1: dv
@@ -542,10 +554,9 @@ __global__ void kd_rb_sweep(int color, const T* __restrict__ coef, const T* __re
     const T B1 = rhs ? -rhs[f * 2 * hw + pc] : c[3 * hw], B2 = rhs ? -rhs[f * 2 * hw + hw + pc] : c[4 * hw];
     const T duc = du[pc], dvc = dv[pc];
     const T sw = ax + ax + ay + ay;
-    const T nu = -(B1 + A12 * dvc) + ax * (du[pL] + du[pR]) + ay * (du[pT] + du[pB]);
-    const T dun = ((T)1 - omega) * duc + omega * (nu / tmax(A11 + sw, eps));
-    const T nv = -(B2 + A12 * (gs ? dun : duc)) + ax * (dv[pL] + dv[pR]) + ay * (dv[pT] + dv[pB]);
-    const T dvn = ((T)1 - omega) * dvc + omega * (nv / tmax(A22 + sw, eps));
+    T dun, dvn;
+    rb_update(duc, dvc, tmax(A11 + sw, eps), tmax(A22 + sw, eps), A12, B1, B2, du[pL] + du[pR], du[pT] + du[pB],
+              dv[pL] + dv[pR], dv[pT] + dv[pB], ax, ay, omega, gs, dun, dvn);
     du[pc] = dun;
     dv[pc] = dvn;
     if (store) {
@@ -1012,6 +1023,127 @@ __global__ void __launch_bounds__(512) kd_rb_adj_window(const T* __restrict__ co
     block_add2(gax, gay, block_slot(galpha));
 }
 
+// All nh half-sweeps of one window in one launch (temporal blocking), with
+// kd_rb_sweep's arithmetic: the same bits.  A CTA owns a TX x TY tile of one frame
+// and computes the pixels within nh - 1 - j of it at half-sweep j, in the order of
+// the ring tables (AdjTable: the tile's own pixels first, then ring by ring), so
+// its threads stay busy as the region shrinks.  The state over the tile grown by
+// nh lies in shared memory, one (du, dv) pair per pixel and colour; a half-sweep
+// moves one colour in place, since it reads the other colour and each pixel
+// itself.  Entry t + q blockDim of either colour is thread t's for the whole
+// window: its coefficients stay in registers, up to NQ pixels per colour.
+// s0 (NULL: zero) is the state before the window, s_out (not s0: tiles read each
+// other's halo) receives it after, hist + j slot the pixels that half-sweep j
+// moved (compressed; NULL: not kept).
+// One launch per half-sweep read the coefficients and the state from memory ten times
+// and left small levels waiting for launches; this one is bound by the shared memory's
+// bandwidth and the halo (1.7 times the pixels).  Training step, 16 frames of 512 x 512,
+// update_lag 5: 53.3 ms before, 47.8 now.
+template <typename T, int NQ, bool EDGE>
+__device__ __forceinline__ void fwd_window_steps(typename Vec2T<T>::type* sS, const T* cf, T* so, T* hist, long long slot,
+                                                 long long f, int x0, int y0, int h, int w, int nh, int Rp1, int n1,
+                                                 const AdjTable& tab, T ax, T ay, T omega, T eps, int gs)
+{
+    using V2 = typename Vec2T<T>::type;
+    const int bd = blockDim.x, t = threadIdx.x;
+    const long long hw = (long long)h * w;
+    const T sw = ax + ax + ay + ay;
+    T den_u[2][NQ], den_v[2][NQ], A12[2][NQ], B1[2][NQ], B2[2][NQ];
+    int at[2][NQ];  // pair in the state buffers, column parity (bit 13), missing neighbours (bits 14-17); -1: none
+#pragma unroll
+    for (int c = 0; c < 2; ++c) {
+        // half-sweep j moves colour j & 1 within nh - 1 - j: colour 0 first
+        const int n = tab.cnt[c][nh - 1 - c];
+#pragma unroll
+        for (int q = 0; q < NQ; ++q) {
+            at[c][q] = -1;
+            den_u[c][q] = den_v[c][q] = (T)1;
+            A12[c][q] = B1[c][q] = B2[c][q] = (T)0;
+            const int i = t + q * bd;
+            if (i >= n) continue;
+            const int2 e = __ldg(tab.e[c] + i);
+            const int gx = x0 + (int)(short)(e.x & 0xffff), gy = y0 + (e.x >> 16);
+            if (EDGE && (gx < 0 || gy < 0 || gx >= w || gy >= h)) continue;
+            int a = ((e.y >> 13) & 0x1fff) | ((e.y >> 26) & 1) << 13;
+            if (EDGE) a |= (gx == 0) << 14 | (gx == w - 1) << 15 | (gy == 0) << 16 | (gy == h - 1) << 17;
+            at[c][q] = a;
+            const T* p = cf + (long long)gy * w + gx;
+            den_u[c][q] = tmax(__ldg(p) + sw, eps);
+            den_v[c][q] = tmax(__ldg(p + hw) + sw, eps);
+            A12[c][q] = __ldg(p + 2 * hw);
+            B1[c][q] = __ldg(p + 3 * hw);
+            B2[c][q] = __ldg(p + 4 * hw);
+        }
+    }
+    cp_async_wait_all();
+    __syncthreads();
+    const int hw2 = (w + 1) >> 1;
+    for (int j2 = 0; j2 < nh; j2 += 2) {
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+            V2* own = sS + c * n1;
+            const V2* oth = sS + (c ^ 1) * n1;
+            const int n_act = tab.cnt[c][nh - 1 - c - j2];
+#pragma unroll
+            for (int q = 0; q < NQ; ++q) {
+                const int a = at[c][q];
+                if (t + q * bd >= n_act || a < 0) continue;
+                const int sb = a & 0x1fff, p = (a >> 13) & 1;
+                const V2 st = own[sb];
+                const V2 sl = EDGE && (a & 1 << 14) ? st : oth[sb - 1 + p], sr = EDGE && (a & 1 << 15) ? st : oth[sb + p];
+                const V2 su = EDGE && (a & 1 << 16) ? st : oth[sb - Rp1], sd = EDGE && (a & 1 << 17) ? st : oth[sb + Rp1];
+                V2 o;
+                rb_update(st.x, st.y, den_u[c][q], den_v[c][q], A12[c][q], B1[c][q], B2[c][q], sl.x + sr.x, su.x + sd.x,
+                          sl.y + sr.y, su.y + sd.y, ax, ay, omega, gs, o.x, o.y);
+                own[sb] = o;
+                if (q == 0 && hist) {  // entry t < blockDim: the tile's own pixel
+                    const int2 e = __ldg(tab.e[c] + t);
+                    const int gx = x0 + (int)(short)(e.x & 0xffff), gy = y0 + (e.x >> 16);
+                    T* d = hist + (long long)(j2 + c) * slot + ((f * 2) * h + gy) * (long long)hw2 + (gx >> 1);
+                    d[0] = o.x;
+                    d[(long long)h * hw2] = o.y;
+                }
+            }
+            __syncthreads();
+        }
+    }
+    // the tile after the window
+#pragma unroll
+    for (int c = 0; c < 2; ++c) {
+        const int2 e = __ldg(tab.e[c] + t);
+        const int gx = x0 + (int)(short)(e.x & 0xffff), gy = y0 + (e.x >> 16);
+        if (gx >= w || gy >= h) continue;
+        const V2 s = sS[c * n1 + ((e.y >> 13) & 0x1fff)];
+        so[(long long)gy * w + gx] = s.x;
+        so[hw + (long long)gy * w + gx] = s.y;
+    }
+}
+
+template <typename T, int NQ>
+__global__ void __launch_bounds__(NQ <= 3 ? 512 : 128, NQ <= 3 && sizeof(T) == 4 ? 2 : 1) kd_rb_window(const T* __restrict__ coef, const T* __restrict__ s0,
+                                                                     T* __restrict__ s_out, T* __restrict__ hist,
+                                                                     long long slot, int h, int w, int nh, int TX, int TY,
+                                                                     AdjTable tab, T ax, T ay, T omega, T eps, int gs)
+{
+    using V2 = typename Vec2T<T>::type;
+    extern __shared__ __align__(16) unsigned char smraw[];
+    V2* const sS = reinterpret_cast<V2*>(smraw);  // colour * n1 + row * Rp1 + pair, over the tile grown by nh + 1
+    const int Rp1 = (TX + 2 * nh + 2) >> 1, Rh1 = TY + 2 * nh + 2, n1 = Rh1 * Rp1;
+    const long long f = blockIdx.z, hw = (long long)h * w;
+    const int x0 = blockIdx.x * TX, y0 = blockIdx.y * TY;
+    const int rx1 = x0 - nh - 1, ry1 = y0 - nh - 1;
+    const float inv_rp1 = 1.0f / (float)Rp1;
+    const StateSlice<T> src{s0, s0 ? 1 : 0};
+    stage_colour<T>(sS, 0, src, f, h, w, 0, rx1, ry1, Rh1, Rp1, inv_rp1);
+    stage_colour<T>(sS + n1, 1, src, f, h, w, 0, rx1, ry1, Rh1, Rp1, inv_rp1);
+    const T* cf = coef + f * 5 * hw;
+    T* so = s_out + f * 2 * hw;
+    if (rx1 < 0 || ry1 < 0 || rx1 + 2 * Rp1 > w || ry1 + Rh1 > h)
+        fwd_window_steps<T, NQ, true>(sS, cf, so, hist, slot, f, x0, y0, h, w, nh, Rp1, n1, tab, ax, ay, omega, eps, gs);
+    else
+        fwd_window_steps<T, NQ, false>(sS, cf, so, hist, slot, f, x0, y0, h, w, nh, Rp1, n1, tab, ax, ay, omega, eps, gs);
+}
+
 // The closing gather of a window: pixels of colour `color` (which did not move
 // in the window's first half-sweep) add w * a_0 of their moving neighbours.
 template <typename T>
@@ -1469,6 +1601,36 @@ cudaError_t rb_adj_window(const T* coef, const T* s0, const T* hist, long long s
     return cudaGetLastError();
 }
 
+// Pixels of one colour per thread of kd_rb_window (the tile grown by nh - 1);
+// 0: more than its registers take (or no tile).  Such windows (update_lag over 6)
+// run half-sweep by half-sweep: a tile whose coefficients spill, or whose halo holds
+// more pixels than the tile four times over, gains nothing.
+int rb_window_pixels(int nh, int tile)
+{
+    if ((tile != 16 && tile != 32) || nh < 2) return 0;
+    const int n = (tile + 2 * nh - 2) * (tile + 2 * nh - 2) / 2, bd = tile * tile / 2, q = (n + bd - 1) / bd;
+    return q <= (tile == 32 ? 3 : 6) ? q : 0;
+}
+
+// nh half-sweeps of a window in one launch (rb_window_pixels(nh, tile) > 0).
+template <typename T>
+cudaError_t rb_window(const T* coef, const T* s0, T* s_out, T* hist, long long slot, int F, int h, int w, int nh, int tile,
+                      const AdjTable& tab, double ax, double ay, double omega, double eps, int gs, cudaStream_t st)
+{
+    const int bd = tile * tile / 2, n1 = (tile + 2 * nh + 2) * ((tile + 2 * nh + 2) / 2);
+    const dim3 grid((w + tile - 1) / tile, (h + tile - 1) / tile, F);
+    const auto run = [&](auto kern) -> cudaError_t {
+        const cudaError_t e = ensure_max_dyn_smem((const void*)kern, (int)kAdjWindowSmem);
+        if (e != cudaSuccess) return e;
+        kern<<<grid, bd, 4 * (size_t)n1 * sizeof(T), st>>>(coef, s0, s_out, hist, slot, h, w, nh, tile, tile, tab, (T)ax,
+                                                            (T)ay, (T)omega, (T)eps, gs);
+        return cudaGetLastError();
+    };
+    const int q = rb_window_pixels(nh, tile);
+    if (q == 0) return cudaErrorInvalidValue;
+    return q <= 3 ? run(kd_rb_window<T, 3>) : run(kd_rb_window<T, 6>);
+}
+
 cudaError_t reduce_slots(double* part, int F, long long n_slots, double* galpha, cudaStream_t st)
 {
     kd_reduce_slots<<<F, 256, 0, st>>>(part, n_slots, galpha);
@@ -1534,6 +1696,8 @@ cudaError_t median_adj(const T* d, const T* g, int32_t* am, int F, int h, int w,
                                  double, double, double, T*, T*, cudaStream_t);                                 \
     template cudaError_t rb_sweep<T>(int, const T*, const T*, T*, T*, int, int, int, double, double, double,     \
                                      double, int, cudaStream_t);                                                \
+    template cudaError_t rb_window<T>(const T*, const T*, T*, T*, long long, int, int, int, int, int,            \
+                                      const AdjTable&, double, double, double, double, int, cudaStream_t);      \
     template cudaError_t implicit_assemble<T>(const T*, const T*, int, int, int, T*, double, double, double*,    \
                                               cudaStream_t);                                                    \
     template cudaError_t rb_adj_step<T>(int, const T*, const T*, const T*, const T*, T*, const T*, T*, int, int, \

@@ -205,6 +205,15 @@ int make_adj_tables(frg_diff_plan* pl)
     return FRG_OK;
 }
 
+// The ring table of a window of n_half half-sweeps that kd_rb_window can run; NULL: none.
+const frg::diff::AdjTable* window_table(const frg_diff_plan* pl, int n_half)
+{
+    if (!pl->adj_tile || !frg::diff::rb_window_pixels(n_half, pl->adj_tile)) return nullptr;
+    for (int q = 0; q < 2; ++q)
+        if (pl->adj_nh[q] == n_half) return &pl->adj_tab[q];
+    return nullptr;
+}
+
 // Uploads forward tables (ix/wx over out_w, iy/wy over out_h) and their inverses.
 int put_tables(frg_diff_plan* pl, DTab* d, const int32_t* ix, const float* wx, const int32_t* iy, const float* wy)
 {
@@ -296,29 +305,72 @@ int run_forward(frg_diff_plan* pl, int F, const T* fixed, const T* moving, const
         L.ax = (pl->alpha_x * L.scale) / (L.h_col * L.h_col);
         L.ay = (pl->alpha_y * L.scale) / (L.h_row * L.h_row);
         T* s = (T*)pl->st;
-        DCUDA(cudaMemsetAsync(s, 0, (size_t)F * 2 * hw * sizeof(T), st));
+        const size_t plane2 = (size_t)F * 2 * hw;
         const size_t slot = (size_t)F * 2 * h * ((w + 1) / 2);
-        for (int it = 0; it < I; ++it) {
-            if (it % lag == 0) {
-                const int k = it / lag;
-                T* ck = k > 0 ? (T*)L.ck_ticks + (size_t)(k - 1) * F * 2 * hw : nullptr;
-                // with stored sweeps each window's coefficients are kept too (the backward reads them)
+        bool fused = true;
+        for (int k = 0; k < pl->n_ticks; ++k) fused = fused && window_table(pl, 2 * std::min(lag, I - k * lag)) != nullptr;
+        if (fused) {
+            // one launch per window, from one tick's state straight into the next one's checkpoint
+            for (int k = 0; k < pl->n_ticks; ++k) {
+                const int n_half = 2 * std::min(lag, I - k * lag);
+                const bool last = k == pl->n_ticks - 1;
+                const T* s0 = k > 0 ? (const T*)L.ck_ticks + (size_t)(k - 1) * plane2 : nullptr;
+                T* s1 = !last ? (T*)L.ck_ticks + (size_t)k * plane2 : pl->store_sweeps ? (T*)L.ck_final : (T*)pl->st;
                 coef = pl->store_sweeps ? (T*)L.ck_coef + (size_t)k * F * 5 * hw : (T*)pl->coef;
-                DLAUNCH(1, tick<T>(J, (const T*)L.Wl, k > 0 ? s : (const T*)nullptr, uv, F, K, h, w, pl->a_data, kEps,
-                                   L.ax, L.ay, coef, ck, st));
+                DLAUNCH(1, tick<T>(J, (const T*)L.Wl, s0, uv, F, K, h, w, pl->a_data, kEps, L.ax, L.ay, coef, (T*)nullptr,
+                                   st));
+                DLAUNCH(1, rb_window<T>(coef, s0, s1, pl->store_sweeps ? (T*)L.ck_sweeps + (size_t)(2 * k * lag) * slot : nullptr,
+                                        (long long)slot, F, h, w, n_half, pl->adj_tile, *window_table(pl, n_half), L.ax,
+                                        L.ay, om, kEps, pl->gs, st));
+                s = s1;
             }
-            for (int c = 0; c < 2; ++c) {
-                T* store = pl->store_sweeps ? (T*)L.ck_sweeps + (size_t)(2 * it + c) * slot : nullptr;
-                DLAUNCH(1, rb_sweep<T>(c, coef, (const T*)nullptr, s, store, F, h, w, L.ax, L.ay, om, kEps, pl->gs, st));
+        } else {
+            DCUDA(cudaMemsetAsync(s, 0, plane2 * sizeof(T), st));
+            for (int it = 0; it < I; ++it) {
+                if (it % lag == 0) {
+                    const int k = it / lag;
+                    T* ck = k > 0 ? (T*)L.ck_ticks + (size_t)(k - 1) * plane2 : nullptr;
+                    // with stored sweeps each window's coefficients are kept too (the backward reads them)
+                    coef = pl->store_sweeps ? (T*)L.ck_coef + (size_t)k * F * 5 * hw : (T*)pl->coef;
+                    DLAUNCH(1, tick<T>(J, (const T*)L.Wl, k > 0 ? s : (const T*)nullptr, uv, F, K, h, w, pl->a_data, kEps,
+                                       L.ax, L.ay, coef, ck, st));
+                }
+                for (int c = 0; c < 2; ++c) {
+                    T* store = pl->store_sweeps ? (T*)L.ck_sweeps + (size_t)(2 * it + c) * slot : nullptr;
+                    DLAUNCH(1, rb_sweep<T>(c, coef, (const T*)nullptr, s, store, F, h, w, L.ax, L.ay, om, kEps, pl->gs, st));
+                }
             }
+            if (pl->store_sweeps)
+                DCUDA(cudaMemcpyAsync(L.ck_final, s, plane2 * sizeof(T), cudaMemcpyDeviceToDevice, st));
         }
-        if (pl->store_sweeps)
-            DCUDA(cudaMemcpyAsync(L.ck_final, s, (size_t)F * 2 * hw * sizeof(T), cudaMemcpyDeviceToDevice, st));
         DLAUNCH(1, median_add<T>(s, uv, (T*)pl->uvc[cur ^ 1], F, h, w, std::min(h, w) > 5 ? 1 : 0, st));
         cur ^= 1;
         prev = &L;
     }
     DCUDA(cudaMemcpyAsync(flow_out, pl->uvc[cur], (size_t)F * 2 * H * W * sizeof(T), cudaMemcpyDeviceToDevice, st));
+    return FRG_OK;
+}
+
+// The half-sweeps of a window again, from s0 (NULL: zero) into s.
+template <typename T>
+int rerun_window(frg_diff_plan* pl, const DLevel& L, int F, const T* coef, const T* s0, T* s, T* hist, size_t slot, int n_half,
+                 cudaStream_t st)
+{
+    using namespace frg::diff;
+    const double om = pl->p.omega;
+    if (const AdjTable* tb = window_table(pl, n_half)) {
+        DLAUNCH(1, rb_window<T>(coef, s0, s, hist, (long long)slot, F, L.h, L.w, n_half, pl->adj_tile, *tb, L.ax, L.ay, om,
+                                kEps, pl->gs, st));
+        return FRG_OK;
+    }
+    const size_t bytes = (size_t)F * 2 * L.h * L.w * sizeof(T);
+    if (s0)
+        DCUDA(cudaMemcpyAsync(s, s0, bytes, cudaMemcpyDeviceToDevice, st));
+    else
+        DCUDA(cudaMemsetAsync(s, 0, bytes, st));
+    for (int j = 0; j < n_half; ++j)
+        DLAUNCH(1, rb_sweep<T>(j & 1, coef, (const T*)nullptr, s, hist ? hist + (size_t)j * slot : nullptr, F, L.h, L.w, L.ax,
+                               L.ay, om, kEps, pl->gs, st));
     return FRG_OK;
 }
 
@@ -380,13 +432,7 @@ int run_backward(frg_diff_plan* pl, const T* g_flow, T* g_fixed, T* g_moving, do
             DLAUNCH(1, tick<T>(J, Wl, s0, uv, F, K, h, w, pl->a_data, kEps, L.ax, L.ay, coef, (T*)nullptr, st));
             const T* fin = (const T*)L.ck_final;
             if (!pl->store_sweeps) {
-                if (s0)
-                    DCUDA(cudaMemcpyAsync(s, s0, plane2 * es, cudaMemcpyDeviceToDevice, st));
-                else
-                    DCUDA(cudaMemsetAsync(s, 0, plane2 * es, st));
-                for (int j = 0; j < 2 * n_it; ++j)
-                    DLAUNCH(1, rb_sweep<T>(j & 1, coef, (const T*)nullptr, s, (T*)nullptr, F, h, w, L.ax, L.ay, om, kEps,
-                                           pl->gs, st));
+                if (const int rc = rerun_window<T>(pl, L, F, coef, s0, s, nullptr, slot, 2 * n_it, st)) return rc;
                 fin = s;
             }
             T* g = (T*)pl->lam[1];
@@ -415,13 +461,7 @@ int run_backward(frg_diff_plan* pl, const T* g_flow, T* g_fixed, T* g_moving, do
                 base = (T*)L.ck_sweeps + (size_t)(2 * start) * slot;
             } else {
                 base = (T*)pl->states;
-                if (s0)
-                    DCUDA(cudaMemcpyAsync(s, s0, plane2 * es, cudaMemcpyDeviceToDevice, st));
-                else
-                    DCUDA(cudaMemsetAsync(s, 0, plane2 * es, st));
-                for (int j = 0; j < n_half; ++j)
-                    DLAUNCH(1, rb_sweep<T>(j & 1, coef, (const T*)nullptr, s, base + (size_t)j * slot, F, h, w, L.ax,
-                                           L.ay, om, kEps, pl->gs, st));
+                if (const int rc = rerun_window<T>(pl, L, F, coef, s0, s, base, slot, n_half, st)) return rc;
             }
             if (k == pl->n_ticks - 1) {
                 const T* fin = pl->store_sweeps ? (const T*)L.ck_final : s;

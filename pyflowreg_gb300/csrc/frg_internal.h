@@ -384,6 +384,10 @@ struct AdjTable {
 };
 bool build_adj_table(int tile, int nh, std::vector<int2>& e0, std::vector<int2>& e1, int cnt[2][kAdjMaxNh + 1]);
 int rb_adj_window_tile(int nh, int elem_bytes);
+int rb_window_pixels(int nh, int tile);
+template <typename T>
+cudaError_t rb_window(const T* coef, const T* s0, T* s_out, T* hist, long long slot, int F, int h, int w, int nh, int tile,
+                      const AdjTable& tab, double ax, double ay, double omega, double eps, int gs, cudaStream_t st);
 template <typename T>
 cudaError_t rb_adj_window(const T* coef, const T* s0, const T* hist, long long slot, const T* lam_in, T* lam_out,
                           int F, int h, int w, int nh, int tile, const AdjTable& tab, double ax, double ay,
