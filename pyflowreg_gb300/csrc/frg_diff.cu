@@ -776,13 +776,12 @@ __device__ __forceinline__ void adj_px_load(AdjPx<T>& q, int2 e, int x0, int y0,
     q.self = EDGE ? ax * (T)((hasL ? 0 : 1) + (hasR ? 0 : 1)) + ay * (T)((hasT ? 0 : 1) + (hasB ? 0 : 1)) : (T)0;
 }
 
-// The step itself; with ACC the coefficient gradients go to g and the
-// (sx, sy)-scaled alpha gradients to (gax, gay).  Writes lam and (au, av).
+// The step's arithmetic: the pixel's new lam and (au, av); with ACC the coefficient
+// gradients go to g and the (sx, sy)-scaled alpha gradients to (gax, gay).
 template <typename T, bool ACC>
-__device__ __forceinline__ void adj_px_step(const AdjPx<T>& q, T ax, T ay, T omega, int gs, const AdjPlanes<T>& P,
-                                            T (&g)[5], T& gax, T& gay, T sx, T sy)
+__device__ __forceinline__ void adj_px_math(const AdjPx<T>& q, T ax, T ay, T omega, int gs, typename Vec2T<T>::type& nl,
+                                            typename Vec2T<T>::type& na, T (&g)[5], T& gax, T& gay, T sx, T sy)
 {
-    using V2 = typename Vec2T<T>::type;
     const T A12 = q.c0.x, B1 = q.c0.y, B2 = q.c1.x, idu = q.c1.y, idv = q.idv;
     const T duc = q.st.x, dvc = q.st.y;
     const T av = omega * q.lam.y * idv;
@@ -792,14 +791,10 @@ __device__ __forceinline__ void adj_px_step(const AdjPx<T>& q, T ax, T ay, T ome
     const T dun = ((T)1 - omega) * duc + omega * ru;
     const T du_for_v = gs ? dun : duc;
     const T rv = (-(B2 + A12 * du_for_v) + ax * q.Xdv + ay * q.Ydv) * idv;
-    V2 nl;
     nl.x = ((T)1 - omega) * lue + q.self * au - (gs ? (T)0 : A12 * av);
     nl.y = ((T)1 - omega) * q.lam.y - A12 * au + q.self * av;
-    P.L[q.li] = nl;
-    V2 na;
     na.x = au;
     na.y = av;
-    P.A[q.li] = na;
     if (ACC) {
         g[0] -= au * ru;
         g[1] -= av * rv;
@@ -810,6 +805,17 @@ __device__ __forceinline__ void adj_px_step(const AdjPx<T>& q, T ax, T ay, T ome
         gax += (au * q.Xdu + av * q.Xdv - rr) * sx;
         gay += (au * q.Ydu + av * q.Ydv - rr) * sy;
     }
+}
+
+// The step on the shared-memory planes: writes lam and (au, av).
+template <typename T, bool ACC>
+__device__ __forceinline__ void adj_px_step(const AdjPx<T>& q, T ax, T ay, T omega, int gs, const AdjPlanes<T>& P,
+                                            T (&g)[5], T& gax, T& gay, T sx, T sy)
+{
+    typename Vec2T<T>::type nl, na;
+    adj_px_math<T, ACC>(q, ax, ay, omega, gs, nl, na, g, gax, gay, sx, sy);
+    P.L[q.li] = nl;
+    P.A[q.li] = na;
 }
 
 // The steps of one window, from half-sweep nh - 1 down to 0 (see
@@ -1142,6 +1148,207 @@ __global__ void __launch_bounds__(NQ <= 3 ? 512 : 128, NQ <= 3 && sizeof(T) == 4
         fwd_window_steps<T, NQ, true>(sS, cf, so, hist, slot, f, x0, y0, h, w, nh, Rp1, n1, tab, ax, ay, omega, eps, gs);
     else
         fwd_window_steps<T, NQ, false>(sS, cf, so, hist, slot, f, x0, y0, h, w, nh, Rp1, n1, tab, ax, ay, omega, eps, gs);
+}
+
+// The same with a pixel's coefficients, lam and gradients in its thread's registers:
+// entry t + q blockDim of either colour's ring table is thread t's for the whole window
+// (NQ of each colour at most).  Shared memory holds what neighbours read: the latest (au,
+// av) and the states, both one word pair per pixel and colour over the tile grown by
+// nh + 1.  The form above moves a pixel's coefficients, lam and place in the table
+// through shared memory at every step as well, whose bandwidth bounds it.  The places
+// that a thread copies states from are worked out once.  16 frames, a window of ten
+// half-sweeps at 512 x 512: 635 us before, 450 now; at 23 x 23: 19.5 and 15.4.
+template <typename T, int NQ, bool EDGE>
+__device__ __forceinline__ void adj_regs_steps(typename Vec2T<T>::type* sS, typename Vec2T<T>::type* sA, const T* cf,
+                                               const T* s0, const T* hist, long long slot, const T* lam_in, T* lam_out,
+                                               T* gcoef, long long f, int x0, int y0, int h, int w, int nh, int rx1, int ry1,
+                                               int Rh1, int Rp1, float inv_rp1, const AdjTable& tab, T ax, T ay, T omega,
+                                               T eps, int gs, T tsx, T tsy, T& gax, T& gay)
+{
+    using V2 = typename Vec2T<T>::type;
+    const int bd = blockDim.x, t = threadIdx.x, n1 = Rh1 * Rp1, hw2 = (w + 1) >> 1;
+    const long long hw = (long long)h * w;
+    const T sw = ax + ax + ay + ay;
+    T idu[2][NQ], idv[2][NQ], A12[2][NQ], B1[2][NQ], B2[2][NQ], lu[2][NQ], lv[2][NQ];
+    int at[2][NQ];  // as in fwd_window_steps
+    T g[2][5];
+#pragma unroll
+    for (int c = 0; c < 2; ++c) {
+        // half-sweep j moves colour j & 1 within j + 1 of the tile
+        const int n = tab.cnt[c][nh - 1 + c];
+#pragma unroll
+        for (int i = 0; i < 5; ++i) g[c][i] = (T)0;
+#pragma unroll
+        for (int q = 0; q < NQ; ++q) {
+            at[c][q] = -1;
+            idu[c][q] = idv[c][q] = A12[c][q] = B1[c][q] = B2[c][q] = lu[c][q] = lv[c][q] = (T)0;
+            const int i = t + q * bd;
+            if (i >= n) continue;
+            const int2 e = __ldg(tab.e[c] + i);
+            const int gx = x0 + (int)(short)(e.x & 0xffff), gy = y0 + (e.x >> 16);
+            if (EDGE && (gx < 0 || gy < 0 || gx >= w || gy >= h)) continue;
+            int a = ((e.y >> 13) & 0x1fff) | ((e.y >> 26) & 1) << 13;
+            if (EDGE) a |= (gx == 0) << 14 | (gx == w - 1) << 15 | (gy == 0) << 16 | (gy == h - 1) << 17;
+            at[c][q] = a;
+            const long long o = (long long)gy * w + gx;
+            idu[c][q] = __ldg(cf + o);
+            idv[c][q] = __ldg(cf + hw + o);
+            A12[c][q] = __ldg(cf + 2 * hw + o);
+            B1[c][q] = __ldg(cf + 3 * hw + o);
+            B2[c][q] = __ldg(cf + 4 * hw + o);
+            lu[c][q] = __ldg(lam_in + o);
+            lv[c][q] = __ldg(lam_in + hw + o);
+        }
+    }
+#pragma unroll
+    for (int c = 0; c < 2; ++c)
+#pragma unroll
+        for (int q = 0; q < NQ; ++q) {
+            idu[c][q] = (T)1 / tmax(idu[c][q] + sw, eps);
+            idv[c][q] = (T)1 / tmax(idv[c][q] + sw, eps);
+        }
+    cp_async_wait_all();
+    __syncthreads();
+    // the pixels of a colour's state that this thread copies, in the compressed planes; -1: outside the level
+    int from[2][NQ];
+#pragma unroll
+    for (int c = 0; c < 2; ++c)
+#pragma unroll
+        for (int q = 0; q < NQ; ++q) {
+            const int i = t + q * bd, row = (int)(((float)i + 0.5f) * inv_rp1), gy = ry1 + row;
+            const int gx = rx1 + 2 * (i - row * Rp1) + ((c - rx1 - gy) & 1);
+            from[c][q] = i < n1 && gy >= 0 && gy < h && gx >= 0 && gx < w ? gy * hw2 + (gx >> 1) : -1;
+        }
+    const T* hf = hist + f * 2 * h * hw2;
+    const long long hp = (long long)h * hw2;
+    // the four neighbours' words of pixel a in a plane of the other colour
+    auto gather = [&](int a, const V2* A, T& su, T& sv) {
+        const int sb = a & 0x1fff, p = (a >> 13) & 1;
+        if (!(EDGE && (a & 1 << 14))) { const V2 v = A[sb - 1 + p]; su += ax * v.x; sv += ax * v.y; }
+        if (!(EDGE && (a & 1 << 15))) { const V2 v = A[sb + p]; su += ax * v.x; sv += ax * v.y; }
+        if (!(EDGE && (a & 1 << 16))) { const V2 v = A[sb - Rp1]; su += ay * v.x; sv += ay * v.y; }
+        if (!(EDGE && (a & 1 << 17))) { const V2 v = A[sb + Rp1]; su += ay * v.x; sv += ay * v.y; }
+    };
+    int cur[2] = {0, 0};
+    for (int j2 = nh - 2; j2 >= 0; j2 -= 2) {
+#pragma unroll
+        for (int c = 1; c >= 0; --c) {
+            const int j = j2 + c;
+            const V2* own = sS + (c * 2 + cur[c]) * n1;
+            const V2* oth = sS + ((c ^ 1) * 2 + cur[c ^ 1]) * n1;
+            // the other colour's state for step j - 1 (its values after j - 3), one step ahead
+            if (j >= 3) {
+                const T* src = hf + (long long)(j - 3) * slot;
+                V2* dst = sS + ((c ^ 1) * 2 + (cur[c ^ 1] ^ 1)) * n1 + t;
+#pragma unroll
+                for (int q = 0; q < NQ; ++q)
+                    if (from[c ^ 1][q] >= 0) {
+                        T* d = reinterpret_cast<T*>(dst + q * bd);
+                        cp_async_el(d, src + from[c ^ 1][q]);
+                        cp_async_el(d + 1, src + hp + from[c ^ 1][q]);
+                    }
+                cp_async_commit();
+            } else if (j >= 1) {
+                stage_colour<T>(sS + ((c ^ 1) * 2 + (cur[c ^ 1] ^ 1)) * n1, c ^ 1, StateSlice<T>{s0, s0 ? 1 : 0}, f, h, w, hw2,
+                                rx1, ry1, Rh1, Rp1, inv_rp1);
+            }
+            const int n_act = tab.cnt[c][j + 1];
+#pragma unroll
+            for (int q = 0; q < NQ; ++q) {
+                const int a = at[c][q];
+                if (t + q * bd >= n_act || a < 0) continue;
+                const int sb = a & 0x1fff, p = (a >> 13) & 1;
+                AdjPx<T> x;
+                x.lam.x = lu[c][q];
+                x.lam.y = lv[c][q];
+                if (j < nh - 1) {
+                    T su = 0, sv = 0;
+                    gather(a, sA + (c ^ 1) * n1, su, sv);
+                    x.lam.x += su;
+                    x.lam.y += sv;
+                }
+                x.c0.x = A12[c][q];
+                x.c0.y = B1[c][q];
+                x.c1.x = B2[c][q];
+                x.c1.y = idu[c][q];
+                x.idv = idv[c][q];
+                x.st = own[sb];
+                const bool eL = EDGE && (a & 1 << 14), eR = EDGE && (a & 1 << 15), eT = EDGE && (a & 1 << 16),
+                           eB = EDGE && (a & 1 << 17);
+                const V2 sl = eL ? x.st : oth[sb - 1 + p], sr = eR ? x.st : oth[sb + p];
+                const V2 su = eT ? x.st : oth[sb - Rp1], sd = eB ? x.st : oth[sb + Rp1];
+                x.Xdu = sl.x + sr.x;
+                x.Ydu = su.x + sd.x;
+                x.Xdv = sl.y + sr.y;
+                x.Ydv = su.y + sd.y;
+                x.self = EDGE ? ax * (T)((int)eL + (int)eR) + ay * (T)((int)eT + (int)eB) : (T)0;
+                V2 nl, na;
+                if (q == 0) {  // entry t < blockDim: the tile's own pixel
+                    adj_px_math<T, true>(x, ax, ay, omega, gs, nl, na, g[c], gax, gay, tsx, tsy);
+                } else {
+                    T dummy[5], da = 0, db = 0;
+                    adj_px_math<T, false>(x, ax, ay, omega, gs, nl, na, dummy, da, db, tsx, tsy);
+                }
+                lu[c][q] = nl.x;
+                lv[c][q] = nl.y;
+                sA[c * n1 + sb] = na;
+            }
+            cp_async_wait_all();
+            __syncthreads();
+            cur[c ^ 1] ^= 1;
+        }
+    }
+    // the closing gather (colour 1), then the tile's lam and coefficient gradients
+#pragma unroll
+    for (int c = 0; c < 2; ++c) {
+        if (at[c][0] < 0) continue;
+        const int2 e = __ldg(tab.e[c] + t);
+        const long long o = (long long)(y0 + (e.x >> 16)) * w + x0 + (int)(short)(e.x & 0xffff);
+        T su = 0, sv = 0;
+        if (c == 1) gather(at[1][0], sA, su, sv);
+        lam_out[o] = c == 1 ? lu[c][0] + su : lu[c][0];
+        lam_out[hw + o] = c == 1 ? lv[c][0] + sv : lv[c][0];
+#pragma unroll
+        for (int i = 0; i < 5; ++i) gcoef[i * hw + o] = g[c][i];
+    }
+}
+
+template <typename T, int NQ>
+__global__ void __launch_bounds__(512) kd_rb_adj_regs(const T* __restrict__ coef, const T* __restrict__ s0,
+                                                      const T* __restrict__ hist, long long slot,
+                                                      const T* __restrict__ lam_in, T* __restrict__ lam_out, int h, int w,
+                                                      int nh, int TX, int TY, AdjTable tab, T ax, T ay, T omega, T eps,
+                                                      int gs, T* __restrict__ gcoef, double sx, double sy,
+                                                      double* __restrict__ galpha)
+{
+    using V2 = typename Vec2T<T>::type;
+    extern __shared__ __align__(16) unsigned char smraw[];
+    const int Rp1 = (TX + 2 * nh + 2) >> 1, Rh1 = TY + 2 * nh + 2, n1 = Rh1 * Rp1;
+    V2* const sS = reinterpret_cast<V2*>(smraw);  // (colour * 2 + buffer) * n1
+    V2* const sA = sS + 4 * n1;                   // colour * n1
+    const long long f = blockIdx.z, hw = (long long)h * w;
+    const int x0 = blockIdx.x * TX, y0 = blockIdx.y * TY;
+    const int rx1 = x0 - nh - 1, ry1 = y0 - nh - 1;
+    const float inv_rp1 = 1.0f / (float)Rp1;
+    auto slice = [&](int k) -> StateSlice<T> {
+        if (k >= 0) return StateSlice<T>{hist + (long long)k * slot, 2};
+        return StateSlice<T>{s0, s0 ? 1 : 0};
+    };
+    // the states before half-sweep nh - 1 (colour 1): colour 1 after nh - 3, colour 0 after nh - 2
+    stage_colour<T>(sS + 2 * n1, 1, slice(nh - 3), f, h, w, (w + 1) >> 1, rx1, ry1, Rh1, Rp1, inv_rp1);
+    stage_colour<T>(sS, 0, slice(nh - 2), f, h, w, (w + 1) >> 1, rx1, ry1, Rh1, Rp1, inv_rp1);
+    T gax = 0, gay = 0;
+    const T* cf = coef + f * 5 * hw;
+    const T* li = lam_in + f * 2 * hw;
+    T* lo = lam_out + f * 2 * hw;
+    T* gc = gcoef + f * 5 * hw;
+    if (rx1 < 0 || ry1 < 0 || rx1 + 2 * Rp1 > w || ry1 + Rh1 > h)
+        adj_regs_steps<T, NQ, true>(sS, sA, cf, s0, hist, slot, li, lo, gc, f, x0, y0, h, w, nh, rx1, ry1, Rh1, Rp1, inv_rp1,
+                                    tab, ax, ay, omega, eps, gs, (T)sx, (T)sy, gax, gay);
+    else
+        adj_regs_steps<T, NQ, false>(sS, sA, cf, s0, hist, slot, li, lo, gc, f, x0, y0, h, w, nh, rx1, ry1, Rh1, Rp1, inv_rp1,
+                                     tab, ax, ay, omega, eps, gs, (T)sx, (T)sy, gax, gay);
+    block_add2(gax, gay, block_slot(galpha));
 }
 
 // The closing gather of a window: pixels of colour `color` (which did not move
@@ -1592,6 +1799,21 @@ cudaError_t rb_adj_window(const T* coef, const T* s0, const T* hist, long long s
 {
     const size_t bytes = adj_window_smem(tile, nh, (int)sizeof(T));
     if ((tile != 16 && tile != 32) || nh < 1 || bytes > kAdjWindowSmem) return cudaErrorInvalidValue;
+    // float32 windows whose pixels, two words of state each, are at most three per thread and colour: the form with the
+    // coefficients in registers.  float64 would spill (128 registers), longer windows too.
+    if constexpr (sizeof(T) == 4) {
+        if (tile == 32 && (nh & 1) == 0 && (tile + 2 * nh + 2) * (tile + 2 * nh + 2) / 2 <= 3 * (tile * tile / 2)) {
+            auto kern = kd_rb_adj_regs<T, 3>;
+            const cudaError_t e = ensure_max_dyn_smem((const void*)kern, (int)kAdjWindowSmem);
+            if (e != cudaSuccess) return e;
+            const int edge = tile + 2 * nh + 2;
+            const dim3 grid((w + tile - 1) / tile, (h + tile - 1) / tile, F);
+            kern<<<grid, tile * tile / 2, 6 * (size_t)edge * edge * sizeof(T), st>>>(
+                coef, s0, hist, slot, lam_in, lam_out, h, w, nh, tile, tile, tab, (T)ax, (T)ay, (T)omega, (T)eps, gs, gcoef, sx, sy,
+                galpha);
+            return cudaGetLastError();
+        }
+    }
     const cudaError_t e = ensure_max_dyn_smem((const void*)kd_rb_adj_window<T>, (int)kAdjWindowSmem);
     if (e != cudaSuccess) return e;
     const dim3 grid((w + tile - 1) / tile, (h + tile - 1) / tile, F);
@@ -1603,8 +1825,7 @@ cudaError_t rb_adj_window(const T* coef, const T* s0, const T* hist, long long s
 
 // Pixels of one colour per thread of kd_rb_window (the tile grown by nh - 1);
 // 0: more than its registers take (or no tile).  Such windows (update_lag over 6)
-// run half-sweep by half-sweep: a tile whose coefficients spill, or whose halo holds
-// more pixels than the tile four times over, gains nothing.
+// run half-sweep by half-sweep.
 int rb_window_pixels(int nh, int tile)
 {
     if ((tile != 16 && tile != 32) || nh < 2) return 0;
