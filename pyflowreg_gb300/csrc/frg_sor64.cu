@@ -36,7 +36,7 @@
 // instructions at 64 to 76 clocks over four pipes, about 2000 clocks of a
 // measured 2300 per step.
 #include "frg_dpow.cuh"
-#include "frg_split.cuh"
+#include "frg_split_sor.cuh"
 
 #include <algorithm>
 #include <cmath>
@@ -154,42 +154,9 @@ constexpr int kG64 = kGMax;        // iterations pipelined per pass, as a templa
 constexpr int kMaxStrips64 = 16;   // cluster size (over 8: the non-portable opt-in)
 constexpr int kPortableStrips = 8;
 
-struct Sor64Args {
-    const double* J;    // [6][K][D*P] per frame: J11, J22, J33 + 1e-5, 2 J12, 2 J13, 2 J23
-    long long J_fs;
-    const double* W;    // [2][K][D*P] per frame, W then W * a_data (W_fs 0: shared by all frames)
-    long long W_fs;
-    const double* lap;  // [2][D*P]: the u- and v-parts of the smoothness numerator from u, v
-    long long lap_fs;
-    double* coef;       // [5][D*P]: folded coefficients of passes that continue a group
-    long long coef_fs;
-    double* du;         // [D*P] pass-to-pass state
-    double* dv;
-    long long st_fs;
-    double* out_du;     // final pass: du, dv at out + r * out_rs + c (frame stride out_fs)
-    double* out_dv;
-    long long out_fs;
-    int out_rs;
-    DiagGeom g;
-    double wa, wb;      // smoothness weights of the row neighbours (y) and the column neighbours (x)
-    double wsum;        // ((wx + wx) + wy) + wy, the reference's order
-    double omega, one_m_omega;
+struct Sor64Args : SplitArgs<double> {
     double a_m1[kMaxK];  // a_data - 1
     PowTab64 pw[kMaxK];  // the power's table per channel (null table: the general power)
-    int nc;              // CTAs per frame
-    int ahead;           // steps a fold may run ahead: at most the columns of a row less one
-    const int* marks;    // frames to compute (fx_recompute); null: all
-    int ring;            // the final pass also writes the border copies around the output
-};
-
-// The fold's inputs of one pixel (J, W, lap; or the stored coefficients),
-// loaded at the start of the step whose end folds them: a step of float64
-// work takes several microseconds, far longer than the loads.
-template <int K>
-struct FoldIn64 {
-    double j[6 * K];
-    double w[K];
-    double lu, lv;
 };
 
 struct Coef64 {
@@ -236,7 +203,7 @@ __device__ __forceinline__ double omega_over(double omega, double den)
 // uses them; the sums over them are then twice the sums above, exactly, and
 // A12 = sum / 2, BU = fma(-1/2, sum, lap_u) give the same bits.
 template <int K>
-__device__ __forceinline__ Coef64 fold64(const Sor64Args& A, int pk, const FoldIn64<K>& r, double du, double dv)
+__device__ __forceinline__ Coef64 fold64(const Sor64Args& A, int pk, const FoldIn<double, K>& r, double du, double dv)
 {
     Coef64 o;
     if (pk & kPkCoef) {
@@ -298,267 +265,25 @@ __device__ __forceinline__ double2 sor_point64(double2 c, double2 up, double2 dn
     return make_double2(dun, dvn);
 }
 
-// Shared memory of a CTA of M strips of 32 rows: ring double2[3][kRingSlots][32 M + 1]
-// (A12, BU | BV, iDu | state, whose last row is the next strip's first) and
-// double[kRingSlots][32 M + 1] (iDv) | iteration buffers double2[G][3][32 M + 2] |
-// mbarriers: full[M][kRingSlots], empty[M][kRingSlots], edge[2 parities] | a word
-// for waits that ran out.
-template <int M>
-struct Split64Smem {
-    static constexpr int rows = 32 * M;
-    static constexpr int plane = kRingSlots * (rows + 1);
-    static constexpr int buf = rows + 2;
-    static constexpr size_t bytes = ((size_t)3 * plane + (size_t)kGMax * 3 * buf) * sizeof(double2) +
-                                    (size_t)plane * sizeof(double) + (size_t)(2 * M * kRingSlots + 2) * 8 + 16;
+template <int K_>
+struct Ar64 {
+    static constexpr int K = K_;
+    static constexpr bool tick_weights = true, rings = true;
+    using T = double;
+    using T2 = double2;
+    using Args = Sor64Args;
+    using Coef = Coef64;
+    __device__ static double2 pair(double x, double y) { return make_double2(x, y); }
+    __device__ static Coef64 fold(const Args& A, int pk, const FoldIn<double, K>& r, double du, double dv)
+    {
+        return fold64<K>(A, pk, r, du, dv);
+    }
+    __device__ static double2 point(const Args& A, double2 c, double2 up, double2 dn, double2 lf, double2 rt, double2 ca,
+                                    double2 cb, double iDv)
+    {
+        return sor_point64(c, up, dn, lf, rt, ca, cb, iDv, A.wa, A.wb, A.one_m_omega);
+    }
 };
-
-// The chained solver, one step of the wavefront divided among warps (see the
-// file's head).  MB: CTAs per SM that the registers are to allow.
-template <int K, int M, int NU, int FC, int MB>
-__global__ void __launch_bounds__(32 * SplitRoles<M, NU, FC>::warps, MB) k_sor_split64(Sor64Args A, PassTable T)
-{
-    using SM = Split64Smem<M>;
-    using Roles = SplitRoles<M, NU, FC>;
-    constexpr int G = kG64;
-    constexpr int S = kRingSlots;
-    constexpr int ROWS = SM::rows, PL = SM::plane, SR = ROWS + 1, BUF = SM::buf, WU = Roles::WU;
-    extern __shared__ __align__(16) double sm64[];
-    double2* ring = reinterpret_cast<double2*>(sm64);  // planes kA, kB, kS
-    constexpr int kA = 0, kB = PL, kS = 2 * PL;
-    double2* bufs = ring + 3 * PL;
-    double* ringd = reinterpret_cast<double*>(bufs + G * 3 * BUF);
-    unsigned long long* bars = reinterpret_cast<unsigned long long*>(ringd + PL);
-    int* gave_up = reinterpret_cast<int*>(bars + 2 * M * S + 2);
-    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
-    const int nc = A.nc;
-    const int cta = nc > 1 ? (int)(blockIdx.x % nc) : 0;
-    const int f = nc > 1 ? (int)(blockIdx.x / nc) : (int)blockIdx.x;
-    if (A.marks && !fx_recompute(A.marks[f])) return;  // the same for every CTA of a cluster
-    const bool update = warp < WU;
-    const int strip = (update ? warp : Roles::fold(warp)) % M;
-    const int row = strip * 32 + lane;  // in the CTA
-    const int r = cta * ROWS + row;     // in the level
-    const DiagGeom g = A.g;
-    const int P = g.P, h = g.h, w = g.w;
-    const int pl = g.D * P;
-    const bool row_ok = r < h;
-    const bool above = cta > 0, below = cta + 1 < nc;  // other CTAs of the frame
-    auto full_bar = [&](int st, int slot) { return smem_addr(bars + st * S + slot); };
-    auto empty_bar = [&](int st, int slot) { return smem_addr(bars + M * S + st * S + slot); };
-    auto edge_bar = [&](int par) { return smem_addr(bars + 2 * M * S + par); };
-    // bytes a step's edge rows bring: every iteration's from above, all but the last one's from below
-    const unsigned edge_bytes = (above ? G * sizeof(double2) : 0) + (below ? (G - 1) * sizeof(double2) : 0);
-    if (t == 0) {
-        *gave_up = 0;
-        for (int i = 0; i < 2 * M * S + 2; ++i) mbar_init(smem_addr(bars + i), 1);
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-        if (nc > 1)
-            for (int par = 0; par < 2; ++par) mbar_expect(edge_bar(par), edge_bytes);
-    }
-    auto sync_all = [&]() {
-        if (nc > 1)
-            cooperative_groups::this_cluster().sync();
-        else
-            __syncthreads();
-    };
-    sync_all();
-
-    double* odu = A.out_du + f * A.out_fs;
-    double* odv = A.out_dv + f * A.out_fs;
-    int total = 0;
-    for (int p = 0; p < T.n; ++p) total += pass_span(w, T.pk[p]);
-    const int nsteps = total + h - 1;
-    bool dead = false;
-    Cursor cur;
-    cur.init(T, w);
-
-    if (!update && warp != Roles::wait && warp != Roles::idle) {
-        // ------------------------------------------------------------ fold
-        const int fj = Roles::fold(warp) / M;
-        const double* Jr = A.J + f * A.J_fs + r;
-        const double* Wr = A.W + f * A.W_fs + r;
-        const double* lapr = A.lap + f * A.lap_fs + r;
-        double* coefr = A.coef + f * A.coef_fs + r;
-        const double* dur = A.du + f * A.st_fs + r;
-        const double* dvr = A.dv + f * A.st_fs + r;
-        // the first row's state also goes to the CTA above, as the row below its last one
-        const bool sends = above && row == 0;
-        unsigned halo = smem_addr(ring + kS + ROWS), halo_bar = full_bar(M - 1, 0);
-        if (sends) {
-            asm("mapa.shared::cluster.u32 %0, %0, %1;" : "+r"(halo) : "r"(cta - 1));
-            asm("mapa.shared::cluster.u32 %0, %0, %1;" : "+r"(halo_bar) : "r"(cta - 1));
-        }
-        const bool gets = below && strip == M - 1;
-        for (int s = fj; s < nsteps; s += FC) {
-            const int slot = (unsigned)s % S;
-            // the update has finished step s - ahead: the slot is free, and the states stored up to then can be read
-            if (s >= A.ahead) mbar_wait(empty_bar(strip, slot), ((unsigned)(s - A.ahead) / S) & 1, dead);
-            cur.advance(T, w, s - r);
-            const int c = s - r - cur.start, pk = cur.pk, o = (r + c) * P;
-            const bool in_level = row_ok && (unsigned)c < (unsigned)w;
-            FoldIn64<K> in;
-            double su = 0.0, sv = 0.0;
-            if (in_level) {
-                if (!(pk & kPkZero)) {
-                    su = dur[o];
-                    sv = dvr[o];
-                }
-                if (pk & kPkCoef) {
-#pragma unroll
-                    for (int q = 0; q < 5; ++q) in.j[q] = coefr[q * pl + o];
-                } else {
-#pragma unroll
-                    for (int q = 0; q < 6 * K; ++q) in.j[q] = __ldg(Jr + q * pl + o);
-                    const double* wsrc = (pk & kPkTick) ? Wr + K * pl : Wr;  // W * a_data on a tick
-#pragma unroll
-                    for (int k = 0; k < K; ++k) in.w[k] = __ldg(wsrc + k * pl + o);
-                    in.lu = __ldg(lapr + o);
-                    in.lv = __ldg(lapr + pl + o);
-                }
-            }
-            const int ro = slot * SR + row;
-            const double2 st = make_double2(su, sv);
-            ring[kS + ro] = st;
-            st_async_if(sends, halo + slot * SR * 16, *reinterpret_cast<const int4*>(&st), halo_bar + slot * 8);
-            if (in_level) {
-                const Coef64 cf = fold64<K>(A, pk, in, su, sv);
-                if (pk & kPkStore) {
-                    coefr[o] = cf.A12;
-                    coefr[pl + o] = cf.BU;
-                    coefr[2 * pl + o] = cf.BV;
-                    coefr[3 * pl + o] = cf.iDu;
-                    coefr[4 * pl + o] = cf.iDv;
-                }
-                ring[kA + ro] = make_double2(cf.A12, cf.BU);
-                ring[kB + ro] = make_double2(cf.BV, cf.iDu);
-                ringd[ro] = cf.iDv;
-            }
-            __syncwarp();
-            if (lane == 0) {
-                if (gets)
-                    mbar_arrive_expect(full_bar(strip, slot), sizeof(double2));
-                else
-                    mbar_arrive(full_bar(strip, slot));
-            }
-        }
-    } else if (warp == Roles::wait) {
-        // ------------------------------------------------------------ wait
-        // What a step needs from other warps and CTAs is awaited here, beside the update of the
-        // step before: the fold's slots and the neighbouring CTAs' edge rows.
-        auto wait_full = [&](int s) {
-            if (s < nsteps)
-                for (int st = 0; st < M; ++st) mbar_wait(full_bar(st, (unsigned)s % S), ((unsigned)s / S) & 1, dead);
-        };
-        wait_full(0);
-        wait_full(1);
-        asm volatile("bar.sync 1, %0;" ::"n"(32 * (WU + 1)) : "memory");
-        for (int s = 0; s < nsteps; ++s) {
-            wait_full(s + 2);
-            if (nc > 1 && s + 1 < nsteps) {
-                mbar_wait(edge_bar(s & 1), ((unsigned)s >> 1) & 1, dead);
-                if (lane == 0) mbar_expect(edge_bar(s & 1), edge_bytes);
-            }
-            asm volatile("bar.sync 1, %0;" ::"n"(32 * (WU + 1)) : "memory");
-            // step s is done by every iteration: the slot of the pixel that entered 2 (G - 1) steps ago is free
-            if (lane < M) mbar_arrive(empty_bar(lane, (unsigned)(s + A.ahead) % S));
-        }
-    } else if (update) {
-        // ---------------------------------------------------------- update
-        constexpr int NG = (G + NU - 1) / NU;  // iterations of this warp: g0, g0 + NU, ...
-        const int g0 = warp / M;
-        const double omm = A.one_m_omega, wa = A.wa, wb = A.wb;
-        const bool first_row = r == 0, last_row = r == h - 1;
-        // edge rows to the neighbouring CTAs: the last row's values go below, the first row's above
-        const bool send_dn = below && row == ROWS - 1, send_up = above && row == 0;
-        unsigned ebuf = smem_addr(bufs + (send_dn ? 0 : ROWS + 1)), ebar = edge_bar(0);
-        if (send_dn || send_up) {
-            const int peer = send_dn ? cta + 1 : cta - 1;
-            asm("mapa.shared::cluster.u32 %0, %0, %1;" : "+r"(ebuf) : "r"(peer));
-            asm("mapa.shared::cluster.u32 %0, %0, %1;" : "+r"(ebar) : "r"(peer));
-        }
-        double2 lf[NG], own[NG];  // the values left of the current pixel, and the pixel's own
-        double2* myring = ring + row;
-        int co[NG];               // ring offset of iteration i's pixel
-#pragma unroll
-        for (int i = 0; i < NG; ++i) {
-            lf[i] = own[i] = make_double2(0.0, 0.0);
-            co[i] = (unsigned)(-2 * (g0 + i * NU)) % S * SR;
-        }
-        auto next_slot = [&](int o) { return o == (S - 1) * SR ? 0 : o + SR; };
-        int so = 0, so1 = SR;                // state slots of steps s and s + 1
-        int b0 = 0, b1 = 2 * BUF, b2 = BUF;  // the buffers of steps s, s - 1, s - 2
-        double* sdu = A.du + f * A.st_fs + r;
-        double* sdv = A.dv + f * A.st_fs + r;
-        asm volatile("bar.sync 1, %0;" ::"n"(32 * (WU + 1)) : "memory");
-        if (g0 == 0) own[0] = myring[kS];
-        for (int s = 0; s < nsteps; ++s) {
-            cur.advance(T, w, s - r);
-            const int Gp = cur.pk >> 8;
-            const int d0 = s - cur.start;  // the diagonal of iteration 0's pixel
-#pragma unroll
-            for (int i = 0; i < NG; ++i) {
-                const int gi = g0 + i * NU;
-                if (gi >= G) break;
-                const int c = d0 - r - 2 * gi;
-                // where the iteration before has its values: of this pixel (before), and what it wrote
-                // in the last step: the right neighbour, and in the next row the lower one (prev)
-                const double2* base = gi == 0 ? myring + kS : bufs + (gi - 1) * 3 * BUF + row + 1;
-                const double2* before = base + (gi == 0 ? so : b2);
-                const double2* prev = base + (gi == 0 ? so1 : b1);
-                double2* mybuf = bufs + gi * 3 * BUF + row + 1;
-                // border copies: the neighbour outside is the pixel's own value before the update
-                const double2 rt = *(c == w - 1 ? before : prev);
-                double2 n = lf[i];
-                const bool valid = gi < Gp && row_ok && (unsigned)c < (unsigned)w;
-                if (valid) {
-                    const double2 dn = *(last_row ? before : prev + 1);
-                    const double2 up = *(first_row ? before : mybuf + b1 - 1);
-                    const double2 ow = own[i];
-                    n = sor_point64(ow, up, dn, c == 0 ? ow : lf[i], rt, myring[kA + co[i]], myring[kB + co[i]],
-                                    ringd[row + co[i]], wa, wb, omm);
-                    if (gi == Gp - 1) {
-                        if (cur.p < T.n - 1) {
-                            sdu[(d0 - 2 * gi) * P] = n.x;
-                            sdv[(d0 - 2 * gi) * P] = n.y;
-                        } else {
-                            const long long o = (long long)r * A.out_rs + c;
-                            odu[o] = n.x;
-                            odv[o] = n.y;
-                            if (A.ring && (c == 0 || c == w - 1 || r == 0 || r == h - 1))
-                                for (int yr = r == 0 ? -1 : 0; yr <= (r == h - 1 ? 1 : 0); ++yr)
-                                    for (int xc = c == 0 ? -1 : 0; xc <= (c == w - 1 ? 1 : 0); ++xc)
-                                        if (yr | xc) {
-                                            odu[o + (long long)yr * A.out_rs + xc] = ow.x;
-                                            odv[o + (long long)yr * A.out_rs + xc] = ow.y;
-                                        }
-                        }
-                    }
-                }
-                mybuf[b0] = n;
-                st_async_if((send_dn || (send_up && gi + 1 < G)) && s + 1 < nsteps, ebuf + (gi * 3 * BUF + b0) * 16,
-                            *reinterpret_cast<const int4*>(&n), ebar + (s & 1) * 8);
-                lf[i] = n;
-                own[i] = rt;
-                co[i] = next_slot(co[i]);
-            }
-            asm volatile("bar.sync 1, %0;" ::"n"(32 * (WU + 1)) : "memory");
-            so = so1;
-            so1 = next_slot(so1);
-            const int b = b2;
-            b2 = b1;
-            b1 = b0;
-            b0 = b;
-        }
-    }
-    if (dead) *gave_up = 1;
-    __syncthreads();
-    if (*gave_up && row_ok && update)  // a wait ran out: the rows' result is void
-        for (int c = warp / M; c < w; c += NU) {
-            const long long o = (long long)r * A.out_rs + c;
-            odu[o] = odv[o] = __longlong_as_double(0x7ff8000000000000ll);
-        }
-    sync_all();  // no CTA leaves while another may still write into its shared memory
-}
 
 // Row strips of a level with at most `rows` rows per CTA (256, 128 or 64).
 void split64(const DiagGeom& g, int rows, int* nc, int* nt)
@@ -568,43 +293,26 @@ void split64(const DiagGeom& g, int rows, int* nc, int* nt)
     *nt = ((g.P + n - 1) / n + 31) / 32 * 32;
 }
 
-template <int K, int M, int NU, int FC, int MB>
-cudaError_t run_split64(Sor64Args A, const PassTable& T, int n_frames, cudaStream_t st)
-{
-    constexpr size_t smem = Split64Smem<M>::bytes;
-    A.ahead = std::min(kFoldAhead, A.g.w - 1);
-    A.nc = (A.g.P / 32 + M - 1) / M;
-    if (A.nc > kMaxSplitCluster || (long long)n_frames * A.nc > 0x7fffffffLL) return cudaErrorInvalidValue;
-    auto kern = k_sor_split64<K, M, NU, FC, MB>;
-    cudaError_t e = ensure_max_dyn_smem((const void*)kern, (int)smem);
-    if (e != cudaSuccess) return e;
-    if (A.nc > kPortableStrips && (e = ensure_nonportable_clusters((const void*)kern)) != cudaSuccess) return e;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)(n_frames * A.nc));
-    cfg.blockDim = dim3(32 * SplitRoles<M, NU, FC>::warps);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = st;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = (unsigned)A.nc;
-    at[0].val.clusterDim.y = 1;
-    at[0].val.clusterDim.z = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = A.nc > 1 ? 1 : 0;
-    return cudaLaunchKernelEx(&cfg, kern, A, T);
-}
-
-// Warps per 32 rows by what the launch has to fill: at most one CTA per SM, all
-// registers; more, two CTAs per SM (100 frames 291 ms against 364).  Levels over
-// 512 and 1024 rows need 64 and 128 rows per CTA.  Other counts of update and
-// fold warps measured within 3 % or worse.
+// Rows per CTA and warps per 32 rows.  32 rows while the launch has at most one CTA
+// per SM (all registers).  With more CTAs what counts is how a frame's cluster packs
+// into the GPCs (14 to 20 SMs): 16 CTAs of 32 rows leave 40 of 152 SMs without a CTA,
+// 8 CTAs of 64 rows none, while 13 CTAs of 32 rows fill 143 SMs and 7 of 64 rows,
+// one strip of which is empty, 136.  So the shorter of both by `cost`; at 100 frames
+// of 512 x 512 x 2: 71 ms with 64 rows against 91, and over all smaller levels 182
+// against 162.  Levels over 512 and 1024 rows need 64 and 128 rows; 16 frames of
+// 1024 x 1024 x 2: 222 ms with two CTAs of fewer warps per SM, 239 with one.
 template <int K>
-cudaError_t run_split64_m(const Sor64Args& A, const PassTable& T, int m, int n_frames, int n_sms, cudaStream_t st)
+cudaError_t run_split64_m(const Sor64Args& A, const PassTable& T, int m, int n_frames, int dev, int n_sms, cudaStream_t st)
 {
-    if (m == 4) return run_split64<K, 4, 3, 3, 1>(A, T, n_frames, st);
-    if (m == 2) return run_split64<K, 2, 5, 6, 1>(A, T, n_frames, st);
-    if ((long long)n_frames * (A.g.P / 32) <= n_sms) return run_split64<K, 1, 5, 6, 1>(A, T, n_frames, st);
-    return run_split64<K, 1, 5, 6, 2>(A, T, n_frames, st);
+    using One = SplitLaunch<Ar64<K>, 1, 5, 6, 1>;
+    using Two = SplitLaunch<Ar64<K>, 1, 5, 6, 2>;
+    using Tall = SplitLaunch<Ar64<K>, 2, 3, 4, 2>;
+    if (m == 4) return SplitLaunch<Ar64<K>, 4, 2, 4, 1>::run(A, T, n_frames, st);
+    if (m == 2 && (long long)n_frames * Tall::ctas(A.g) <= n_sms) return SplitLaunch<Ar64<K>, 2, 5, 6, 1>::run(A, T, n_frames, st);
+    if (m == 2) return Tall::run(A, T, n_frames, st);
+    if ((long long)n_frames * One::ctas(A.g) <= n_sms) return One::run(A, T, n_frames, st);
+    return Tall::cost(dev, A.g, n_frames) < Two::cost(dev, A.g, n_frames) ? Tall::run(A, T, n_frames, st)
+                                                                          : Two::run(A, T, n_frames, st);
 }
 
 }  // namespace
@@ -684,10 +392,10 @@ cudaError_t launch_sor_chain64(const double* J, long long J_fs, const double* W,
     int m = strips <= kMaxSplitCluster ? 1 : (strips <= 2 * kMaxSplitCluster ? 2 : 4);
     if (rows >= 64) m = std::max(m, rows >= 128 ? 4 : 2);
     switch (K) {
-        case 1: return run_split64_m<1>(A, T, m, n_frames, n_sms, st);
-        case 2: return run_split64_m<2>(A, T, m, n_frames, n_sms, st);
-        case 3: return run_split64_m<3>(A, T, m, n_frames, n_sms, st);
-        default: return run_split64_m<4>(A, T, m, n_frames, n_sms, st);
+        case 1: return run_split64_m<1>(A, T, m, n_frames, dev, n_sms, st);
+        case 2: return run_split64_m<2>(A, T, m, n_frames, dev, n_sms, st);
+        case 3: return run_split64_m<3>(A, T, m, n_frames, dev, n_sms, st);
+        default: return run_split64_m<4>(A, T, m, n_frames, dev, n_sms, st);
     }
 }
 

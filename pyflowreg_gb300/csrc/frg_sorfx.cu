@@ -1,6 +1,6 @@
 // Exact-order chained SOR of a single level (the level_solver seam) with the
 // updates in 64-bit fixed point, as exact as float64 but not its bits.  The
-// pyramid keeps k_sor_split64: there a last-bit difference moves psi by up to
+// pyramid keeps k_sor_split: there a last-bit difference moves psi by up to
 // 1e-7 where the residual cancels, and among the 1e8 pixels of a batch some 1/32
 // px warp sample of the next level comes out another one.
 //
@@ -36,9 +36,9 @@
 // marks the frame, and so does a level whose result is nowhere above 2^42 units
 // but not zero (so small that a float64 state would hold more bits).  Marked
 // frames are solved again by a second launch with a wider format, and what that
-// one marks by k_sor_split64.
+// one marks by k_sor_split.
 //
-// Schedule: that of k_sor_split64 (row r's local time is tau = s - r; pixel
+// Schedule: that of k_sor_split (row r's local time is tau = s - r; pixel
 // (r, c) of pipelined iteration gi of a pass is updated at tau = start + c +
 // 2 gi), with the work split over specialised warps.  Every 32 rows have NU
 // update warps, which share the five pipelined iterations, and FC fold warps,

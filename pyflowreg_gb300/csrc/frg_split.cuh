@@ -1,5 +1,4 @@
-// What the split forms of the chained float64 SOR share (k_sor_split64,
-// k_sor_fx): the work of 32 rows is divided among update warps (one per
+// What the split forms of the chained SOR share (k_sor_split, k_sor_fx): the work of 32 rows is divided among update warps (one per
 // pipelined iteration), fold warps that run ahead of them and one warp that waits
 // for both and for the neighbouring CTAs; rings, barriers and the place of a row
 // in the chain of passes.
@@ -66,6 +65,19 @@ __device__ __forceinline__ void st_async_if(bool p, unsigned addr, int4 v, unsig
                  : "memory");
 }
 
+__device__ __forceinline__ void st_async_if(bool p, unsigned addr, double2 v, unsigned mb)
+{
+    st_async_if(p, addr, *reinterpret_cast<const int4*>(&v), mb);
+}
+
+__device__ __forceinline__ void st_async_if(bool p, unsigned addr, float2 v, unsigned mb)
+{
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.s32 p, %4, 0;\n\t"
+                 "@p st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v2.b32 [%0], {%1, %2}, [%3];\n\t}" ::"r"(addr),
+                 "r"(__float_as_int(v.x)), "r"(__float_as_int(v.y)), "r"(mb), "r"((int)p)
+                 : "memory");
+}
+
 __device__ __forceinline__ bool mbar_test(unsigned mb, unsigned parity)
 {
     unsigned ok;
@@ -102,10 +114,11 @@ __device__ __forceinline__ int pass_span(int w, int pk)
 template <int M, int NU, int FC>
 struct SplitRoles {
     static constexpr int WU = M * NU;
-    static constexpr bool spread = M == 1 && NU == 5;
+    static constexpr bool spread = M == 1 && NU == 5 && FC >= 3;  // warp 8 waits: it has to be there
     static constexpr int wait = spread ? 8 : WU;
     static constexpr int idle = spread && FC > 6 ? 12 : -1;
     static constexpr int warps = WU + 1 + M * FC + (idle >= 0 ? 1 : 0);
+    static_assert(FC >= 1 && NU >= 1 && NU <= kGMax && wait < warps && idle < warps && warps <= 32, "every role has its warps");
     __device__ static int fold(int warp) { return spread ? warp - (warp < 8 ? 5 : (warp < 12 ? 6 : 7)) : warp - WU - 1; }
 };
 
