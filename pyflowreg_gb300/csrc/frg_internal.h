@@ -107,14 +107,13 @@ cudaError_t launch_sor_regs(const float* J, long long J_fs, const float* W, long
                             int n_frames, int K, DiagGeom g, int G, int mode, int store_coef, const float* a_data,
                             float wx, float wy, float omega, cudaStream_t st, float* out_du = nullptr,
                             float* out_dv = nullptr, long long out_fs = 0);
-// Every pass of a level in one launch of the rows-in-registers SOR (frg_sor.cu,
-// k_sor_chain): a row starts its next pass as soon as it has finished the
+// Every pass of a level in one launch (frg_sor.cu: k_sor_split, or k_sor_chain for
+// levels over 2048 rows): a row starts its next pass as soon as it has finished the
 // current one, so the passes follow each other without restarting the
 // wavefront.  Pass p is the launch_sor_regs pass (G, mode, store_coef); the
 // level's last pass writes out_du/out_dv when given.  Every level
-// launch_sor_regs serves (levels over 512 rows as clusters of row strips),
-// w >= 3, at most kMaxChain passes; bit-identical to one launch_sor_regs call
-// per pass.
+// launch_sor_regs serves (in clusters of row strips), w >= 3, at most kMaxChain
+// passes; bit-identical to one launch_sor_regs call per pass.
 constexpr int kMaxChain = 64;
 struct ChainPass {
     int G, mode, store_coef;
@@ -139,7 +138,7 @@ struct PowTab64 {
 // Host: fills tab (kPowTabN entries) and the series constants of *pt for
 // exponent b (pt->t untouched); false, with nothing written, when |b| > 1.
 bool make_pow_table(double b, double2* tab, PowTab64* pt);
-// The chained SOR in float64 (frg_sor64.cu, k_sor_split64): the schedule of
+// The chained SOR in float64 (frg_sor64.cu, k_sor_split): the schedule of
 // launch_sor_chain with float64 state, coefficients and arithmetic (the parity
 // precision).  J [6][K][D*P] (J11, J22, J33 + 1e-5, 2 J12, 2 J13, 2 J23), W
 // [2][K][D*P] (W, then W * a_data), lap [2][D*P], coef [5][D*P] and the state

@@ -19,6 +19,7 @@
 #include "frg_internal.h"
 
 #include <cooperative_groups.h>
+#include "frg_split_sor.cuh"
 
 namespace frg {
 
@@ -97,8 +98,8 @@ struct Coef {
     float A12, BU, BV, iDu, iDv;
 };
 
-template <int K>
-__device__ __forceinline__ Coef fold_m(const SorArgs& A, int mode, const Raw<K>& r)
+template <int K, class Args>
+__device__ __forceinline__ Coef fold_m(const Args& A, int mode, const Raw<K>& r)
 {
     Coef o;
     if (mode < 0) {
@@ -547,8 +548,6 @@ struct ChainTable {
     int n;
     int pk[kMaxChain];
 };
-
-constexpr int kPkZero = 1, kPkTick = 2, kPkCoef = 4, kPkStore = 8;
 
 // fold of k_sor_regs (fold_m) with the pass's mode given as flags
 template <int K, bool CO>
@@ -999,6 +998,61 @@ bool sor_chain_supports(int K, const DiagGeom& g, int n_passes)
            plane * (6 * K + 2) < 0x7fffffffLL && (long long)g.h * g.w < 0x7fffffffLL;
 }
 
+namespace {
+
+struct Sor32Args : SplitArgs<float> {
+    float a_data[kMaxK];
+};
+
+template <int K_>
+struct Ar32 {
+    static constexpr int K = K_;
+    static constexpr bool tick_weights = false, rings = false;
+    using T = float;
+    using T2 = float2;
+    using Args = Sor32Args;
+    using Coef = frg::Coef;
+    __device__ static float2 pair(float x, float y) { return make_float2(x, y); }
+    __device__ static Coef fold(const Args& A, int pk, const FoldIn<float, K>& in, float du, float dv)
+    {
+        Raw<K> r;
+#pragma unroll
+        for (int q = 0; q < 6 * K; ++q) r.j[q] = in.j[q];
+#pragma unroll
+        for (int k = 0; k < K; ++k) r.w[k] = in.w[k];
+        r.lu = in.lu;
+        r.lv = in.lv;
+        r.du = du;
+        r.dv = dv;
+        return fold_m<K>(A, (pk & kPkCoef) ? -1 : ((pk & kPkTick) ? 2 : 0), r);
+    }
+    __device__ static float2 point(const Args& A, float2 c, float2 up, float2 dn, float2 lf, float2 rt, float2 ca, float2 cb,
+                                   float iDv)
+    {
+        return sor_point(c, up, dn, lf, rt, make_float4(ca.x, ca.y, cb.x, cb.y), iDv, A.wa, A.wb, A.omega, A.one_m_omega);
+    }
+};
+
+// Strips of 32 rows over as many CTAs as a cluster holds, 64 and 128 rows per CTA for
+// levels over 512 and 1024 rows.  k_sor_chain keeps a frame's rows, updates and folds in
+// one CTA of up to 512 threads, where a step is one thread's chain of five updates and a
+// fold (2400 clocks even for 32 rows); here a step is one update (about 500 clocks) while
+// SMs are free, and with many frames both issue the same instructions.  Whole calls, ms,
+// k_sor_chain -> this: one frame of 512 x 512 x 2 47.7 -> 12.6, 64 frames 56.0 -> 36.0,
+// 128 frames in one plan 64.0 -> 64.1 and in two lanes 64.7 -> 60.8; 16 of 1024 x 1024 x
+// 2 123 -> 50, 4 of 2048 x 2048 x 2 257 -> 87.  Four fold warps and four CTAs per SM: other counts (three to
+// six fold warps, one to four update warps, 64 or 128 rows) measured 0 to 60 % more.
+template <int K>
+cudaError_t run_split32(const Sor32Args& A, const PassTable& T, int n_frames, cudaStream_t st)
+{
+    const int strips = A.g.P / 32;
+    if (strips > 2 * kMaxSplitCluster) return SplitLaunch<Ar32<K>, 4, 3, 2, 1>::run(A, T, n_frames, st);
+    if (strips > kMaxSplitCluster) return SplitLaunch<Ar32<K>, 2, 5, 4, 2>::run(A, T, n_frames, st);
+    return SplitLaunch<Ar32<K>, 1, 5, 4, 4>::run(A, T, n_frames, st);
+}
+
+}  // namespace
+
 cudaError_t launch_sor_chain(const float* J, long long J_fs, const float* W, long long W_fs, const float* lap,
                              long long lap_fs, float* coef, long long coef_fs, float* du, float* dv, long long st_fs,
                              int n_frames, int K, DiagGeom g, const ChainPass* passes, int n_passes,
@@ -1010,7 +1064,8 @@ cudaError_t launch_sor_chain(const float* J, long long J_fs, const float* W, lon
     if (!sor_chain_supports(K, g, n_passes) || n_frames < 1 || (long long)n_frames * nc > 0x7fffffffLL)
         return cudaErrorInvalidValue;
     ChainTable T;
-    T.n = n_passes;
+    PassTable TS;
+    T.n = TS.n = n_passes;
     int gmax = 1;
     bool co = false;
     for (int p = 0; p < n_passes; ++p) {
@@ -1023,6 +1078,39 @@ cudaError_t launch_sor_chain(const float* J, long long J_fs, const float* W, lon
         gmax = q.G > gmax ? q.G : gmax;
     }
     for (int p = n_passes; p < kMaxChain; ++p) T.pk[p] = 1 << 8;
+    // up to 2048 rows: clusters of at most 16 CTAs of 128 rows
+    if (g.P / 32 <= kMaxSplitStrips) {
+        for (int p = 0; p < kMaxChain; ++p) TS.pk[p] = T.pk[p];
+        Sor32Args S = {};
+        S.J = J;
+        S.J_fs = J_fs;
+        S.W = W;
+        S.W_fs = W_fs;
+        S.lap = lap;
+        S.lap_fs = lap_fs;
+        S.coef = coef;
+        S.coef_fs = coef_fs;
+        S.du = du;
+        S.dv = dv;
+        S.st_fs = st_fs;
+        S.out_du = out_du;
+        S.out_dv = out_dv;
+        S.out_fs = out_fs;
+        S.out_rs = g.w;
+        S.g = g;
+        S.wa = wy;  // the thread index runs along rows: row neighbours carry the y weight
+        S.wb = wx;
+        S.wsum = ((wx + wx) + wy) + wy;
+        S.omega = omega;
+        S.one_m_omega = 1.0f - omega;
+        for (int k = 0; k < kMaxK; ++k) S.a_data[k] = k < K ? a_data[k] : 0.0f;
+        switch (K) {
+            case 1: return run_split32<1>(S, TS, n_frames, st);
+            case 2: return run_split32<2>(S, TS, n_frames, st);
+            case 3: return run_split32<3>(S, TS, n_frames, st);
+            default: return run_split32<4>(S, TS, n_frames, st);
+        }
+    }
     if (sor_regs_smem(gmax, nt) > (size_t)kSmemLimit) return cudaErrorInvalidValue;
     SorArgs A = make_args(J, J_fs, W, W_fs, lap, lap_fs, coef, coef_fs, du, dv, st_fs, K, g, gmax, 0, 0, a_data, wx,
                           wy, omega, out_du, out_dv, out_fs);
