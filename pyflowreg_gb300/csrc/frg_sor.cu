@@ -557,11 +557,11 @@ __device__ __forceinline__ Coef fold_pk(const SorArgs& A, int pk, const Raw<K>& 
     return fold_m<K>(A, (pk & kPkTick) ? 2 : 0, r);
 }
 
-// CL: the level's rows are cut into A.nc strips of NT rows, one CTA each, the
+// The level's rows are cut into A.nc strips of NT rows, one CTA each, the
 // strips of a frame forming a thread-block cluster, exactly as k_sor_regs's
 // cluster form (edge rows through distributed shared memory, a cluster barrier
 // per step; every CTA runs the same step count).
-template <int K, int G, bool CO, bool CL>
+template <int K, int G, bool CO>
 __global__ void __launch_bounds__(kMaxLane) k_sor_chain(SorArgs A, ChainTable T)
 {
     extern __shared__ __align__(16) float sm[];
@@ -569,9 +569,9 @@ __global__ void __launch_bounds__(kMaxLane) k_sor_chain(SorArgs A, ChainTable T)
     const DiagGeom g = A.g;
     const int P = g.P, h = g.h, w = g.w;
     const int NT = blockDim.x, t = threadIdx.x, lane = t & 31, warp = t >> 5, NW = NT >> 5;
-    const int nc = CL ? A.nc : 1;
-    const int strip = CL ? (int)(blockIdx.x % nc) : 0;
-    const int f = CL ? (int)(blockIdx.x / nc) : (int)blockIdx.x;
+    const int nc = A.nc;
+    const int strip = (int)(blockIdx.x % nc);
+    const int f = (int)(blockIdx.x / nc);
     const int r = strip * NT + t;  // the level row of this thread
     float4* C4 = reinterpret_cast<float4*>(sm);
     float* C1 = sm + 4 * S * NT;
@@ -636,13 +636,8 @@ __global__ void __launch_bounds__(kMaxLane) k_sor_chain(SorArgs A, ChainTable T)
         }
     };
     auto xs = [&](int par, int wp, int dir, int gi) -> float2& { return X[((par * NW + wp) * 2 + dir) * G + gi]; };
-    auto step_barrier = [&]() {
-        if constexpr (CL)
-            cooperative_groups::this_cluster().sync();
-        else
-            __syncthreads();
-    };
-    if constexpr (CL) step_barrier();  // every CTA of the cluster is running before any remote write
+    auto step_barrier = [&]() { cooperative_groups::this_cluster().sync(); };
+    step_barrier();  // every CTA of the cluster is running before any remote write
 
     // the row's current pass (of the update at tau = s - r): index, local start and
     // end, its flags and those of the next pass; the fold (tau + 1) and the prefetch
@@ -696,14 +691,14 @@ __global__ void __launch_bounds__(kMaxLane) k_sor_chain(SorArgs A, ChainTable T)
                     up.x = __shfl_up_sync(0xffffffffu, V1[gi].x, 1);
                     up.y = __shfl_up_sync(0xffffffffu, V1[gi].y, 1);
                     if (lane == 0 && warp > 0) up = xs(pin, warp - 1, 0, gi);
-                    if (CL && t == 0 && strip > 0) up = XE[(pin * 2 + 0) * G + gi];
+                    if (t == 0 && strip > 0) up = XE[(pin * 2 + 0) * G + gi];
                     if (gi == 0) {
                         dn = dn1;
                     } else {
                         dn.x = __shfl_down_sync(0xffffffffu, V1[gi - 1].x, 1);
                         dn.y = __shfl_down_sync(0xffffffffu, V1[gi - 1].y, 1);
                         if (lane == 31 && warp < NW - 1) dn = xs(pin, warp + 1, 1, gi - 1);
-                        if (CL && t == NT - 1 && strip < nc - 1) dn = XE[(pin * 2 + 1) * G + gi - 1];
+                        if (t == NT - 1 && strip < nc - 1) dn = XE[(pin * 2 + 1) * G + gi - 1];
                     }
                     const int c = c0 - 2 * gi;
                     if (gi < Gp && row_ok && c >= 0 && c < w) {
@@ -737,19 +732,17 @@ __global__ void __launch_bounds__(kMaxLane) k_sor_chain(SorArgs A, ChainTable T)
 #pragma unroll
                     for (int gi = 0; gi + 1 < G; ++gi) xs(pout, warp, 1, gi) = V0[gi];
                 }
-                if constexpr (CL) {
-                    // strip edges: the last row feeds the next strip's "up", the first row the
-                    // previous strip's "down", in the neighbouring CTA's shared memory
-                    if (t == NT - 1 && strip < nc - 1) {
-                        float2* dst = cooperative_groups::this_cluster().map_shared_rank(XE, strip + 1);
+                // strip edges: the last row feeds the next strip's "up", the first row the
+                // previous strip's "down", in the neighbouring CTA's shared memory
+                if (t == NT - 1 && strip < nc - 1) {
+                    float2* dst = cooperative_groups::this_cluster().map_shared_rank(XE, strip + 1);
 #pragma unroll
-                        for (int gi = 0; gi < G; ++gi) dst[(pout * 2 + 0) * G + gi] = V0[gi];
-                    }
-                    if (t == 0 && strip > 0) {
-                        float2* dst = cooperative_groups::this_cluster().map_shared_rank(XE, strip - 1);
+                    for (int gi = 0; gi < G; ++gi) dst[(pout * 2 + 0) * G + gi] = V0[gi];
+                }
+                if (t == 0 && strip > 0) {
+                    float2* dst = cooperative_groups::this_cluster().map_shared_rank(XE, strip - 1);
 #pragma unroll
-                        for (int gi = 0; gi + 1 < G; ++gi) dst[(pout * 2 + 1) * G + gi] = V0[gi];
-                    }
+                    for (int gi = 0; gi + 1 < G; ++gi) dst[(pout * 2 + 1) * G + gi] = V0[gi];
                 }
 #pragma unroll
                 for (int gi = 0; gi < G; ++gi) {
@@ -936,35 +929,23 @@ namespace {
 template <int K, int G, bool CO>
 cudaError_t run_chain_t(const SorArgs& A, const ChainTable& T, int n_frames, int nt, cudaStream_t st)
 {
-    if (A.nc == 1) {
-        {
-            const cudaError_t e = ensure_max_dyn_smem((const void*)k_sor_chain<K, G, CO, false>, kSmemLimit);
-            if (e != cudaSuccess) return e;
-        }
-        k_sor_chain<K, G, CO, false><<<n_frames, nt, sor_regs_smem(G, nt), st>>>(A, T);
-        return cudaGetLastError();
+    {
+        const cudaError_t e = ensure_max_dyn_smem((const void*)k_sor_chain<K, G, CO>, kSmemLimit);
+        if (e != cudaSuccess) return e;
     }
-    if constexpr (K <= 2) {
-        {
-            const cudaError_t e = ensure_max_dyn_smem((const void*)k_sor_chain<K, G, CO, true>, kSmemLimit);
-            if (e != cudaSuccess) return e;
-        }
-        cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3((unsigned)(n_frames * A.nc));
-        cfg.blockDim = dim3((unsigned)nt);
-        cfg.dynamicSmemBytes = sor_regs_smem(G, nt);
-        cfg.stream = st;
-        cudaLaunchAttribute at[1];
-        at[0].id = cudaLaunchAttributeClusterDimension;
-        at[0].val.clusterDim.x = (unsigned)A.nc;
-        at[0].val.clusterDim.y = 1;
-        at[0].val.clusterDim.z = 1;
-        cfg.attrs = at;
-        cfg.numAttrs = 1;
-        return cudaLaunchKernelEx(&cfg, k_sor_chain<K, G, CO, true>, A, T);
-    } else {
-        return cudaErrorInvalidValue;
-    }
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(n_frames * A.nc));
+    cfg.blockDim = dim3((unsigned)nt);
+    cfg.dynamicSmemBytes = sor_regs_smem(G, nt);
+    cfg.stream = st;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = (unsigned)A.nc;
+    at[0].val.clusterDim.y = 1;
+    at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, k_sor_chain<K, G, CO>, A, T);
 }
 
 template <int K, bool CO>
@@ -1118,9 +1099,8 @@ cudaError_t launch_sor_chain(const float* J, long long J_fs, const float* W, lon
     switch (K) {
         case 1: return run_chain<1>(A, T, co, gmax, n_frames, nt, st);
         case 2: return run_chain<2>(A, T, co, gmax, n_frames, nt, st);
-        case 3: return run_chain<3>(A, T, co, gmax, n_frames, nt, st);
-        default: return run_chain<4>(A, T, co, gmax, n_frames, nt, st);
     }
+    return cudaErrorInvalidValue;  // more channels: levels of at most 512 rows, above
 }
 
 cudaError_t launch_sor_fused(const float* J, long long J_fs, const float* W, long long W_fs, const float* lap,

@@ -11,7 +11,7 @@ pytestmark = pytest.mark.gpu
 
 @pytest.mark.parametrize("H,W,K,T,its,lag", [
     (9, 40, 1, 1, 7, 5), (31, 33, 2, 3, 12, 5), (33, 16, 3, 2, 11, 3), (65, 20, 4, 1, 9, 1), (97, 50, 2, 40, 14, 7),
-    (512, 24, 1, 2, 8, 5), (530, 20, 2, 1, 13, 11), (1060, 18, 1, 1, 6, 2), (2040, 12, 2, 1, 5, 5)])
+    (512, 24, 1, 2, 8, 5), (530, 20, 2, 1, 13, 11), (1060, 18, 1, 1, 6, 2), (2040, 12, 2, 1, 5, 5), (2080, 12, 2, 1, 6, 5)])
 def test_same_bits_as_one_launch_per_pass(H, W, K, T, its, lag):
     from pyflowreg_gb300 import api
 
