@@ -544,7 +544,7 @@ def profiled_traffic(fp64=False):
     """DRAM bytes per algorithmic byte of the SOR kernel (float64 or float32)
     from the committed ncu summary."""
     path = os.path.join(REPO, "profiles", "dram_traffic.txt")
-    key = "k_sor_chain64" if fp64 else "k_sor"
+    key = "k_sor_split_f64" if fp64 else "k_sor_split_f32"
     try:
         for line in open(path):
             parts = line.split()
@@ -641,7 +641,7 @@ def profiled_fp64_ops():
     try:
         for line in open(path):
             parts = line.split()
-            if len(parts) >= 3 and parts[0] == "k_sor_chain64" and parts[1] == "fp64_flops_per_pixel_update":
+            if len(parts) >= 3 and parts[0] == "k_sor_split_f64" and parts[1] == "fp64_flops_per_pixel_update":
                 return float(parts[2])
     except OSError:
         pass
@@ -752,7 +752,7 @@ def run_gb300(args):
         chosen = plan.autotune(frames, n_levels=args.autotune_levels, reps=1)
         if fp64:
             tuning = {f"level {i} ({plan.level_tuning()[i][3]} rows)":
-                      {"kernel": "k_sor_chain64", "rows_per_cta": t or "by batch size"}
+                      {"kernel": "k_sor_split", "rows_per_cta": t or "by batch size"}
                       for i, (v, g, t, _) in chosen.items()}
         else:
             tuning = {f"level {i} ({plan.level_tuning()[i][3]} rows)":
@@ -826,10 +826,10 @@ def run_gb300(args):
     ratio = profiled_traffic(fp64)
     bpp = 72 if fp64 else 36
     roofline = {
-        "kernel": ("k_sor_chain64 (float64 exact-order chained wavefront SOR, one thread per row, state in "
-                   "registers, coefficients folded once per pass, row strips of 64-256 rows as clusters)" if fp64
-                   else "k_sor_chain (float32 exact-order chained wavefront SOR, one thread per row, state in "
-                   "registers, fold in the loader)"),
+        "kernel": ("k_sor_split (float64 exact-order chained wavefront SOR, update and fold warps per 32 rows, "
+                   "row strips as clusters)" if fp64
+                   else "k_sor_split (float32 exact-order chained wavefront SOR, update and fold warps per 32 "
+                   "rows, row strips as clusters)"),
         "bound": "hbm",
         "achieved": achieved,
         "peak": peak,
