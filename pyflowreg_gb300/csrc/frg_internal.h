@@ -8,10 +8,11 @@
 #include <string>
 #include <vector>
 
+#include "frg_split_schedule.h"
+
 namespace frg {
 
 constexpr int kMaxK = 8;        // channels per frame handled by one plan
-constexpr int kGMax = 5;        // SOR iterations pipelined per wavefront pass
 constexpr int kMaxLane = 512;   // longest diagonal (rows of the level) per CTA
 constexpr int kRing = 2 * kGMax + 2;
 constexpr int kPrefetch = 4;    // diagonals loaded ahead into registers
@@ -114,7 +115,6 @@ cudaError_t launch_sor_regs(const float* J, long long J_fs, const float* W, long
 // level's last pass writes out_du/out_dv when given.  Every level
 // launch_sor_regs serves (in clusters of row strips), w >= 3, at most kMaxChain
 // passes; bit-identical to one launch_sor_regs call per pass.
-constexpr int kMaxChain = 64;
 struct ChainPass {
     int G, mode, store_coef;
 };

@@ -88,7 +88,7 @@ struct FxArgs {
     FxPow pw[4];
     int *marks, *marks2;   // [n_frames] of the first and the second launch
     int lim, kmax, reach;
-    int ahead;           // steps a fold may run ahead: at most the columns of a row less one
+    int ahead;           // steps a fold may run ahead (fold_ahead)
     int second;          // second launch: frames the first one marked, format wider by kFxWider bits
     int nc;              // CTAs per frame
 };
@@ -669,7 +669,7 @@ template <int K, bool ISO, int M, int NU, int FC, int MB>
 cudaError_t run_fx(FxArgs A, const PassTable& T, int n_frames, cudaStream_t st)
 {
     constexpr size_t smem = FxSmem<M, ISO>::bytes_all;
-    A.ahead = std::min(kFoldAhead, A.g.w - 1);
+    A.ahead = fold_ahead(A.g.w);
     A.nc = (A.g.P / 32 + M - 1) / M;
     if (A.nc > kMaxSplitCluster) return cudaErrorInvalidValue;
     auto kern = k_sor_fx<K, ISO, M, NU, FC, MB>;
@@ -744,8 +744,7 @@ void place_fx_pow(void* dev, FxPow* P) { place_fx(dev, P); }
 
 bool sor_fx_supports(int K, const DiagGeom& g, int n_passes, double omega)
 {
-    // three columns or more, so that a state is stored before a fold (at least two steps ahead of
-    // the update) reads it; omega in [1, 2) keeps |1 - omega| < 1 and c < 1/2
+    // three columns or more: the least a fold runs ahead (fold_ahead); omega in [1, 2) keeps |1 - omega| < 1 and c < 1/2
     return K >= 1 && K <= 4 && (g.P & 31) == 0 && g.w >= 3 && n_passes >= 1 && n_passes <= kMaxChain &&
            g.P / 32 <= kMaxSplitStrips && omega >= 1.0 && omega < 2.0 &&
            (long long)g.D * g.P * (6 * K + 2) < 0x7fffffffLL;

@@ -8,6 +8,7 @@
 #pragma once
 
 #include "frg_internal.h"
+#include "frg_split_schedule.h"
 
 #include <cooperative_groups.h>
 
@@ -15,17 +16,9 @@ namespace frg {
 
 namespace {
 
-constexpr int kRingSlots = 16;          // ring slots: a pixel's coefficients are read for 2 (G - 1) + 1 = 9 steps
-constexpr int kRingUse = 2 * (kGMax - 1);
-constexpr int kFoldAhead = kRingSlots - kRingUse;  // most steps a fold may run ahead of the update
 constexpr int kMaxSplitStrips = 64;
 constexpr int kMaxSplitCluster = 16;
 constexpr unsigned kMaxTries = 500000u;  // tries of a wait, of at most 2 us each
-
-struct PassTable {
-    int n;
-    int pk[kMaxChain];  // G << 8 | store << 3 | coef << 2 | tick << 1 | zero
-};
 
 constexpr int kPkZero = 1, kPkTick = 2, kPkCoef = 4, kPkStore = 8;
 
@@ -99,15 +92,6 @@ __device__ __forceinline__ void mbar_wait(unsigned mb, unsigned parity, bool& de
     dead = true;
 }
 
-// Steps a row spends in a pass.  After a single iteration one step more, so that
-// the step before a row's first pixel of the next pass (which takes that
-// pixel's value as its right neighbour) is free.
-__device__ __forceinline__ int pass_span(int w, int pk)
-{
-    const int n = pk >> 8;
-    return w + (n > 1 ? 2 * (n - 1) : 1);
-}
-
 // Which warp does what.  Warp i runs on scheduler i % 4, and with five update
 // warps two share one: that scheduler gets the waiting warp besides and no fold
 // (one idle warp fills its place when there are more than six).
@@ -120,27 +104,6 @@ struct SplitRoles {
     static constexpr int warps = WU + 1 + M * FC + (idle >= 0 ? 1 : 0);
     static_assert(FC >= 1 && NU >= 1 && NU <= kGMax && wait < warps && idle < warps && warps <= 32, "every role has its warps");
     __device__ static int fold(int warp) { return spread ? warp - (warp < 8 ? 5 : (warp < 12 ? 6 : 7)) : warp - WU - 1; }
-};
-
-// A row's place in the chain of passes at local time tau.
-struct Cursor {
-    int p, start, end, pk;
-    __device__ __forceinline__ void init(const PassTable& T, int w)
-    {
-        p = 0;
-        start = 0;
-        pk = T.pk[0];
-        end = pass_span(w, pk);
-    }
-    __device__ __forceinline__ void advance(const PassTable& T, int w, int tau)
-    {
-        if (tau >= end && p < T.n - 1) {
-            ++p;
-            start = end;
-            pk = T.pk[p];
-            end = start + pass_span(w, pk);
-        }
-    }
 };
 
 }  // namespace

@@ -33,7 +33,7 @@ struct SplitArgs {
     T wsum;        // ((wx + wx) + wy) + wy, the reference's order
     T omega, one_m_omega;
     int nc;              // CTAs per frame
-    int ahead;           // steps a fold may run ahead: at most the columns of a row less one
+    int ahead;           // steps a fold may run ahead (fold_ahead)
     const int* marks;    // frames to compute (fx_recompute); null: all
     int ring;            // the final pass also writes the border copies around the output
 };
@@ -383,7 +383,7 @@ struct SplitLaunch {
     }
     static cudaError_t run(typename Ar::Args A, const PassTable& T, int n_frames, cudaStream_t st)
     {
-        A.ahead = std::min(kFoldAhead, A.g.w - 1);
+        A.ahead = fold_ahead(A.g.w);
         A.nc = ctas(A.g);
         if (A.nc > kMaxSplitCluster || (long long)n_frames * A.nc > 0x7fffffffLL) return cudaErrorInvalidValue;
         const cudaError_t e = prepare(A.nc);
