@@ -479,7 +479,7 @@ __global__ void __launch_bounds__(32 * SplitRoles<M, NU, FC>::warps, MB) k_sor_f
             const int slot = (unsigned)s % S;
             // the update has finished step s - ahead: the slot is free, and the states stored up to then can be read
             if (s >= A.ahead) mbar_wait(empty_bar(strip, slot), ((unsigned)(s - A.ahead) / S) & 1, dead);
-            cur.advance(T, w, s - r);
+            cur.seek(T, w, s - r);
             const int c = s - r - cur.start, pk = cur.pk, o = (r + c) * P;
             const bool in_level = row_ok && (unsigned)c < (unsigned)w;
             FxIn<K> in;

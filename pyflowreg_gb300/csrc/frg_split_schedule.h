@@ -48,14 +48,22 @@ struct Cursor {
         pk = T.pk[0];
         end = pass_span(w, pk);
     }
+    FRG_HD void next(const PassTable& T, int w)
+    {
+        ++p;
+        start = end;
+        pk = T.pk[p];
+        end = start + pass_span(w, pk);
+    }
+    // For a caller that comes by every step: no pass is shorter than that.
     FRG_HD void advance(const PassTable& T, int w, int tau)
     {
-        if (tau >= end && p < T.n - 1) {
-            ++p;
-            start = end;
-            pk = T.pk[p];
-            end = start + pass_span(w, pk);
-        }
+        if (tau >= end && p < T.n - 1) next(T, w);
+    }
+    // For a fold warp, whose steps lie FC apart: a pass of few columns may lie between two of them.
+    FRG_HD void seek(const PassTable& T, int w, int tau)
+    {
+        while (tau >= end && p < T.n - 1) next(T, w);
     }
 };
 

@@ -88,7 +88,7 @@ extern "C" int split_model(int h, int w, int M, int FC, int n, const int* G, con
             cur.init(R.T, w);
             for (int s = j; s < N; s += FC) {
                 const int tau = s - r;
-                cur.advance(R.T, w, tau);
+                cur.seek(R.T, w, tau);
                 int p = 0;
                 while (p + 1 < n && tau >= R.start[p + 1]) ++p;
                 const int c = tau - R.start[p];

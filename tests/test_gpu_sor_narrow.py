@@ -60,3 +60,22 @@ def test_flow_fp32_same_bits(H, W, K, T):
     plan.close()
     assert bool(torch.isfinite(out[2]).all())
     assert torch.equal(out[1], out[2])
+
+
+@pytest.mark.parametrize("w", [3, 4, 5, 6])
+@pytest.mark.parametrize("lag", [1, 2, 3, 6, 11])
+@pytest.mark.parametrize("scale", [1.0, 3e3])
+def test_level_short_passes(oracle, w, lag, scale):
+    got, ref = _both(oracle, _case(37, w, 2, w + lag, scale), (1.5, 1.2), 23, lag, 0.45)
+    _close(got, ref)
+
+
+@pytest.mark.parametrize("W,lag", [(3, 1), (4, 1), (5, 2)])
+def test_flow_short_passes(oracle, W, lag):
+    from pyflowreg_gb300 import api
+
+    fixed, moving = _frames(45, W, 1, 1, W + lag)
+    kw = dict(alpha=(1.5, 1.5), iterations=20, update_lag=lag, levels=100, eta=0.8)
+    got = api.get_displacement_device(fixed, moving, precision="fp64", **kw).cpu().numpy()
+    ref = oracle.get_displacement(fixed[..., 0].cpu().numpy(), moving[0, ..., 0].cpu().numpy(), **kw)
+    assert np.abs(got[0] - ref).max() <= 1e-3

@@ -39,3 +39,12 @@ def _run(model, h, w, M, FC, iterations, lag):
 def test_waits_end_and_values_are_there(model, w, M, FC):
     for h in (1, 31, 33, 64, 130, 300):
         _run(model, h, w, M, FC, 15, 5)
+
+
+@pytest.mark.parametrize("lag", [1, 2, 3, 6, 11, 16])
+@pytest.mark.parametrize("w", list(range(3, 11)))
+def test_folds_take_the_entering_pixels(model, w, lag):
+    """Passes shorter than the stride of a fold warp: several pass boundaries between two of its steps."""
+    for M, FC in DIVISIONS:
+        for h in (1, 20, 33, 70):
+            _run(model, h, w, M, FC, 23, lag)
