@@ -235,11 +235,18 @@ int frg_level_solve_noalloc(int m, int n, int K, const float* J, const float* we
                             double omega, float* du, float* dv, void* stream);
 size_t frg_level_solve_noalloc_capacity(void);
 
-/* The level solver in the reference's own precision and operation order, for
- * the level_solver_backend seam fed with the reference's float64 arrays
+/* The level solver in float64 and in the reference's update order, for the
+ * level_solver_backend seam fed with the reference's float64 arrays
  * (core/optical_flow.py:348-411): compute_flow (core/level_solver.py:158-369)
  * when gnc_beta < 0, compute_flow_gnc (core/level_solver.py:372-555) with
- * that stage weight when gnc_beta is in [0, 1]; any a_smooth > 0.  Layouts as
+ * that stage weight when gnc_beta is in [0, 1]; any a_smooth > 0.
+ * With a_smooth = 1, gnc_beta < 0, at most 4 channels, 3 columns or more and at
+ * most 2048 rows the terms of an update are grouped as in an FP64 plan's levels
+ * (coefficients folded once per psi update): as near to the exact result as the
+ * reference's own operations (relative error about 1e-14 after 50 iterations
+ * either way), not their bits, and the same bits on captured streams.  Everything
+ * else, and a call for whose scratch there is no memory, runs the reference's
+ * operations one by one.  Layouts as
  * frg_level_solve, all arrays double on the device; du, dv receive the whole
  * (m, n) result, their rings as set_boundary_2d left them at the start of the
  * last iteration.  Allocates its scratch with cudaMallocAsync on `stream`. */

@@ -877,9 +877,10 @@ def level_solver(J11, J22, J33, J12, J13, J23, weight, u, v, alpha, iterations, 
 
     Runs compute_flow's exact update order on the device and returns (du, dv)
     as float64 (m, n) arrays.  precision "fp64" (default; taken as well
-    whenever a_smooth != 1 or gnc_beta is given) computes in the reference's
-    float64 arithmetic, compute_flow_gnc when gnc_beta is not None; "fp32" is
-    the float32 solver (a_smooth = 1, no GNC).
+    whenever a_smooth != 1 or gnc_beta is given) computes in float64, within
+    float64 rounding of the reference (about 1e-14 relative),
+    compute_flow_gnc when gnc_beta is not None; "fp32" is the float32 solver
+    (a_smooth = 1, no GNC).
     """
     _require_cuda()
     if precision not in PRECISIONS:

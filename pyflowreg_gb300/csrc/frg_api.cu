@@ -448,18 +448,6 @@ int make_pow_tables(frg_plan* pl, int channels)
     return FRG_OK;
 }
 
-// Whether the fixed-point SOR serves every channel's power.
-bool fx_exponents_ok(int K, const double* a_data)
-{
-    for (int k = 0; k < K; ++k)
-        if (!(a_data[k] > 0.0 && a_data[k] <= 2.0)) return false;
-    return true;
-}
-
-// The fixed-point form's first guess of a single level's |du|, |dv|: below 2^4 px
-// (its second launch reaches 2^7).
-constexpr int kFxReach = 4;
-
 int upload_tables(frg_plan* pl, const HostTables& t, int n_out_x, const HostTables& ty, int n_out_y,
                   DevTables* d)
 {
@@ -1481,58 +1469,43 @@ int frg_level_solve(int m, int n, int K, const float* J, const float* weight, co
 namespace {
 
 // compute_flow through the chained SOR: a_smooth = 1, no GNC, the levels
-// launch_sor_chain64 serves.  Fixed point first (one level alone may differ from
-// float64 in the last bits), float64 for what lies outside its ranges.  410 x 410 x
-// 2, 50 iterations, host arrays in and out: 7.9 ms; launch_x_sor, which takes every
-// other level, 540 ms.
+// launch_sor_chain64 serves, with the operations that the pyramid's levels have (the
+// general power: a table of its own for each call would cost more than it saves).
+// 410 x 410 x 2, 50 iterations, host arrays in and out: 8.2 ms; launch_x_sor, which
+// takes every other level, 539 ms.
+// Capturable: nothing is copied from the host.  *served = false, with nothing
+// launched, when the diagonal-major scratch, up to (h + w) / min(h, w) times the
+// arrays' size, cannot be had.
 int seam_chain64(int h, int w, int K, const DiagGeom& g, const double* J, const double* weight, const double* u,
                  const double* v, double alpha_x, double alpha_y, const Pass* ps, int np, const double* a_data,
-                 double hx, double hy, double omega, double* du, double* dv, cudaStream_t st)
+                 double hx, double hy, double omega, double* du, double* dv, cudaStream_t st, bool* served)
 {
-    if (int rc = ensure_remap_tables()) return rc;
+    FRG_CUDA(upload_dpow_tables());
     const double wx = alpha_x / (hx * hx), wy = alpha_y / (hy * hy);
     ChainPass cp[kMaxChain];
     chain_passes(ps, np, cp);
-    const bool fx = sor_fx_supports(K, g, np, omega) && fx_exponents_ok(K, a_data);
     const long long dp = (long long)g.D * g.P;
-    const size_t tab = fx_pow_bytes();
-    const size_t doubles = (size_t)(6 * K + 4 * K + 2 + 5 + 2) * dp;
-    char* scratch = nullptr;
-    FRG_CUDA(cudaMallocAsync((void**)&scratch, doubles * sizeof(double) + K * tab + 2 * sizeof(int), st));
-    double* Jd = (double*)scratch;
+    double* Jd = nullptr;
+    cudaError_t e = cudaMallocAsync((void**)&Jd, (size_t)(6 * K + 2 * K + 2 + 5 + 2) * dp * sizeof(double), st);
+    *served = e != cudaErrorMemoryAllocation;
+    if (!*served) {
+        cudaGetLastError();
+        return FRG_OK;
+    }
+    FRG_CUDA(e);
     double* Wd = Jd + 6LL * K * dp;
-    double* Wfx = Wd + 2LL * K * dp;
-    double* lap = Wfx + 2LL * K * dp;
+    double* lap = Wd + 2LL * K * dp;
     double* coef = lap + 2 * dp;
     double* sdu = coef + 5 * dp;
     double* sdv = sdu + dp;
-    char* tabs = (char*)(sdv + dp);
-    int* marks = (int*)(tabs + K * tab);
     auto run = [&]() -> int {
-        FRG_LAUNCH(launch_x_seam_to_diag(J, weight, u, v, K, h, w, g, wx, wy, a_data, Jd, Wd, Wfx, lap, st));
-        double* odu = du + (w + 2) + 1;
-        double* odv = dv + (w + 2) + 1;
-        if (fx) {
-            FxPow pows[kMaxK];
-            std::vector<char> host(K * tab);
-            for (int k = 0; k < K; ++k) {
-                if (!make_fx_pow(a_data[k] - 1.0, host.data() + k * tab, &pows[k])) return fail(FRG_EINVAL, "a_data");
-                place_fx_pow(tabs + k * tab, &pows[k]);
-            }
-            // from pageable memory: returns once the tables are staged
-            FRG_CUDA(cudaMemcpyAsync(tabs, host.data(), host.size(), cudaMemcpyHostToDevice, st));
-            FRG_CUDA(cudaMemsetAsync(marks, 0, 2 * sizeof(int), st));
-            for (int second = 0; second < 2; ++second)
-                FRG_LAUNCH(launch_sor_fx(Jd, 0, Wfx, 0, lap, 0, coef, 0, sdu, sdv, 0, 1, K, g, cp, np, wx, wy, omega, st,
-                                         odu, odv, 0, w + 2, 1, pows, kFxReach, second, marks, marks + 1));
-        }
+        FRG_LAUNCH(launch_x_seam_to_diag(J, weight, u, v, K, h, w, g, wx, wy, a_data, Jd, Wd, lap, st));
         FRG_LAUNCH(launch_sor_chain64(Jd, 0, Wd, 0, lap, 0, coef, 0, sdu, sdv, 0, 1, K, g, cp, np, a_data, wx, wy, omega,
-                                      st, odu, odv, 0, w + 2, 0, nullptr,
-                                      fx ? marks + 1 : nullptr, 1));
+                                      st, du + (w + 2) + 1, dv + (w + 2) + 1, 0, w + 2, 0, nullptr, 1));
         return FRG_OK;
     };
     const int rc = run();
-    const cudaError_t e = cudaFreeAsync(scratch, st);
+    e = cudaFreeAsync(Jd, st);
     if (rc == FRG_OK && e != cudaSuccess) return fail(FRG_ECUDA, cudaGetErrorString(e));
     return rc;
 }
@@ -1559,11 +1532,12 @@ int frg_level_solve_f64(int m, int n, int K, const double* J, const double* weig
     if (!smooth && gnc_beta < 0.0) {
         Pass ps[kMaxChain];
         const int np = fill_passes(iterations, update_lag, kGMax, ps, kMaxChain);
-        // not while the stream is captured: the chained form uploads tables from the call's own memory
-        cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-        FRG_CUDA(cudaStreamIsCapturing(st, &cap));
-        if (cap == cudaStreamCaptureStatusNone && sor_chain64_supports(K, g, np))
-            return seam_chain64(h, w, K, g, J, weight, u, v, alpha_x, alpha_y, ps, np, a_data, hx, hy, omega, du, dv, st);
+        bool served = sor_chain64_supports(K, g, np);
+        if (served) {
+            const int rc = seam_chain64(h, w, K, g, J, weight, u, v, alpha_x, alpha_y, ps, np, a_data, hx, hy, omega, du,
+                                        dv, st, &served);
+            if (served) return rc;
+        }
     }
     double* scratch = nullptr;
     const size_t elems = (size_t)(6 * K + 2 * K + (smooth ? 3 : 0)) * mn;

@@ -1175,7 +1175,7 @@ cudaError_t launch_x_pad_to_diag(const double* src, int K, int h, int w, DiagGeo
 __global__ void kx_seam_to_diag(const double* __restrict__ J, const double* __restrict__ wgt, const double* __restrict__ u,
                                 const double* __restrict__ v, int K, int h, int w, DiagGeom g, double wx, double wy,
                                 ChannelScale ad, double* __restrict__ Jd, double* __restrict__ Wd,
-                                double* __restrict__ Wfx, double per_wsum, double* __restrict__ lap)
+                                double* __restrict__ lap)
 {
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
     const int r = blockIdx.y;
@@ -1191,8 +1191,6 @@ __global__ void kx_seam_to_diag(const double* __restrict__ J, const double* __re
         const double x = wgt[o * K + k];
         Wd[k * plane + di] = x;
         Wd[(K + k) * plane + di] = dmul(x, ad.s[k]);
-        Wfx[k * plane + di] = dmul(x, per_wsum);
-        Wfx[(K + k) * plane + di] = dmul(dmul(x, ad.s[k]), per_wsum);
     }
     for (int q = 0; q < 2; ++q) {
         const double* a = q ? v : u;
@@ -1207,13 +1205,13 @@ __global__ void kx_seam_to_diag(const double* __restrict__ J, const double* __re
 
 cudaError_t launch_x_seam_to_diag(const double* J, const double* wgt, const double* u, const double* v, int K, int h,
                                   int w, DiagGeom g, double wx, double wy, const double* a_data, double* Jd, double* Wd,
-                                  double* Wfx, double* lap, cudaStream_t st)
+                                  double* lap, cudaStream_t st)
 {
     if (K < 1 || K > kMaxK) return cudaErrorInvalidValue;
     ChannelScale sc = {};
     for (int k = 0; k < K; ++k) sc.s[k] = a_data[k];
     dim3 blk(128), grd((w + 127) / 128, h);
-    kx_seam_to_diag<<<grd, blk, 0, st>>>(J, wgt, u, v, K, h, w, g, wx, wy, sc, Jd, Wd, Wfx, 1.0 / (((wx + wx) + wy) + wy), lap);
+    kx_seam_to_diag<<<grd, blk, 0, st>>>(J, wgt, u, v, K, h, w, g, wx, wy, sc, Jd, Wd, lap);
     return cudaGetLastError();
 }
 

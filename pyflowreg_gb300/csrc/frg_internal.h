@@ -156,39 +156,9 @@ cudaError_t launch_sor_chain64(const double* J, long long J_fs, const double* W,
                                long long st_fs, int n_frames, int K, DiagGeom g, const ChainPass* passes,
                                int n_passes, const double* a_data, double wx, double wy, double omega,
                                cudaStream_t st, double* out_du, double* out_dv, long long out_fs, int out_rs,
-                               int rows = 0, const PowTab64* pows = nullptr, const int* marks = nullptr, int ring = 0);
-// marks (optional, one per frame, of launch_sor_fx): frames without a mark are
-// skipped.  ring: the border copies around the output (rows -1 and h, columns
-// -1 and w) are written too, as set_boundary_2d left them before the last
-// iteration.
-//
-// The same solver with fixed-point updates (frg_sorfx.cu, k_sor_fx), run twice:
-// a first launch for all frames, and a second one (second = 1) with a wider
-// number format for the frames the first one marked; a frame that the second
-// one marks too (fx_recompute(marks2[f])) is left to launch_sor_chain64.
-// W: the weights divided by wsum = 2 (wx + wy) (both planes).  wp [K][D*P] (weights
-// times psi of passes that continue a group) and the state du, dv [D*P] are
-// workspaces of 64-bit words.  32 rows per CTA, more where the level would need over
-// 16 CTAs.  reach: 2^reach px bounds the level's |du|, |dv|.
-struct FxPow {
-    const longlong2* A = nullptr;     // [64] 2^(e b) = A.x 2^(A.y - 61), e from kPowEMin
-    const long long* B = nullptr;     // [256] (2^16 / R)^b, 60 fraction bits
-    const unsigned* R = nullptr;      // [256]
-    long long c1 = 0, c2 = 0;         // binomial coefficients, 60 fraction bits
-    int c3 = 0, c4 = 0, c5 = 0, c6 = 0;  // 30 fraction bits
-};
-__host__ __device__ inline bool fx_recompute(int mark) { return (mark & 1) || ((mark & 4) && !(mark & 2)); }
-size_t fx_pow_bytes();
-// Host: fills `host` (fx_pow_bytes()) and the constants of *P for exponent b;
-// false when |b| > 1.  place_fx_pow: the table's place on the device.
-bool make_fx_pow(double b, void* host, FxPow* P);
-void place_fx_pow(void* dev, FxPow* P);
-bool sor_fx_supports(int K, const DiagGeom& g, int n_passes, double omega);
-cudaError_t launch_sor_fx(const double* J, long long J_fs, const double* W, long long W_fs, const double* lap,
-                          long long lap_fs, double* wp, long long wp_fs, double* du, double* dv, long long st_fs,
-                          int n_frames, int K, DiagGeom g, const ChainPass* passes, int n_passes, double wx, double wy,
-                          double omega, cudaStream_t st, double* out_du, double* out_dv, long long out_fs, int out_rs,
-                          int ring, const FxPow* pows, int reach, int second, int* marks, int* marks2);
+                               int rows = 0, const PowTab64* pows = nullptr, int ring = 0);
+// ring: the border copies around the output (rows -1 and h, columns -1 and w) are
+// written too, as set_boundary_2d left them before the last iteration.
 // x^b elementwise by the float64 solver's power (frg_dpow.cuh), with the table
 // path for |b| <= 1; upload_dpow_tables must have run on the current device.
 cudaError_t launch_pow64(long long n, const double* x, double b, double* out, cudaStream_t st);
@@ -253,10 +223,10 @@ cudaError_t launch_x_sor_smooth(const double* J, const double* W, const double* 
 cudaError_t launch_x_to_float(const double* src, long long n, float* dst, cudaStream_t st);
 // Padded (K, (h+2)*(w+2)) float64 planes to diagonal-major (K, D*P).
 // The level solver seam's (m, n, K) arrays in the chained SOR's form: Jd (6, K,
-// D*P), Wd (2, K, D*P), Wfx the same over wsum = 2 (wx + wy), lap (2, D*P).
+// D*P), Wd (2, K, D*P), lap (2, D*P).
 cudaError_t launch_x_seam_to_diag(const double* J, const double* wgt, const double* u, const double* v, int K, int h,
                                   int w, DiagGeom g, double wx, double wy, const double* a_data, double* Jd, double* Wd,
-                                  double* Wfx, double* lap, cudaStream_t st);
+                                  double* lap, cudaStream_t st);
 // Padded (K, h + 2, w + 2) float64 planes to diagonal-major (K, D*P) at dst;
 // with scale (K host values), also each plane times scale[k] at dst + K*D*P
 // (the float64 chained SOR's weights W and W * a_data).

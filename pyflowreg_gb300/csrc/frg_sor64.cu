@@ -48,7 +48,8 @@
 namespace frg {
 
 // The tables of dpow_tab, from the host's long double log2 / exp2 (extended or
-// quadruple precision), rounded to double once.
+// quadruple precision), rounded to double once.  Copied on a stream of its own, so
+// that the first call may come while the caller's stream is being captured.
 cudaError_t upload_dpow_tables()
 {
     static std::mutex mu;
@@ -72,10 +73,19 @@ cudaError_t upload_dpow_tables()
         lt[3 * j + 2] = Llo;
     }
     for (int i = 0; i < kDpowExpN; ++i) et[i] = (double)exp2l((long double)i / (long double)kDpowExpN);
-    if ((e = cudaMemcpyToSymbol(g_dpow_log, lt, sizeof(lt))) != cudaSuccess) return e;
-    if ((e = cudaMemcpyToSymbol(g_dpow_exp, et, sizeof(et))) != cudaSuccess) return e;
-    done.insert(dev);
-    return cudaSuccess;
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    if ((e = cudaThreadExchangeStreamCaptureMode(&mode)) != cudaSuccess) return e;
+    cudaStream_t own = nullptr;
+    if ((e = cudaStreamCreateWithFlags(&own, cudaStreamNonBlocking)) == cudaSuccess) {
+        e = cudaMemcpyToSymbolAsync(g_dpow_log, lt, sizeof(lt), 0, cudaMemcpyHostToDevice, own);
+        if (e == cudaSuccess) e = cudaMemcpyToSymbolAsync(g_dpow_exp, et, sizeof(et), 0, cudaMemcpyHostToDevice, own);
+        const cudaError_t s = cudaStreamSynchronize(own);  // lt and et are this call's
+        if (e == cudaSuccess) e = s;
+        cudaStreamDestroy(own);
+    }
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    if (e == cudaSuccess) done.insert(dev);
+    return e;
 }
 
 // dpow_b's table for exponent b: T(e, j) = 2^(e b) (1 / inv_j)^b in long double,
@@ -341,7 +351,7 @@ cudaError_t launch_sor_chain64(const double* J, long long J_fs, const double* W,
                                long long st_fs, int n_frames, int K, DiagGeom g, const ChainPass* passes,
                                int n_passes, const double* a_data, double wx, double wy, double omega,
                                cudaStream_t st, double* out_du, double* out_dv, long long out_fs, int out_rs,
-                               int rows, const PowTab64* pows, const int* marks, int ring)
+                               int rows, const PowTab64* pows, int ring)
 {
     if (!sor_chain64_supports(K, g, n_passes) || n_frames < 1) return cudaErrorInvalidValue;
     if (rows != 0 && !sor_chain64_rows_ok(g, rows)) return cudaErrorInvalidValue;
@@ -375,7 +385,6 @@ cudaError_t launch_sor_chain64(const double* J, long long J_fs, const double* W,
     A.out_dv = out_dv;
     A.out_fs = out_fs;
     A.out_rs = out_rs;
-    A.marks = marks;
     A.ring = ring;
     A.g = g;
     A.wa = wy;  // the thread index runs along rows: row neighbours carry the y weight

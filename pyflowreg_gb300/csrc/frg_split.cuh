@@ -1,7 +1,6 @@
-// What the split forms of the chained SOR share (k_sor_split, k_sor_fx): the work of 32 rows is divided among update warps (one per
-// pipelined iteration), fold warps that run ahead of them and one warp that waits
-// for both and for the neighbouring CTAs; rings, barriers and the place of a row
-// in the chain of passes.
+// Parts of the split chained SOR (k_sor_split, frg_split_sor.cuh): the work of 32 rows
+// is divided among update warps (one per pipelined iteration), fold warps that run
+// ahead of them and one warp that waits for both and for the neighbouring CTAs.
 //
 // Every wait is bounded: a wait that runs out is given up, and so is every later
 // one of that warp, so that the kernel ends; the caller of mbar_wait reports it.
@@ -83,7 +82,7 @@ __device__ __forceinline__ bool mbar_test(unsigned mb, unsigned parity)
 }
 
 // Waits for the phase with this parity to complete.  After one wait has run
-// out no further one is made (the frame is marked and recomputed).
+// out no further one is made.
 __device__ __forceinline__ void mbar_wait(unsigned mb, unsigned parity, bool& dead)
 {
     if (dead) return;

@@ -34,7 +34,6 @@ struct SplitArgs {
     T omega, one_m_omega;
     int nc;              // CTAs per frame
     int ahead;           // steps a fold may run ahead (fold_ahead)
-    const int* marks;    // frames to compute (fx_recompute); null: all
     int ring;            // the final pass also writes the border copies around the output
 };
 
@@ -85,7 +84,6 @@ __global__ void __launch_bounds__(32 * SplitRoles<M, NU, FC>::warps, MB) k_sor_s
     const int nc = A.nc;
     const int cta = nc > 1 ? (int)(blockIdx.x % nc) : 0;
     const int f = nc > 1 ? (int)(blockIdx.x / nc) : (int)blockIdx.x;
-    if (A.marks && !fx_recompute(A.marks[f])) return;  // the same for every CTA of a cluster
     const bool update = warp < WU;
     const int strip = (update ? warp : Roles::fold(warp)) % M;
     const int row = strip * 32 + lane;  // in the CTA
