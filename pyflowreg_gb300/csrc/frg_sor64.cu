@@ -235,12 +235,15 @@ __device__ __forceinline__ Coef64 fold64(const Sor64Args& A, int pk, const FoldI
             const double a = du, b = dv;
             // E + 1e-5 = a (J11 a + 2 J12 b + 2 J13) + b (J22 b + 2 J23) + (J33 + 1e-5):
             // 5 float64 operations; max(E, 0) + 1e-5 as max(E + 1e-5, 1e-5), compared as
-            // 64-bit integers (the order of non-negative doubles; negative ones are below)
+            // 64-bit integers (the order of non-negative doubles; negative ones are below,
+            // down to -inf: a NaN with its sign set, quiet as an operation's result is, lies
+            // above that as an unsigned integer and stays)
             double t = __fma_rn(j11, a, j13);
             t = __fma_rn(j12, b, t);
             const double q = __fma_rn(j22, b, j23);
             double E = __fma_rn(t, a, __fma_rn(q, b, j33));
-            if (__double_as_longlong(E) < __double_as_longlong(0.00001)) E = 0.00001;
+            if (__double_as_longlong(E) < __double_as_longlong(0.00001) && (unsigned)__double2hiint(E) <= 0xfff00000u)
+                E = 0.00001;
             wp = __dmul_rn(wp, dpow_b(E, A.a_m1[k], A.pw[k]));
         }
         den_u = __fma_rn(wp, j11, den_u);

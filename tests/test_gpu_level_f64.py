@@ -116,3 +116,15 @@ def test_whole_pyramid_through_the_seam(oracle, shape, K):
     own = G.get_displacement(fixed, moving, **kw)
     assert np.abs(own - ref).max() <= 1e-3
     assert np.abs(got - ref).max() <= 1e-3
+
+
+@pytest.mark.parametrize("scale", [1.0, 3e3])
+@pytest.mark.parametrize("q,value", [(2, np.nan), (2, -np.nan), (2, np.inf), (2, -np.inf), (0, np.inf), (1, -np.nan), (5, np.inf)])
+def test_not_a_number_reaches_the_result(oracle, q, value, scale):
+    """A weight psi of a quadratic form that is no number is none either, whatever the NaN's sign."""
+    case = _case(40, 30, 2, 3, scale)
+    case[0][q][20, 15, 1] = value
+    with np.errstate(all="ignore"):
+        got, ref = _both(oracle, case, (1.5, 1.5), 12, 5, 0.45)
+    for g, r in zip(got, ref):
+        assert np.array_equal(np.isnan(g), np.isnan(r))
