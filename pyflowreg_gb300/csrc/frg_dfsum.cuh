@@ -32,6 +32,7 @@ __device__ __forceinline__ double f2d(float f)
 // where a float64 addition holds a scheduler's pipe for 64.
 struct DfSum {
     float hi = 0.0f, lo = 0.0f, mag = 0.0f;
+    unsigned factors = 0;  // the bits of the products' factors: zero when every product is an exact +0
     __device__ __forceinline__ void add(float p)
     {
         const float s = __fadd_rn(hi, p);
@@ -40,17 +41,18 @@ struct DfSum {
         hi = s;
         mag = __fadd_rn(mag, fabsf(p));
     }
-    // p + e, e an error term far below p
-    __device__ __forceinline__ void add_pair(float p, float e)
+    // p + e, the product of a and a weight: p its float32, e an error term far below p
+    __device__ __forceinline__ void add_pair(float a, float p, float e)
     {
         add(p);
         lo = __fadd_rn(lo, e);
+        factors |= __float_as_uint(a);
     }
     // the exact product a * w
     __device__ __forceinline__ void add_product(float a, float w)
     {
         const float p = __fmul_rn(a, w);
-        add_pair(p, __fmaf_rn(a, w, -p));
+        add_pair(a, p, __fmaf_rn(a, w, -p));
     }
     // err: kDfErr(n)
     __device__ __forceinline__ bool value(float err, float* out) const
@@ -58,13 +60,14 @@ struct DfSum {
         const float s = __fadd_rn(hi, lo);
         const float b = __fsub_rn(s, hi);
         const float r = __fadd_rn(__fsub_rn(hi, __fsub_rn(s, b)), __fsub_rn(lo, b));  // hi + lo = s + r
-        *out = mag == 0.0f ? 0.0f : s;
+        *out = s;
         const unsigned u = __float_as_uint(s);
         const unsigned e = (u >> 23) & 0xffu;
         // half the spacing of float32 at s; below a power of two the spacing halves
         const float half = __uint_as_float((e - 24u) << 23);
         const bool usual = e > 60u && e < 0xffu && (u & 0x7fffffu) != 0u;
-        return mag == 0.0f || (usual && __fmaf_rn(mag, err, fabsf(r)) < half);
+        // mag 0: products of factors other than +0 may have underflowed, and only the float64 sum holds them
+        return (mag == 0.0f && factors == 0u) || (usual && __fmaf_rn(mag, err, fabsf(r)) < half);
     }
 };
 

@@ -156,7 +156,7 @@ __device__ __forceinline__ S corr_tile(const double* w, const float2* wf, int r,
         const float c = at(0);
         {
             const float p = __fmul_rn(c, wf[0].x);
-            acc.add_pair(p, __fmaf_rn(c, wf[0].y, __fmaf_rn(c, wf[0].x, -p)));
+            acc.add_pair(c, p, __fmaf_rn(c, wf[0].y, __fmaf_rn(c, wf[0].x, -p)));
         }
         for (int j = r; j >= 1; --j) {
             const float a = at(-j), b = at(j);
@@ -164,7 +164,7 @@ __device__ __forceinline__ S corr_tile(const double* w, const float2* wf, int r,
             const float d = __fadd_rn(__fsub_rn(a, __fsub_rn(s, z)), __fsub_rn(b, z));  // a + b = s + d
             const float2 t = wf[j];
             const float p = __fmul_rn(s, t.x);
-            acc.add_pair(p, __fmaf_rn(d, t.x, __fmaf_rn(s, t.y, __fmaf_rn(s, t.x, -p))));
+            acc.add_pair(s, p, __fmaf_rn(d, t.x, __fmaf_rn(s, t.y, __fmaf_rn(s, t.x, -p))));
         }
         float v;
         if (acc.value(kDfErr(4 * (r + 1)), &v)) return v;
