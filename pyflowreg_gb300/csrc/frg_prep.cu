@@ -224,19 +224,28 @@ __global__ void __launch_bounds__(256) k_prep_tile(PrepArgs A, float* __restrict
     }
 }
 
-// sqrt(s) for s >= 0: the hardware's approximation of 1 / sqrt(s) (about 2^-22)
-// and two corrections g += (s - g^2) / (2 sqrt(s)) with the residual exact (an
-// fma): 6 float64 operations, rounded like the square root but for an ulp at most.
-__device__ __forceinline__ double sqrt_fast(double s)
+// sqrt(s), correctly rounded, for s >= 0: the hardware's approximation of 1 / sqrt(s)
+// and two Newton corrections g += (s - g^2) / (2 sqrt(s)), the residual exact by an
+// fma, bring g to within an ulp; Tuckerman's test then picks the nearest double: with
+// u the spacing at g, g is too small when s - g^2 > g u and too large when
+// s - g^2 <= -g u (u the spacing below g).  7 float64 operations.
+__device__ __forceinline__ double sqrt_rn(double s)
 {
     const int hi = __double2hiint(s);
-    if (hi < 0x03000000 || hi >= 0x7ff00000) return sqrt(s);  // zero, tiny, infinite, NaN
+    if (hi < 0x2c000000 || hi >= 0x54000000) return sqrt(s);  // zero, tiny, huge, infinite, NaN
     double y;
     asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(s));
     const double h = __hiloint2double(__double2hiint(y) - 0x100000, __double2loint(y));
     double g = __dmul_rn(s, y);
     g = __fma_rn(__fma_rn(-g, g, s), h, g);
-    return __fma_rn(__fma_rn(-g, g, s), h, g);
+    g = __fma_rn(__fma_rn(-g, g, s), h, g);
+    const long long r = __double_as_longlong(__fma_rn(-g, g, s));
+    const long long b = __double_as_longlong(g), e = b >> 52;
+    long long gu = b + ((e - 1075) << 52);  // the bits of g u
+    const long long mag = r & 0x7fffffffffffffffll;
+    if (r >= 0) return __longlong_as_double(b + (mag > gu));
+    if ((b << 12) == 0) gu -= 1ll << 52;
+    return __longlong_as_double(b - (mag >= gu));
 }
 
 // Post-registration pass over flows (T, H, W, 2): valid masks and per-block
@@ -275,7 +284,7 @@ __global__ void __launch_bounds__(256) k_flow_post(const float* __restrict__ flo
             const float2 w = PAIRS ? reinterpret_cast<const float2*>(flow)[p] : make_float2(flow[2 * p], flow[2 * p + 1]);
             if (valid) valid[p] = (w.x >= xlo && w.x < xhi && w.y >= -(float)y && w.y < (float)(H - y)) ? 255 : 0;
             const double u = f2d(w.x), v = f2d(w.y);
-            const double mag = sqrt_fast(__fma_rn(u, u, __dmul_rn(v, v)));
+            const double mag = sqrt_rn(__fma_rn(u, u, __dmul_rn(v, v)));
             s_mag = __dadd_rn(s_mag, mag);
             const long long b = __double_as_longlong(mag);
             if (b > m_mag && b <= 0x7ff0000000000000ll) m_mag = b;  // NaN is passed over, as fmax does
