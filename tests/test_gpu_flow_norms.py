@@ -42,3 +42,21 @@ def test_every_magnitude_is_correctly_rounded(kind):
     want = np.sqrt(d[:, 0] * d[:, 0] + d[:, 1] * d[:, 1])
     assert np.array_equal(got[:, 0], want)
     assert np.array_equal(got[:, 1], want)
+
+
+def test_masks_beyond_the_float32_integers():
+    """Columns over 2^24, where x and W - x are no float32s: x + u >= 0 and x + u < W in float64."""
+    from pyflowreg_gb300.prep import flow_statistics_device
+
+    n = (1 << 24) + 4099
+    x = np.arange(n, dtype=np.float64)
+    rng = np.random.default_rng(5)
+    w = np.zeros((n, 2), dtype=np.float32)
+    # onto the borders and a float32 to either side of them
+    u = np.where(rng.random(n) < 0.5, -x, n - x).astype(np.float32)
+    step = rng.integers(-1, 2, n)
+    w[:, 0] = np.where(step == 0, u, np.nextafter(u, np.where(step < 0, -np.inf, np.inf).astype(np.float32)))
+    m = x + w[:, 0].astype(np.float64)
+    want = np.where((m >= 0) & (m < n), 255, 0).astype(np.uint8)
+    valid = flow_statistics_device(torch.tensor(w, device="cuda").view(1, 1, n, 2))[0]
+    assert np.array_equal(valid.cpu().numpy().reshape(-1), want)
