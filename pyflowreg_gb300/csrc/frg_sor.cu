@@ -1027,9 +1027,11 @@ template <int K>
 cudaError_t run_split32(const Sor32Args& A, const PassTable& T, int n_frames, cudaStream_t st)
 {
     const int strips = A.g.P / 32;
-    if (strips > 2 * kMaxSplitCluster) return SplitLaunch<Ar32<K>, 4, 3, 2, 1>::run(A, T, n_frames, st);
-    if (strips > kMaxSplitCluster) return SplitLaunch<Ar32<K>, 2, 5, 4, 2>::run(A, T, n_frames, st);
-    return SplitLaunch<Ar32<K>, 1, 5, 4, 4>::run(A, T, n_frames, st);
+    return launch_or_taller(strips, strips_per_cta(strips, kMaxSplitCluster), [&](int m) {
+        if (m == 4) return SplitLaunch<Ar32<K>, 4, 3, 2, 1>::run(A, T, n_frames, st);
+        if (m == 2) return SplitLaunch<Ar32<K>, 2, 5, 4, 2>::run(A, T, n_frames, st);
+        return SplitLaunch<Ar32<K>, 1, 5, 4, 4>::run(A, T, n_frames, st);
+    });
 }
 
 }  // namespace
@@ -1085,12 +1087,16 @@ cudaError_t launch_sor_chain(const float* J, long long J_fs, const float* W, lon
         S.omega = omega;
         S.one_m_omega = 1.0f - omega;
         for (int k = 0; k < kMaxK; ++k) S.a_data[k] = k < K ? a_data[k] : 0.0f;
+        cudaError_t e;
         switch (K) {
-            case 1: return run_split32<1>(S, TS, n_frames, st);
-            case 2: return run_split32<2>(S, TS, n_frames, st);
-            case 3: return run_split32<3>(S, TS, n_frames, st);
-            default: return run_split32<4>(S, TS, n_frames, st);
+            case 1: e = run_split32<1>(S, TS, n_frames, st); break;
+            case 2: e = run_split32<2>(S, TS, n_frames, st); break;
+            case 3: e = run_split32<3>(S, TS, n_frames, st); break;
+            default: e = run_split32<4>(S, TS, n_frames, st); break;
         }
+        // refused clusters over 1024 rows: k_sor_chain's have at most 8 CTAs (K <= 2 there)
+        if (e == cudaSuccess || strips_per_cta(g.P / 32, kPortableCluster) || K > 2) return e;
+        cudaGetLastError();
     }
     if (sor_regs_smem(gmax, nt) > (size_t)kSmemLimit) return cudaErrorInvalidValue;
     SorArgs A = make_args(J, J_fs, W, W_fs, lap, lap_fs, coef, coef_fs, du, dv, st_fs, K, g, gmax, 0, 0, a_data, wx,

@@ -159,11 +159,6 @@ cudaError_t launch_pow64(long long n, const double* x, double b, double* out, cu
 
 namespace {
 
-constexpr int kLane64 = 256;       // most rows per CTA a caller may ask for
-constexpr int kG64 = kGMax;        // iterations pipelined per pass, as a template maximum
-constexpr int kMaxStrips64 = 16;   // cluster size (over 8: the non-portable opt-in)
-constexpr int kPortableStrips = 8;
-
 struct Sor64Args : SplitArgs<double> {
     double a_m1[kMaxK];  // a_data - 1
     PowTab64 pw[kMaxK];  // the power's table per channel (null table: the general power)
@@ -298,14 +293,6 @@ struct Ar64 {
     }
 };
 
-// Row strips of a level with at most `rows` rows per CTA (256, 128 or 64).
-void split64(const DiagGeom& g, int rows, int* nc, int* nt)
-{
-    const int n = (g.P + rows - 1) / rows;
-    *nc = n;
-    *nt = ((g.P + n - 1) / n + 31) / 32 * 32;
-}
-
 // Rows per CTA and warps per 32 rows.  32 rows while the launch has at most one CTA
 // per SM (all registers).  With more CTAs what counts is how a frame's cluster packs
 // into the GPCs (14 to 20 SMs): 16 CTAs of 32 rows leave 40 of 152 SMs without a CTA,
@@ -332,21 +319,27 @@ cudaError_t run_split64_m(const Sor64Args& A, const PassTable& T, int m, int n_f
 
 bool sor_chain64_rows_ok(const DiagGeom& g, int rows)
 {
-    if (rows != 64 && rows != 128 && rows != kLane64) return false;
-    int nc, nt;
-    split64(g, rows, &nc, &nt);
-    return nc <= kMaxStrips64;
+    return (rows == 64 || rows == 128 || rows == 256) && (g.P + rows - 1) / rows <= kMaxSplitCluster;
 }
 
 bool sor_chain64_supports(int K, const DiagGeom& g, int n_passes)
 {
     if (K < 1 || K > 4 || (g.P & 31) || g.w < 3 || n_passes < 1 || n_passes > kMaxChain) return false;
-    int nc, nt;
-    split64(g, kLane64, &nc, &nt);
     // 32-bit offsets within a frame: the largest plane index read is (6K + 2) planes of D * P
     const long long plane = (long long)g.D * g.P;
-    // the tallest strips must fit a portable cluster: the fallback of a refused larger cluster
-    return nc <= kPortableStrips && plane * (6 * K + 2) < 0x7fffffffLL;
+    const int strips = g.P / 32;
+    if (strips > kMaxSplitStrips || plane * (6 * K + 2) >= 0x7fffffffLL) return false;
+    if (strips_per_cta(strips, kPortableCluster)) return true;
+    // over 1024 rows: a device that takes clusters of over 8 CTAs
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) return false;
+    const int nc = (strips + 3) / 4;
+    switch (K) {
+        case 1: return SplitLaunch<Ar64<1>, 4, 2, 4, 1>::frames_at_once(dev, nc, 1) > 0;
+        case 2: return SplitLaunch<Ar64<2>, 4, 2, 4, 1>::frames_at_once(dev, nc, 1) > 0;
+        case 3: return SplitLaunch<Ar64<3>, 4, 2, 4, 1>::frames_at_once(dev, nc, 1) > 0;
+        default: return SplitLaunch<Ar64<4>, 4, 2, 4, 1>::frames_at_once(dev, nc, 1) > 0;
+    }
 }
 
 cudaError_t launch_sor_chain64(const double* J, long long J_fs, const double* W, long long W_fs, const double* lap,
@@ -366,7 +359,7 @@ cudaError_t launch_sor_chain64(const double* J, long long J_fs, const double* W,
     T.n = n_passes;
     for (int p = 0; p < n_passes; ++p) {
         const ChainPass& q = passes[p];
-        if (q.G < 1 || q.G > kG64 || q.mode < -1 || q.mode > 3) return cudaErrorInvalidValue;
+        if (q.G < 1 || q.G > kGMax || q.mode < -1 || q.mode > 3) return cudaErrorInvalidValue;
         const bool coef_in = q.mode < 0, store = q.mode >= 0 && q.store_coef;
         T.pk[p] = (q.G << 8) | (store ? kPkStore : 0) | (coef_in ? kPkCoef : 0) |
                   (!coef_in && (q.mode & 2) ? kPkTick : 0) | (!coef_in && (q.mode & 1) ? kPkZero : 0);
@@ -401,14 +394,15 @@ cudaError_t launch_sor_chain64(const double* J, long long J_fs, const double* W,
     }
     // rows per CTA: 32 unless the cluster would pass 16 CTAs; a caller's choice of more is taken
     const int strips = g.P / 32;
-    int m = strips <= kMaxSplitCluster ? 1 : (strips <= 2 * kMaxSplitCluster ? 2 : 4);
-    if (rows >= 64) m = std::max(m, rows >= 128 ? 4 : 2);
-    switch (K) {
-        case 1: return run_split64_m<1>(A, T, m, n_frames, dev, n_sms, st);
-        case 2: return run_split64_m<2>(A, T, m, n_frames, dev, n_sms, st);
-        case 3: return run_split64_m<3>(A, T, m, n_frames, dev, n_sms, st);
-        default: return run_split64_m<4>(A, T, m, n_frames, dev, n_sms, st);
-    }
+    const int asked = rows >= 128 ? 4 : (rows >= 64 ? 2 : 1);
+    return launch_or_taller(strips, std::max(asked, strips_per_cta(strips, kMaxSplitCluster)), [&](int m) {
+        switch (K) {
+            case 1: return run_split64_m<1>(A, T, m, n_frames, dev, n_sms, st);
+            case 2: return run_split64_m<2>(A, T, m, n_frames, dev, n_sms, st);
+            case 3: return run_split64_m<3>(A, T, m, n_frames, dev, n_sms, st);
+            default: return run_split64_m<4>(A, T, m, n_frames, dev, n_sms, st);
+        }
+    });
 }
 
 }  // namespace frg

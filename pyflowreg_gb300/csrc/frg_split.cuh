@@ -15,8 +15,6 @@ namespace frg {
 
 namespace {
 
-constexpr int kMaxSplitStrips = 64;
-constexpr int kMaxSplitCluster = 16;
 constexpr unsigned kMaxTries = 500000u;  // tries of a wait, of at most 2 us each
 
 constexpr int kPkZero = 1, kPkTick = 2, kPkCoef = 4, kPkStore = 8;

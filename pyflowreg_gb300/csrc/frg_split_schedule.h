@@ -18,6 +18,19 @@ constexpr int kRingSlots = 16;  // ring slots: a pixel's coefficients are read f
 constexpr int kRingUse = 2 * (kGMax - 1);
 constexpr int kFoldAhead = kRingSlots - kRingUse;  // most steps a fold may run ahead of the update
 
+constexpr int kMaxSplitStrips = 64;   // strips of 32 rows of a level
+constexpr int kMaxSplitCluster = 16;  // CTAs of a frame (over 8: the non-portable opt-in)
+constexpr int kPortableCluster = 8;
+
+// Strips per CTA (1, 2 or 4), the fewest with which a level's CTAs are a cluster of at
+// most `most`; 0: none is enough.
+FRG_HD int strips_per_cta(int strips, int most)
+{
+    for (int m = 1; m <= 4; m *= 2)
+        if ((strips + m - 1) / m <= most) return m;
+    return 0;
+}
+
 struct PassTable {
     int n;
     int pk[kMaxChain];  // G << 8 | store << 3 | coef << 2 | tick << 1 | zero

@@ -394,6 +394,21 @@ struct SplitLaunch {
     }
 };
 
+// launch(m) with m strips per CTA.  A device that cannot schedule a cluster of over 8
+// CTAs refuses the launch (nothing ran, and the error is not sticky): taller CTAs give
+// the same bits in at most 8, up to 1024 rows.
+template <class Launch>
+cudaError_t launch_or_taller(int strips, int m, Launch launch)
+{
+    cudaError_t e = launch(m);
+    const int taller = strips_per_cta(strips, kPortableCluster);
+    if (e != cudaSuccess && (strips + m - 1) / m > kPortableCluster && taller > m) {
+        cudaGetLastError();
+        e = launch(taller);
+    }
+    return e;
+}
+
 }  // namespace
 
 }  // namespace frg

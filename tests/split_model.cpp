@@ -69,6 +69,8 @@ bool finishes(const Run& R, int ahead)
 
 }  // namespace
 
+extern "C" int split_strips_per_cta(int strips, int most) { return strips_per_cta(strips, most); }
+
 // 0: sound; 1: a wait never ends; 2: a fold takes another pixel than the one that
 // enters; 3: a state or stored coefficients are read before they are surely written;
 // 4: a ring slot is written while its last contents may still be read.

@@ -22,7 +22,7 @@ def model(tmp_path_factory):
     so = str(tmp_path_factory.mktemp("model") / "split_model.so")
     subprocess.run(["g++", "-O2", "-std=c++17", "-shared", "-fPIC", "-I", CSRC, os.path.join(HERE, "split_model.cpp"),
                     "-o", so], check=True)
-    return ctypes.CDLL(so).split_model
+    return ctypes.CDLL(so)
 
 
 def _run(model, h, w, M, FC, iterations, lag):
@@ -30,7 +30,7 @@ def _run(model, h, w, M, FC, iterations, lag):
     n = len(ps)
     G = (ctypes.c_int * n)(*[g for g, _ in ps])
     cont = (ctypes.c_int * n)(*[int(m < 0) for _, m in ps])
-    rc = model(h, w, M, FC, n, G, cont)
+    rc = model.split_model(h, w, M, FC, n, G, cont)
     assert rc == 0, f"{w} columns, {h} rows, M={M}, FC={FC}, lag {lag}: {WHAT[rc]}"
 
 
@@ -48,3 +48,12 @@ def test_folds_take_the_entering_pixels(model, w, lag):
     for M, FC in DIVISIONS:
         for h in (1, 20, 33, 70):
             _run(model, h, w, M, FC, 23, lag)
+
+
+def test_strips_fit_the_cluster(model):
+    """Every level of up to 2048 rows fits a cluster of 16 CTAs, and one of 1024 rows the 8 that any device takes."""
+    for strips in range(1, 65):
+        for most, reach in ((16, 64), (8, 32)):
+            m = model.split_strips_per_cta(strips, most)
+            assert m == next((k for k in (1, 2, 4) if -(-strips // k) <= most), 0)
+            assert (m > 0) == (strips <= reach)
