@@ -3,7 +3,7 @@
 // ahead of them and one warp that waits for both and for the neighbouring CTAs.
 //
 // Every wait is bounded: a wait that runs out is given up, and so is every later
-// one of that warp, so that the kernel ends; the caller of mbar_wait reports it.
+// one of that warp, so that the kernel ends; the frame's result is then NaN.
 #pragma once
 
 #include "frg_internal.h"
@@ -42,6 +42,14 @@ __device__ __forceinline__ void mbar_arrive_expect(unsigned mb, unsigned bytes)
 {
     asm volatile("{\n\t.reg .b64 t;\n\tmbarrier.arrive.expect_tx.release.cta.shared::cta.b64 t, [%0], %1;\n\t}" ::"r"(mb),
                  "r"(bytes)
+                 : "memory");
+}
+
+// A word into the shared memory of the cluster's CTA `rank`.
+__device__ __forceinline__ void st_cluster(unsigned addr, int rank, int v)
+{
+    asm volatile("{\n\t.reg .b32 a;\n\tmapa.shared::cluster.u32 a, %0, %1;\n\tst.shared::cluster.b32 [a], %2;\n\t}" ::"r"(addr), "r"(rank),
+                 "r"(v)
                  : "memory");
 }
 

@@ -59,6 +59,28 @@ struct SplitSmem {
                                     (size_t)plane * sizeof(T) + (size_t)(2 * M * kRingSlots + 2) * 8 + 16;
 };
 
+// NaN in place of this CTA's rows of the result, the border copies included.  Its place
+// is read anew: values kept for it through the solve would cost registers there.
+template <class Ar, int M, int NU>
+__device__ __forceinline__ void void_rows(const typename Ar::Args& A)
+{
+    using R = typename Ar::T;
+    int t, block;
+    asm volatile("mov.u32 %0, %%tid.x;\n\tmov.u32 %1, %%ctaid.x;" : "=r"(t), "=r"(block));
+    const int warp = t >> 5, h = A.g.h, w = A.g.w;
+    const long long f = block / A.nc;
+    const int r = (block % A.nc * M + warp % M) * 32 + (t & 31);
+    if (r >= h || warp >= M * NU) return;
+    const R nan = (R)__int_as_float(0x7fc00000);
+    const int b = Ar::rings && A.out_du && A.ring ? 1 : 0;
+    for (int y = r == 0 ? -b : r; y <= (r == h - 1 ? r + b : r); ++y)
+        for (int c = warp / M - b; c < w + b; c += NU) {
+            const long long o = A.out_du ? f * A.out_fs + (long long)y * A.out_rs + c : f * A.st_fs + r + (long long)(r + c) * A.g.P;
+            (A.out_du ? A.out_du : A.du)[o] = nan;
+            (A.out_du ? A.out_dv : A.dv)[o] = nan;
+        }
+}
+
 // The chained solver, one step of the wavefront divided among warps (see the
 // head of frg_sor64.cu).  MB: CTAs per SM that the registers are to allow.
 // Ar: the arithmetic (types, the fold of a pixel's coefficients, a pixel's update).
@@ -303,20 +325,11 @@ __global__ void __launch_bounds__(32 * SplitRoles<M, NU, FC>::warps, MB) k_sor_s
             b0 = b;
         }
     }
-    if (dead) *gave_up = 1;
-    __syncthreads();
-    if (*gave_up && row_ok && update)  // a wait ran out: the rows' result is void
-        for (int c = warp / M; c < w; c += NU) {
-            const R nan = (R)__int_as_float(0x7fc00000);
-            if (odu) {
-                odu[(long long)r * A.out_rs + c] = nan;
-                odv[(long long)r * A.out_rs + c] = nan;
-            } else {
-                A.du[f * A.st_fs + r + (long long)(r + c) * P] = nan;
-                A.dv[f * A.st_fs + r + (long long)(r + c) * P] = nan;
-            }
-        }
+    // A wait ran out: this CTA's rows are void, and with them what the neighbouring CTAs made of its edge rows.
+    if (dead)
+        for (int i = 0; i < nc; ++i) st_cluster(smem_addr(gave_up), i, 1);
     sync_all();  // no CTA leaves while another may still write into its shared memory
+    if (*gave_up) void_rows<Ar, M, NU>(A);
 }
 
 constexpr int kMaxDevices = 64;
