@@ -104,8 +104,8 @@ __global__ void __launch_bounds__(32 * SplitRoles<M, NU, FC>::warps, MB) k_sor_s
     int* gave_up = reinterpret_cast<int*>(bars + 2 * M * S + 2);
     const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
     const int nc = A.nc;
-    const int cta = nc > 1 ? (int)(blockIdx.x % nc) : 0;
-    const int f = nc > 1 ? (int)(blockIdx.x / nc) : (int)blockIdx.x;
+    const int cta = (int)(blockIdx.x % nc);
+    const int f = (int)(blockIdx.x / nc);
     const bool update = warp < WU;
     const int strip = (update ? warp : Roles::fold(warp)) % M;
     const int row = strip * 32 + lane;  // in the CTA
