@@ -180,6 +180,11 @@ int frg_get_displacement(frg_plan* plan, int n_frames, const float* moving, cons
 int frg_get_displacement_f64(frg_plan* plan, int n_frames, const float* moving, const float* uv_init,
                              double* flow_out, void* stream);
 
+/* How many plans run beside each other, on streams of their own (default 1; no
+ * reference counterpart): a hint for the choice between kernels that give the same
+ * bits, since what counts there is the load of all of them. */
+int frg_plan_set_concurrency(frg_plan* plan, int n_plans);
+
 /* Measurement hooks (no reference counterpart; pyflowreg has no tracing,
  * only wall-clock prints in compensate_recording.py:770-890):
  *   frg_launch_count: kernels launched by this library in this process.

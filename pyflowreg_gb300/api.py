@@ -222,6 +222,11 @@ class Plan:
     def device_bytes(self) -> int:
         return int(self.lib.frg_plan_device_bytes(self.handle))
 
+    def set_concurrency(self, n_plans: int) -> None:
+        """How many plans run beside this one, itself included: a hint for the
+        choice between kernels that give the same bits."""
+        _lib.check(self.lib.frg_plan_set_concurrency(self.handle, int(n_plans)), "frg_plan_set_concurrency")
+
     def set_profiling(self, enable: bool) -> None:
         _lib.check(self.lib.frg_plan_set_profiling(self.handle, 1 if enable else 0))
 
@@ -474,6 +479,7 @@ class LanePlan:
             out_t = torch.empty((T, self.H, self.W, 2), dtype=odt, device=moving_t.device)
         n = self.lane_frames
         if T <= n:
+            self.plans[0].set_concurrency(1)
             return self.plans[0].displacement(moving_t, uv_t, out_t, stream=stream)
         s = stream if stream is not None else torch.cuda.current_stream()
         start = torch.cuda.Event()
@@ -484,6 +490,7 @@ class LanePlan:
             if t0 >= t1:
                 break
             ls.wait_event(start)
+            p.set_concurrency(-(-T // per))
             p.displacement(moving_t[t0:t1], uv_t, out_t[t0:t1], stream=ls)
             done = torch.cuda.Event()
             done.record(ls)
@@ -773,6 +780,7 @@ def _run_host(params, fixed, moving, weight, uv, max_frames=None):
             io.up_done.record(st_up)
         ls.wait_event(io.up_done)
         ls.wait_stream(main)
+        lanes[li].set_concurrency(min(len(lanes), len(parts)))
         lanes[li].displacement(io.dev_in[:k], uv_t, io.dev_out[:k], stream=ls)
         done = torch.cuda.Event()
         done.record(ls)

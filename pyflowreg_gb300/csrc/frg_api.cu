@@ -377,6 +377,7 @@ struct frg_plan {
     float* ones = nullptr;    // (H, W, K) default weight
     float a_data[kMaxK] = {0};
     SorProfile prof;
+    int beside = 1;  // plans that run at a time, this one included
     // FP64 reference-order workspace (precision == FRG_FP64_REFERENCE)
     double* xJ = nullptr;     // (T, 6, K, m*n)
     double* xwp = nullptr;    // (T, K, m*n) weight * psi
@@ -520,7 +521,7 @@ int solve_level(int iterations, int update_lag, const float* J, long long J_fs, 
                 long long st_fs, float* coef, long long coef_fs, int T, int K, const DiagGeom& g,
                 const float* a_data, float wx, float wy, float omega, cudaStream_t st,
                 SorProfile* prof = nullptr, float* rm_du = nullptr, float* rm_dv = nullptr, long long rm_fs = 0,
-                int tune_G = 0, int tune_threads = 0, int tune_variant = 0)
+                int tune_G = 0, int tune_threads = 0, int tune_variant = 0, int beside = 1)
 {
     const SorKind kind = sor_kind(K, g);
     const bool regs = tune_variant >= 1 && sor_regs_supports(K, g);
@@ -538,7 +539,7 @@ int solve_level(int iterations, int update_lag, const float* J, long long J_fs, 
             if (rc) return rc;
         }
         FRG_LAUNCH(launch_sor_chain(J, J_fs, W, W_fs, lap, lap_fs, coef, coef_fs, du, dv, st_fs, T, K, g, cp.data(),
-                                    (int)cp.size(), a_data, wx, wy, omega, st, rm_du, rm_dv, rm_fs));
+                                    (int)cp.size(), a_data, wx, wy, omega, st, rm_du, rm_dv, rm_fs, beside));
         if (timed) {
             int rc = record_event(prof, st);
             if (rc) return rc;
@@ -647,6 +648,14 @@ int frg_plan_set_profiling(frg_plan* plan, int enable)
     plan->prof.used = 0;
     plan->prof.bytes = 0.0;
     plan->prof.launches = 0;
+    return FRG_OK;
+}
+
+int frg_plan_set_concurrency(frg_plan* plan, int n_plans)
+{
+    if (!plan) return fail(FRG_EINVAL, "plan is NULL");
+    if (n_plans < 1) return fail(FRG_EINVAL, "n_plans must be >= 1");
+    plan->beside = n_plans;
     return FRG_OK;
 }
 
@@ -1119,7 +1128,7 @@ int frg_get_displacement(frg_plan* pl, int T, const float* moving, const float* 
         int rc = solve_level(pl->p.iterations, pl->p.update_lag, pl->J, J_fs, L.wdiag, 0, pl->lap, 2 * dp, pl->du,
                              pl->dv, dp, pl->coef, 5 * dp, T, K, L.g, pl->a_data, L.wx, L.wy, (float)pl->p.omega, st,
                              &pl->prof, pl->durm, pl->durm + (long long)T * hw, hw, L.sor_G, L.sor_threads,
-                             L.sor_variant);
+                             L.sor_variant, pl->beside);
         if (rc) return rc;
         // 6. median + accumulate (core/optical_flow.py:607-611)
         const int do_median = std::min(h, w) > 5 ? 1 : 0;

@@ -109,12 +109,13 @@ cudaError_t launch_sor_regs(const float* J, long long J_fs, const float* W, long
                             float wx, float wy, float omega, cudaStream_t st, float* out_du = nullptr,
                             float* out_dv = nullptr, long long out_fs = 0);
 // Every pass of a level in one launch (frg_sor.cu: k_sor_split, or k_sor_chain for
-// levels over 2048 rows): a row starts its next pass as soon as it has finished the
+// large batches and levels over 2048 rows): a row starts its next pass as soon as it has finished the
 // current one, so the passes follow each other without restarting the
 // wavefront.  Pass p is the launch_sor_regs pass (G, mode, store_coef); the
 // level's last pass writes out_du/out_dv when given.  Every level
 // launch_sor_regs serves (in clusters of row strips), w >= 3, at most kMaxChain
-// passes; bit-identical to one launch_sor_regs call per pass.
+// passes; bit-identical to one launch_sor_regs call per pass.  beside: launches of
+// this size that share the GPU (frg_plan_set_concurrency).
 struct ChainPass {
     int G, mode, store_coef;
 };
@@ -123,7 +124,7 @@ cudaError_t launch_sor_chain(const float* J, long long J_fs, const float* W, lon
                              long long lap_fs, float* coef, long long coef_fs, float* du, float* dv, long long st_fs,
                              int n_frames, int K, DiagGeom g, const ChainPass* passes, int n_passes,
                              const float* a_data, float wx, float wy, float omega, cudaStream_t st,
-                             float* out_du = nullptr, float* out_dv = nullptr, long long out_fs = 0);
+                             float* out_du = nullptr, float* out_dv = nullptr, long long out_fs = 0, int beside = 1);
 // The float64 solver's power x^b for one exponent b with |b| <= 1 (frg_dpow.cuh,
 // dpow_b): a table of 2^(e b) (1 / inv_j)^b as double-double over the top 20
 // bits of a positive x (unbiased exponent e in [-17, 46], the top 8 fraction

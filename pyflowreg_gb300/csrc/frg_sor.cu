@@ -557,11 +557,11 @@ __device__ __forceinline__ Coef fold_pk(const SorArgs& A, int pk, const Raw<K>& 
     return fold_m<K>(A, (pk & kPkTick) ? 2 : 0, r);
 }
 
-// The level's rows are cut into A.nc strips of NT rows, one CTA each, the
+// CL: the level's rows are cut into A.nc strips of NT rows, one CTA each, the
 // strips of a frame forming a thread-block cluster, exactly as k_sor_regs's
 // cluster form (edge rows through distributed shared memory, a cluster barrier
 // per step; every CTA runs the same step count).
-template <int K, int G, bool CO>
+template <int K, int G, bool CO, bool CL>
 __global__ void __launch_bounds__(kMaxLane) k_sor_chain(SorArgs A, ChainTable T)
 {
     extern __shared__ __align__(16) float sm[];
@@ -569,9 +569,9 @@ __global__ void __launch_bounds__(kMaxLane) k_sor_chain(SorArgs A, ChainTable T)
     const DiagGeom g = A.g;
     const int P = g.P, h = g.h, w = g.w;
     const int NT = blockDim.x, t = threadIdx.x, lane = t & 31, warp = t >> 5, NW = NT >> 5;
-    const int nc = A.nc;
-    const int strip = (int)(blockIdx.x % nc);
-    const int f = (int)(blockIdx.x / nc);
+    const int nc = CL ? A.nc : 1;
+    const int strip = CL ? (int)(blockIdx.x % nc) : 0;
+    const int f = CL ? (int)(blockIdx.x / nc) : (int)blockIdx.x;
     const int r = strip * NT + t;  // the level row of this thread
     float4* C4 = reinterpret_cast<float4*>(sm);
     float* C1 = sm + 4 * S * NT;
@@ -636,8 +636,13 @@ __global__ void __launch_bounds__(kMaxLane) k_sor_chain(SorArgs A, ChainTable T)
         }
     };
     auto xs = [&](int par, int wp, int dir, int gi) -> float2& { return X[((par * NW + wp) * 2 + dir) * G + gi]; };
-    auto step_barrier = [&]() { cooperative_groups::this_cluster().sync(); };
-    step_barrier();  // every CTA of the cluster is running before any remote write
+    auto step_barrier = [&]() {
+        if constexpr (CL)
+            cooperative_groups::this_cluster().sync();
+        else
+            __syncthreads();
+    };
+    if constexpr (CL) step_barrier();  // every CTA of the cluster is running before any remote write
 
     // the row's current pass (of the update at tau = s - r): index, local start and
     // end, its flags and those of the next pass; the fold (tau + 1) and the prefetch
@@ -691,14 +696,14 @@ __global__ void __launch_bounds__(kMaxLane) k_sor_chain(SorArgs A, ChainTable T)
                     up.x = __shfl_up_sync(0xffffffffu, V1[gi].x, 1);
                     up.y = __shfl_up_sync(0xffffffffu, V1[gi].y, 1);
                     if (lane == 0 && warp > 0) up = xs(pin, warp - 1, 0, gi);
-                    if (t == 0 && strip > 0) up = XE[(pin * 2 + 0) * G + gi];
+                    if (CL && t == 0 && strip > 0) up = XE[(pin * 2 + 0) * G + gi];
                     if (gi == 0) {
                         dn = dn1;
                     } else {
                         dn.x = __shfl_down_sync(0xffffffffu, V1[gi - 1].x, 1);
                         dn.y = __shfl_down_sync(0xffffffffu, V1[gi - 1].y, 1);
                         if (lane == 31 && warp < NW - 1) dn = xs(pin, warp + 1, 1, gi - 1);
-                        if (t == NT - 1 && strip < nc - 1) dn = XE[(pin * 2 + 1) * G + gi - 1];
+                        if (CL && t == NT - 1 && strip < nc - 1) dn = XE[(pin * 2 + 1) * G + gi - 1];
                     }
                     const int c = c0 - 2 * gi;
                     if (gi < Gp && row_ok && c >= 0 && c < w) {
@@ -732,17 +737,19 @@ __global__ void __launch_bounds__(kMaxLane) k_sor_chain(SorArgs A, ChainTable T)
 #pragma unroll
                     for (int gi = 0; gi + 1 < G; ++gi) xs(pout, warp, 1, gi) = V0[gi];
                 }
-                // strip edges: the last row feeds the next strip's "up", the first row the
-                // previous strip's "down", in the neighbouring CTA's shared memory
-                if (t == NT - 1 && strip < nc - 1) {
-                    float2* dst = cooperative_groups::this_cluster().map_shared_rank(XE, strip + 1);
+                if constexpr (CL) {
+                    // strip edges: the last row feeds the next strip's "up", the first row the
+                    // previous strip's "down", in the neighbouring CTA's shared memory
+                    if (t == NT - 1 && strip < nc - 1) {
+                        float2* dst = cooperative_groups::this_cluster().map_shared_rank(XE, strip + 1);
 #pragma unroll
-                    for (int gi = 0; gi < G; ++gi) dst[(pout * 2 + 0) * G + gi] = V0[gi];
-                }
-                if (t == 0 && strip > 0) {
-                    float2* dst = cooperative_groups::this_cluster().map_shared_rank(XE, strip - 1);
+                        for (int gi = 0; gi < G; ++gi) dst[(pout * 2 + 0) * G + gi] = V0[gi];
+                    }
+                    if (t == 0 && strip > 0) {
+                        float2* dst = cooperative_groups::this_cluster().map_shared_rank(XE, strip - 1);
 #pragma unroll
-                    for (int gi = 0; gi + 1 < G; ++gi) dst[(pout * 2 + 1) * G + gi] = V0[gi];
+                        for (int gi = 0; gi + 1 < G; ++gi) dst[(pout * 2 + 1) * G + gi] = V0[gi];
+                    }
                 }
 #pragma unroll
                 for (int gi = 0; gi < G; ++gi) {
@@ -929,23 +936,35 @@ namespace {
 template <int K, int G, bool CO>
 cudaError_t run_chain_t(const SorArgs& A, const ChainTable& T, int n_frames, int nt, cudaStream_t st)
 {
-    {
-        const cudaError_t e = ensure_max_dyn_smem((const void*)k_sor_chain<K, G, CO>, kSmemLimit);
-        if (e != cudaSuccess) return e;
+    if (A.nc == 1) {
+        {
+            const cudaError_t e = ensure_max_dyn_smem((const void*)k_sor_chain<K, G, CO, false>, kSmemLimit);
+            if (e != cudaSuccess) return e;
+        }
+        k_sor_chain<K, G, CO, false><<<n_frames, nt, sor_regs_smem(G, nt), st>>>(A, T);
+        return cudaGetLastError();
     }
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)(n_frames * A.nc));
-    cfg.blockDim = dim3((unsigned)nt);
-    cfg.dynamicSmemBytes = sor_regs_smem(G, nt);
-    cfg.stream = st;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = (unsigned)A.nc;
-    at[0].val.clusterDim.y = 1;
-    at[0].val.clusterDim.z = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, k_sor_chain<K, G, CO>, A, T);
+    if constexpr (K <= 2) {
+        {
+            const cudaError_t e = ensure_max_dyn_smem((const void*)k_sor_chain<K, G, CO, true>, kSmemLimit);
+            if (e != cudaSuccess) return e;
+        }
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3((unsigned)(n_frames * A.nc));
+        cfg.blockDim = dim3((unsigned)nt);
+        cfg.dynamicSmemBytes = sor_regs_smem(G, nt);
+        cfg.stream = st;
+        cudaLaunchAttribute at[1];
+        at[0].id = cudaLaunchAttributeClusterDimension;
+        at[0].val.clusterDim.x = (unsigned)A.nc;
+        at[0].val.clusterDim.y = 1;
+        at[0].val.clusterDim.z = 1;
+        cfg.attrs = at;
+        cfg.numAttrs = 1;
+        return cudaLaunchKernelEx(&cfg, k_sor_chain<K, G, CO, true>, A, T);
+    } else {
+        return cudaErrorInvalidValue;
+    }
 }
 
 template <int K, bool CO>
@@ -1018,11 +1037,10 @@ struct Ar32 {
 // levels over 512 and 1024 rows.  k_sor_chain keeps a frame's rows, updates and folds in
 // one CTA of up to 512 threads, where a step is one thread's chain of five updates and a
 // fold (2400 clocks even for 32 rows); here a step is one update (about 500 clocks) while
-// SMs are free, and with many frames both issue the same instructions.  Whole calls, ms,
-// k_sor_chain -> this: one frame of 512 x 512 x 2 47.7 -> 12.6, 64 frames 56.0 -> 36.0,
-// 128 frames in one plan 64.0 -> 64.1 and in two lanes 64.7 -> 60.8; 16 of 1024 x 1024 x
-// 2 123 -> 50, 4 of 2048 x 2048 x 2 257 -> 87.  Four fold warps and four CTAs per SM: other counts (three to
-// six fold warps, one to four update warps, 64 or 128 rows) measured 0 to 60 % more.
+// SMs are free.  Whole calls, ms, k_sor_chain -> this: one frame of 512 x 512 x 2 47.7 ->
+// 12.6, 64 frames 56.0 -> 36.0; 16 of 1024 x 1024 x 2 123 -> 50, 4 of 2048 x 2048 x 2
+// 257 -> 87.  Four fold warps and four CTAs per SM: other counts (three to six fold
+// warps, one to four update warps, 64 or 128 rows) measured 0 to 60 % more.
 template <int K>
 cudaError_t run_split32(const Sor32Args& A, const PassTable& T, int n_frames, cudaStream_t st)
 {
@@ -1034,13 +1052,39 @@ cudaError_t run_split32(const Sor32Args& A, const PassTable& T, int n_frames, cu
     });
 }
 
+// Whether k_sor_chain with one CTA per frame is the shorter launch; frames: of all
+// launches that share the GPU.  It issues fewer
+// instructions per pixel, but needs 16 warps on an SM to cover a step's chain, where
+// k_sor_split covers it with the warps that it divides the step among: so k_sor_chain
+// for large batches.  Times of a wavefront step, in units of 0.145 us: an SM holds 16
+// warps of k_sor_chain, and a round of r of them takes a + b r; k_sor_split takes one
+// unit per strip of 32 rows and SM (fewer with one strip per frame, more where the
+// clusters of tall levels leave SMs empty, and with four channels, whose folds spill).
+// Measured on 152 SMs for 1 to 16 strips, 0.5 to 64 strips per SM, one to four
+// channels: within 8 % of the shorter of both and 4 % of k_sor_split (which keeps 3 %
+// of advantage here), 5 % below it on average and 44 % at 16 strips per SM (152 frames of
+// 512 x 96, one channel: 8.8 ms against 4.95).  Passes of one to three iterations
+// favour k_sor_chain more, by up to three times.
+bool chain_is_shorter(int K, int strips, long long frames, int n_sms)
+{
+    static constexpr float a[5] = {0.0f, 6.2f, 6.6f, 9.6f, 12.6f}, b[5] = {0.0f, 0.29f, 0.33f, 0.4f, 0.47f};
+    if (strips > kMaxLane / 32 || n_sms < 1) return false;
+    const int per_sm = kMaxLane / 32 / strips, at_once = per_sm * n_sms, rest = (int)(frames % at_once);
+    const long long full = frames / at_once;
+    const float chain = (float)full * (a[K] + b[K] * (float)(per_sm * strips)) +
+                        (rest ? a[K] + b[K] * (float)((rest + n_sms - 1) / n_sms * strips) : 0.0f);
+    const float x = (float)frames * (float)strips / (float)n_sms;
+    const float split = (strips == 1 ? 0.85f * x : (strips <= 10 ? x + 1.0f : 1.08f * x + 1.5f)) * (K == 4 ? 1.27f : 1.0f);
+    return 1.03f * chain < split;
+}
+
 }  // namespace
 
 cudaError_t launch_sor_chain(const float* J, long long J_fs, const float* W, long long W_fs, const float* lap,
                              long long lap_fs, float* coef, long long coef_fs, float* du, float* dv, long long st_fs,
                              int n_frames, int K, DiagGeom g, const ChainPass* passes, int n_passes,
                              const float* a_data, float wx, float wy, float omega, cudaStream_t st, float* out_du,
-                             float* out_dv, long long out_fs)
+                             float* out_dv, long long out_fs, int beside)
 {
     int nc = 0, nt = 0;
     regs_split(K, g, &nc, &nt);
@@ -1061,8 +1105,12 @@ cudaError_t launch_sor_chain(const float* J, long long J_fs, const float* W, lon
         gmax = q.G > gmax ? q.G : gmax;
     }
     for (int p = n_passes; p < kMaxChain; ++p) T.pk[p] = 1 << 8;
+    int dev = 0, n_sms = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&n_sms, cudaDevAttrMultiProcessorCount, dev);
+    if (e != cudaSuccess) return e;
     // up to 2048 rows: clusters of at most 16 CTAs of 128 rows
-    if (g.P / 32 <= kMaxSplitStrips) {
+    if (g.P / 32 <= kMaxSplitStrips && !chain_is_shorter(K, g.P / 32, (long long)n_frames * beside, n_sms)) {
         for (int p = 0; p < kMaxChain; ++p) TS.pk[p] = T.pk[p];
         Sor32Args S = {};
         S.J = J;
@@ -1087,7 +1135,6 @@ cudaError_t launch_sor_chain(const float* J, long long J_fs, const float* W, lon
         S.omega = omega;
         S.one_m_omega = 1.0f - omega;
         for (int k = 0; k < kMaxK; ++k) S.a_data[k] = k < K ? a_data[k] : 0.0f;
-        cudaError_t e;
         switch (K) {
             case 1: e = run_split32<1>(S, TS, n_frames, st); break;
             case 2: e = run_split32<2>(S, TS, n_frames, st); break;
@@ -1105,8 +1152,9 @@ cudaError_t launch_sor_chain(const float* J, long long J_fs, const float* W, lon
     switch (K) {
         case 1: return run_chain<1>(A, T, co, gmax, n_frames, nt, st);
         case 2: return run_chain<2>(A, T, co, gmax, n_frames, nt, st);
+        case 3: return run_chain<3>(A, T, co, gmax, n_frames, nt, st);
+        default: return run_chain<4>(A, T, co, gmax, n_frames, nt, st);
     }
-    return cudaErrorInvalidValue;  // more channels: levels of at most 512 rows, above
 }
 
 cudaError_t launch_sor_fused(const float* J, long long J_fs, const float* W, long long W_fs, const float* lap,
