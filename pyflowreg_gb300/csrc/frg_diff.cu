@@ -1126,7 +1126,7 @@ __device__ __forceinline__ void fwd_window_steps(typename Vec2T<T>::type* sS, co
 }
 
 template <typename T, int NQ>
-__global__ void __launch_bounds__(NQ <= 3 ? 512 : 128, NQ <= 3 && sizeof(T) == 4 ? 2 : 1) kd_rb_window(const T* __restrict__ coef, const T* __restrict__ s0,
+__global__ void __launch_bounds__(NQ <= 3 ? 512 : 128, NQ <= 3 ? 2 : 1) kd_rb_window(const T* __restrict__ coef, const T* __restrict__ s0,
                                                                      T* __restrict__ s_out, T* __restrict__ hist,
                                                                      long long slot, int h, int w, int nh, int TX, int TY,
                                                                      AdjTable tab, T ax, T ay, T omega, T eps, int gs)
@@ -1833,23 +1833,26 @@ int rb_window_pixels(int nh, int tile)
     return q <= (tile == 32 ? 3 : 6) ? q : 0;
 }
 
-// nh half-sweeps of a window in one launch (rb_window_pixels(nh, tile) > 0).
+// nh half-sweeps of a window in one launch (rb_window_pixels(nh, tile) > 0); float32.
 template <typename T>
 cudaError_t rb_window(const T* coef, const T* s0, T* s_out, T* hist, long long slot, int F, int h, int w, int nh, int tile,
                       const AdjTable& tab, double ax, double ay, double omega, double eps, int gs, cudaStream_t st)
 {
-    const int bd = tile * tile / 2, n1 = (tile + 2 * nh + 2) * ((tile + 2 * nh + 2) / 2);
-    const dim3 grid((w + tile - 1) / tile, (h + tile - 1) / tile, F);
-    const auto run = [&](auto kern) -> cudaError_t {
-        const cudaError_t e = ensure_max_dyn_smem((const void*)kern, (int)kAdjWindowSmem);
-        if (e != cudaSuccess) return e;
-        kern<<<grid, bd, 4 * (size_t)n1 * sizeof(T), st>>>(coef, s0, s_out, hist, slot, h, w, nh, tile, tile, tab, (T)ax,
-                                                            (T)ay, (T)omega, (T)eps, gs);
-        return cudaGetLastError();
-    };
     const int q = rb_window_pixels(nh, tile);
-    if (q == 0) return cudaErrorInvalidValue;
-    return q <= 3 ? run(kd_rb_window<T, 3>) : run(kd_rb_window<T, 6>);
+    if (q == 0 || sizeof(T) != 4) return cudaErrorInvalidValue;
+    if constexpr (sizeof(T) == 4) {
+        const int bd = tile * tile / 2, n1 = (tile + 2 * nh + 2) * ((tile + 2 * nh + 2) / 2);
+        const dim3 grid((w + tile - 1) / tile, (h + tile - 1) / tile, F);
+        const auto run = [&](auto kern) -> cudaError_t {
+            const cudaError_t e = ensure_max_dyn_smem((const void*)kern, (int)kAdjWindowSmem);
+            if (e != cudaSuccess) return e;
+            kern<<<grid, bd, 4 * (size_t)n1 * sizeof(T), st>>>(coef, s0, s_out, hist, slot, h, w, nh, tile, tile, tab, (T)ax,
+                                                                (T)ay, (T)omega, (T)eps, gs);
+            return cudaGetLastError();
+        };
+        return q <= 3 ? run(kd_rb_window<T, 3>) : run(kd_rb_window<T, 6>);
+    }
+    return cudaErrorInvalidValue;
 }
 
 cudaError_t reduce_slots(double* part, int F, long long n_slots, double* galpha, cudaStream_t st)

@@ -205,10 +205,14 @@ int make_adj_tables(frg_diff_plan* pl)
     return FRG_OK;
 }
 
-// The ring table of a window of n_half half-sweeps that kd_rb_window can run; NULL: none.
+// The ring table of a window of n_half half-sweeps that kd_rb_window can run; NULL:
+// none.  Not in float64, whose pipe bounds the half-sweeps: the window's halo is more
+// work for it than the launches cost (4 frames of 256 x 256, update_lag 6: forward 9.3 ms
+// with windows, 5.4 without; only single frames of 130 to 200 pixels a side gained).
+template <typename T>
 const frg::diff::AdjTable* window_table(const frg_diff_plan* pl, int n_half)
 {
-    if (!pl->adj_tile || !frg::diff::rb_window_pixels(n_half, pl->adj_tile)) return nullptr;
+    if (sizeof(T) == 8 || !pl->adj_tile || !frg::diff::rb_window_pixels(n_half, pl->adj_tile)) return nullptr;
     for (int q = 0; q < 2; ++q)
         if (pl->adj_nh[q] == n_half) return &pl->adj_tab[q];
     return nullptr;
@@ -308,7 +312,7 @@ int run_forward(frg_diff_plan* pl, int F, const T* fixed, const T* moving, const
         const size_t plane2 = (size_t)F * 2 * hw;
         const size_t slot = (size_t)F * 2 * h * ((w + 1) / 2);
         bool fused = true;
-        for (int k = 0; k < pl->n_ticks; ++k) fused = fused && window_table(pl, 2 * std::min(lag, I - k * lag)) != nullptr;
+        for (int k = 0; k < pl->n_ticks; ++k) fused = fused && window_table<T>(pl, 2 * std::min(lag, I - k * lag)) != nullptr;
         if (fused) {
             // one launch per window, from one tick's state straight into the next one's checkpoint
             for (int k = 0; k < pl->n_ticks; ++k) {
@@ -320,7 +324,7 @@ int run_forward(frg_diff_plan* pl, int F, const T* fixed, const T* moving, const
                 DLAUNCH(1, tick<T>(J, (const T*)L.Wl, s0, uv, F, K, h, w, pl->a_data, kEps, L.ax, L.ay, coef, (T*)nullptr,
                                    st));
                 DLAUNCH(1, rb_window<T>(coef, s0, s1, pl->store_sweeps ? (T*)L.ck_sweeps + (size_t)(2 * k * lag) * slot : nullptr,
-                                        (long long)slot, F, h, w, n_half, pl->adj_tile, *window_table(pl, n_half), L.ax,
+                                        (long long)slot, F, h, w, n_half, pl->adj_tile, *window_table<T>(pl, n_half), L.ax,
                                         L.ay, om, kEps, pl->gs, st));
                 s = s1;
             }
@@ -358,7 +362,7 @@ int rerun_window(frg_diff_plan* pl, const DLevel& L, int F, const T* coef, const
 {
     using namespace frg::diff;
     const double om = pl->p.omega;
-    if (const AdjTable* tb = window_table(pl, n_half)) {
+    if (const AdjTable* tb = window_table<T>(pl, n_half)) {
         DLAUNCH(1, rb_window<T>(coef, s0, s, hist, (long long)slot, F, L.h, L.w, n_half, pl->adj_tile, *tb, L.ax, L.ay, om,
                                 kEps, pl->gs, st));
         return FRG_OK;
