@@ -145,7 +145,7 @@ __global__ void k_prep_cols(PrepArgs A, const S* __restrict__ tmp, float* __rest
 // taps split into two float32s, left + right exact as a two-sum), which gives the
 // bits of the float64 sum; samples stored in float64 are summed in float64.
 // 200 frames of 512 x 512 x 2, sigma 1, with the flow statistics below: 19.1 ms
-// before, 4.39 ms now.
+// before, 4.28 ms now.
 constexpr int kPrepTile = 32;
 
 template <typename S, typename F>
@@ -250,7 +250,7 @@ __device__ __forceinline__ double sqrt_rn(double s)
 
 // Post-registration pass over flows (T, H, W, 2): valid masks and per-block
 // partials (sum |w|, max |w|, sum div, sum u, sum v) at part[(f, block)][5]; a
-// block takes 256 columns of kPostRows rows.
+// block takes 256 columns of ROWS rows.
 //
 // np.gradient's divergence (central inside, one-sided at the edges) summed over a
 // row telescopes: sum du/dx = -3/2 u[0] + 1/2 u[1] - 1/2 u[W-2] + 3/2 u[W-1], and
@@ -259,15 +259,18 @@ __device__ __forceinline__ double sqrt_rn(double s)
 // x + u >= 0 and x + u < W are u >= -x and u < W - x, exact in float32 (beyond 2^24
 // with -x and W - x rounded up: no float32 lies between).  About 12
 // float64 operations per pixel are left of about 45.
-constexpr int kPostRows = 16;
+// A block of small frames takes fewer rows, since the rows are its chain (one frame of
+// 256 x 256 44 us with 16 rows, 37 with four), by the frame's size alone, so that a
+// frame's sums do not depend on the batch that it comes in.
+constexpr int kPostRows = 16, kPostRowsSmall = 4;
 
 // PAIRS: the flow lies on an 8-byte boundary, so (u, v) is one load.
-template <bool PAIRS>
+template <bool PAIRS, int ROWS>
 __global__ void __launch_bounds__(256) k_flow_post(const float* __restrict__ flow, int H, int W, uint8_t* __restrict__ valid,
                                                    double* __restrict__ part)
 {
     const int x = blockIdx.x * 256 + threadIdx.x;
-    const int y0 = blockIdx.y * kPostRows;
+    const int y0 = blockIdx.y * ROWS;
     const long long f = blockIdx.z;
     double s_mag = 0, s_div = 0, s_u = 0, s_v = 0;
     long long m_mag = 0;  // the bits of the largest magnitude
@@ -278,7 +281,7 @@ __global__ void __launch_bounds__(256) k_flow_post(const float* __restrict__ flo
         const double ex = edge(x, W);
         const bool inner_x = x > 0 && x < W - 1;
         const float xlo = -__int2float_rd(x), xhi = __int2float_ru(W - x);
-        const int y1 = min(y0 + kPostRows, H);
+        const int y1 = min(y0 + ROWS, H);
 #pragma unroll 4
         for (int y = y0; y < y1; ++y) {
             const long long p = (f * H + y) * W + x;
@@ -303,21 +306,18 @@ __global__ void __launch_bounds__(256) k_flow_post(const float* __restrict__ flo
     }
     __shared__ double red[5][8];
     const int t = threadIdx.x;
-    double m = __longlong_as_double(m_mag);
-    for (int o = 16; o > 0; o >>= 1) {
-        s_mag += __shfl_down_sync(~0u, s_mag, o);
-        m = fmax(m, __shfl_down_sync(~0u, m, o));
-        s_div += __shfl_down_sync(~0u, s_div, o);
-        s_u += __shfl_down_sync(~0u, s_u, o);
-        s_v += __shfl_down_sync(~0u, s_v, o);
-    }
-    if ((t & 31) == 0) {
-        const int w = t >> 5;
-        red[0][w] = s_mag;
-        red[1][w] = m;
-        red[2][w] = s_div;
-        red[3][w] = s_u;
-        red[4][w] = s_v;
+    // the warp's four sums at once: half of the lanes go on with two of them, a quarter with one (6 float64 additions
+    // where one sum at a time takes 20); the maximum as integers
+    for (int o = 16; o > 0; o >>= 1) m_mag = max(m_mag, __shfl_xor_sync(~0u, m_mag, o));
+    const bool h16 = t & 16, h8 = t & 8;
+    const double p0 = __dadd_rn(h16 ? s_u : s_mag, __shfl_xor_sync(~0u, h16 ? s_mag : s_u, 16));
+    const double p1 = __dadd_rn(h16 ? s_v : s_div, __shfl_xor_sync(~0u, h16 ? s_div : s_v, 16));
+    double q = __dadd_rn(h8 ? p1 : p0, __shfl_xor_sync(~0u, h8 ? p0 : p1, 8));
+    for (int o = 4; o > 0; o >>= 1) q = __dadd_rn(q, __shfl_xor_sync(~0u, q, o));
+    if ((t & 7) == 0) {
+        const int i = (t & 31) >> 3;  // magnitude, divergence, u, v
+        red[i == 0 ? 0 : i + 1][t >> 5] = q;
+        if (i == 0) red[1][t >> 5] = __longlong_as_double(m_mag);
     }
     __syncthreads();
     if (t < 5) {
@@ -433,11 +433,14 @@ cudaError_t launch_preprocess(const float* raw, const double* raw64, int T, int 
 cudaError_t launch_flow_post(const float* flow, int T, int H, int W, uint8_t* valid, double* part, double* stats,
                              cudaStream_t st)
 {
-    const dim3 grid((unsigned)((W + 255) / 256), (unsigned)((H + kPostRows - 1) / kPostRows), (unsigned)T);
-    if (((uintptr_t)flow & 7) == 0)
-        k_flow_post<true><<<grid, 256, 0, st>>>(flow, H, W, valid, part);
-    else
-        k_flow_post<false><<<grid, 256, 0, st>>>(flow, H, W, valid, part);
+    const int bx = (W + 255) / 256;
+    const bool small = (long long)bx * ((H + kPostRows - 1) / kPostRows) < 64;
+    const int rows = small ? kPostRowsSmall : kPostRows;
+    const dim3 grid((unsigned)bx, (unsigned)((H + rows - 1) / rows), (unsigned)T);
+    const bool pairs = ((uintptr_t)flow & 7) == 0;
+    const auto kern = pairs ? (small ? k_flow_post<true, kPostRowsSmall> : k_flow_post<true, kPostRows>)
+                            : (small ? k_flow_post<false, kPostRowsSmall> : k_flow_post<false, kPostRows>);
+    kern<<<grid, 256, 0, st>>>(flow, H, W, valid, part);
     k_flow_stats<<<T, 256, 0, st>>>(part, (long long)grid.y * grid.x, (double)H * W, stats);
     return cudaGetLastError();
 }
