@@ -27,21 +27,24 @@ __device__ __forceinline__ double ddiv(double a, double b) { return __ddiv_rn(a,
 // Resize with numba typing (util/resize_util.py:116-141): float32 input and
 // products, float64 accumulator, float32 result (stored as float or double).
 // ---------------------------------------------------------------------------
-// Horizontal pass.  A block holds RW rows of one plane in shared memory, columns
-// first (pitch RW + 1: no bank conflicts either way), so that a warp's lanes take
-// RW rows of the same 32 / RW output columns: the taps are conflict-free at every
-// scale and the tap table is read once per warp.  The outputs go through shared
-// memory to be stored row by row.  What bounds it is the float64 additions of the
-// general form (64 issue slots each), which DfSum keeps off that pipe.
+// Horizontal pass.  A block holds kRxRows rows of one plane in shared memory, columns
+// first (odd pitch: no bank conflicts either way), so that a warp's lanes take eight
+// rows of the same four output columns: the taps are conflict-free at every scale and
+// the tap table is read once per warp.  The outputs go through shared memory to be
+// stored row by row.  What bounds it is the float64 additions that a plain sum has (64
+// issue slots each), which DfSum keeps off that pipe, then the latency of the loads:
+// eight rows per block against 32, all levels of 100 frames of 512 x 512 x 2 8.2 and
+// 9.8 ms, of 16 frames 1.7 and 2.6.
 constexpr int kRxCols = 64;  // output columns per store tile
+constexpr int kRxRows = 8;
 
-template <typename Tin, int RW>
+template <typename Tin>
 __global__ void __launch_bounds__(256) kx_resize_h_rows(const Tin* __restrict__ src, long long fs, long long ps, long long rs,
                                                         long long cs, int n_planes, int ih, int iw, float* __restrict__ dst,
                                                         int ow, const int32_t* __restrict__ ix,
                                                         const float* __restrict__ wx, int P, float err)
 {
-    constexpr int pitch = RW + 1, XW = 32 / RW, XB = 8 * XW;  // columns per warp and per block at a time
+    constexpr int RW = kRxRows, pitch = RW + 1, XW = 32 / RW, XB = 8 * XW;  // columns per warp and per block at a time
     extern __shared__ float sx[];
     float* tile = sx + (size_t)iw * pitch;  // [RW][kRxCols + 1]
     const int y0 = blockIdx.x * RW;
@@ -80,11 +83,12 @@ __global__ void __launch_bounds__(256) kx_resize_h_rows(const Tin* __restrict__ 
     }
 }
 
-// The general form, for rows too long for shared memory.
+// One output per thread from memory, for few rows (more blocks) and rows too long for
+// shared memory.
 template <typename Tin>
 __global__ void kx_resize_h(const Tin* __restrict__ src, long long fs, long long ps, long long rs, long long cs,
                             int n_planes, int ih, float* __restrict__ dst, int ow, const int32_t* __restrict__ ix,
-                            const float* __restrict__ wx, int P)
+                            const float* __restrict__ wx, int P, float err)
 {
     const int x = blockIdx.x * blockDim.x + threadIdx.x;
     const int y = blockIdx.y;
@@ -92,20 +96,22 @@ __global__ void kx_resize_h(const Tin* __restrict__ src, long long fs, long long
     if (x >= ow) return;
     const int f = fp / n_planes, pl = fp - f * n_planes;
     const Tin* row = src + f * fs + pl * ps + (long long)y * rs;
-    double s = 0.0;
-    for (int p = 0; p < P; ++p) {
-        const float a = (float)row[(long long)ix[(long long)x * P + p] * cs];
-        s = dadd(s, f2d(__fmul_rn(a, wx[(long long)x * P + p])));
+    const int32_t* ixr = ix + (long long)x * P;
+    const float* wxr = wx + (long long)x * P;
+    DfSum acc;
+#pragma unroll 4
+    for (int p = 0; p < P; ++p) acc.add(__fmul_rn((float)__ldg(row + (long long)__ldg(ixr + p) * cs), __ldg(wxr + p)));
+    float v;
+    if (!acc.value(err, &v)) {
+        double s = 0.0;
+        for (int p = 0; p < P; ++p) s = dadd(s, f2d(__fmul_rn((float)row[(long long)ixr[p] * cs], wxr[p])));
+        v = (float)s;
     }
-    dst[((long long)fp * ih + y) * ow + x] = (float)s;
+    dst[((long long)fp * ih + y) * ow + x] = v;
 }
 
 // ring: 0 none, 1 edge-replicated ring (add_boundary), 2 zero ring
 // (cv2.copyMakeBorder BORDER_CONSTANT 0, core/optical_flow.py:565-568).
-// Four output rows per thread: their sums are independent, which covers the
-// latency of the loads and of the dependent additions.
-constexpr int kRvx = 4;
-
 template <typename Tout>
 __global__ void kx_resize_v(const float* __restrict__ src, int n_planes, int ih, int ow, Tout* __restrict__ dst,
                             long long fs, long long ps, long long rs, int oh, int ring,
@@ -113,65 +119,54 @@ __global__ void kx_resize_v(const float* __restrict__ src, int n_planes, int ih,
 {
     const int pad = ring ? 1 : 0;
     const int xo = blockIdx.x * blockDim.x + threadIdx.x;
+    const int yo = blockIdx.y;
     const int fp = blockIdx.z;
     if (xo >= ow + 2 * pad) return;
     const int f = fp / n_planes, pl = fp - f * n_planes;
+    Tout* out = dst + f * fs + pl * ps + (long long)yo * rs + xo;
+    const bool inside = xo >= pad && xo < ow + pad && yo >= pad && yo < oh + pad;
+    if (!inside && ring == 2) {
+        *out = (Tout)0;
+        return;
+    }
     const int x = xclamp(xo - pad, 0, ow - 1);
+    const int y = xclamp(yo - pad, 0, oh - 1);
     const float* col = src + (long long)fp * ih * ow + x;
-    const int32_t* iyr[kRvx];
-    const float* wyr[kRvx];
-#pragma unroll
-    for (int q = 0; q < kRvx; ++q) {
-        const int y = xclamp((int)blockIdx.y * kRvx + q - pad, 0, oh - 1);
-        iyr[q] = iy + (long long)y * P;
-        wyr[q] = wy + (long long)y * P;
+    const int32_t* iyr = iy + (long long)y * P;
+    const float* wyr = wy + (long long)y * P;
+    DfSum acc;
+#pragma unroll 4
+    for (int p = 0; p < P; ++p) acc.add(__fmul_rn(__ldg(col + (long long)__ldg(iyr + p) * ow), __ldg(wyr + p)));
+    float v;
+    if (!acc.value(err, &v)) {
+        double s = 0.0;
+        for (int p = 0; p < P; ++p) s = dadd(s, f2d(__fmul_rn(col[(long long)iyr[p] * ow], wyr[p])));
+        v = (float)s;
     }
-    DfSum acc[kRvx];
-    for (int p = 0; p < P; ++p) {
-#pragma unroll
-        for (int q = 0; q < kRvx; ++q)
-            acc[q].add(__fmul_rn(__ldg(col + (long long)__ldg(iyr[q] + p) * ow), __ldg(wyr[q] + p)));
-    }
-#pragma unroll
-    for (int q = 0; q < kRvx; ++q) {
-        const int yo = blockIdx.y * kRvx + q;
-        if (yo >= oh + 2 * pad) break;
-        float v;
-        if (!acc[q].value(err, &v)) {
-            double s = 0.0;
-            for (int p = 0; p < P; ++p) s = dadd(s, f2d(__fmul_rn(col[(long long)iyr[q][p] * ow], wyr[q][p])));
-            v = (float)s;
-        }
-        const bool inside = xo >= pad && xo < ow + pad && yo >= pad && yo < oh + pad;
-        dst[f * fs + pl * ps + (long long)yo * rs + xo] = !inside && ring == 2 ? (Tout)0 : (Tout)v;
-    }
+    *out = (Tout)v;
 }
 
-// Rows per block by the shared memory they take: 32 while two blocks share an SM
-// (rows up to 817 columns), then 16 and 8 (up to 3357 and 6399), else rows read from
-// memory.  Everything but the solver on 100 frames of 512 x 512 x 2, this, the
-// vertical pass and kx_warp included: 54 ms before, 38 ms now.
+// Rows of up to 6399 columns in shared memory, from 256 blocks on; with fewer blocks one
+// output per thread covers the loads better.  All levels' passes: one frame of 256 x 256
+// 270 us per thread and 386 in rows, of 512 x 512 x 2 543 and 694, four of 256 x 256 x 2
+// 407 and 410, four of 512 x 512 x 2 1039 and 824.
 template <typename Tin>
 static cudaError_t launch_x_resize_h(const Tin* src, long long fs, long long ps, long long rs, long long cs, int n_frames,
                                      int n_planes, int ih, int iw, float* dst, int ow, const int32_t* ix,
                                      const float* wx, int P, cudaStream_t st)
 {
-    const auto bytes = [&](int rw) { return ((size_t)iw * (rw + 1) + (size_t)rw * (kRxCols + 1)) * sizeof(float); };
+    const size_t bytes = ((size_t)iw * (kRxRows + 1) + (size_t)kRxRows * (kRxCols + 1)) * sizeof(float);
     constexpr size_t most = 232448;
-    const auto run = [&](auto kern, int rw) -> cudaError_t {
-        const cudaError_t e = ensure_max_dyn_smem((const void*)kern, (int)most);
+    const long long row_blocks = (long long)((ih + kRxRows - 1) / kRxRows) * n_frames * n_planes;
+    if (bytes <= most && row_blocks >= 256 && n_frames * n_planes <= 65535) {
+        const cudaError_t e = ensure_max_dyn_smem((const void*)kx_resize_h_rows<Tin>, (int)most);
         if (e != cudaSuccess) return e;
-        dim3 grd((ih + rw - 1) / rw, n_frames * n_planes);
-        kern<<<grd, 256, bytes(rw), st>>>(src, fs, ps, rs, cs, n_planes, ih, iw, dst, ow, ix, wx, P, kDfErr(P));
+        dim3 grd((ih + kRxRows - 1) / kRxRows, n_frames * n_planes);
+        kx_resize_h_rows<Tin><<<grd, 256, bytes, st>>>(src, fs, ps, rs, cs, n_planes, ih, iw, dst, ow, ix, wx, P, kDfErr(P));
         return cudaGetLastError();
-    };
-    if (n_frames * n_planes <= 65535) {
-        if (bytes(32) <= most / 2) return run(kx_resize_h_rows<Tin, 32>, 32);
-        if (bytes(16) <= most) return run(kx_resize_h_rows<Tin, 16>, 16);
-        if (bytes(8) <= most) return run(kx_resize_h_rows<Tin, 8>, 8);
     }
-    dim3 blk(128), grd((ow + 127) / 128, ih, n_frames * n_planes);
-    kx_resize_h<Tin><<<grd, blk, 0, st>>>(src, fs, ps, rs, cs, n_planes, ih, dst, ow, ix, wx, P);
+    dim3 blk(64), grd((ow + 63) / 64, ih, n_frames * n_planes);
+    kx_resize_h<Tin><<<grd, blk, 0, st>>>(src, fs, ps, rs, cs, n_planes, ih, dst, ow, ix, wx, P, kDfErr(P));
     return cudaGetLastError();
 }
 
@@ -196,7 +191,7 @@ static cudaError_t launch_x_resize_v(const float* src, int n_frames, int n_plane
 {
     const int owp = ow + (ring ? 2 : 0), ohp = oh + (ring ? 2 : 0);
     const int bx = owp >= 96 ? 128 : (owp >= 48 ? 64 : 32);
-    dim3 blk(bx), grd((owp + bx - 1) / bx, (ohp + kRvx - 1) / kRvx, n_frames * n_planes);
+    dim3 blk(bx), grd((owp + bx - 1) / bx, ohp, n_frames * n_planes);
     kx_resize_v<Tout><<<grd, blk, 0, st>>>(src, n_planes, ih, ow, dst, fs, ps, rs, oh, ring, iy, wy, P, kDfErr(P));
     return cudaGetLastError();
 }
