@@ -300,7 +300,9 @@ class Plan:
         chosen = {}
         for i in list(range(len(tun) - 1, -1, -1))[:n_levels]:
             best = None
-            for rows in (0, 256, 128, 64):
+            # the heights that are another launch than the default's (32 rows up to 512, 64 up to 1024, 128 above)
+            height = tun[i][3]
+            for rows in (0,) + ((128,) if height <= 1024 else ()) + ((64,) if height <= 512 else ()):
                 try:
                     self.set_level_tuning(i, 0, rows)
                 except ValueError:
