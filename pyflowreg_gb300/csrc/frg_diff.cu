@@ -1839,7 +1839,7 @@ cudaError_t rb_window(const T* coef, const T* s0, T* s_out, T* hist, long long s
                       const AdjTable& tab, double ax, double ay, double omega, double eps, int gs, cudaStream_t st)
 {
     const int q = rb_window_pixels(nh, tile);
-    if (q == 0 || sizeof(T) != 4) return cudaErrorInvalidValue;
+    if (q == 0) return cudaErrorInvalidValue;
     if constexpr (sizeof(T) == 4) {
         const int bd = tile * tile / 2, n1 = (tile + 2 * nh + 2) * ((tile + 2 * nh + 2) / 2);
         const dim3 grid((w + tile - 1) / tile, (h + tile - 1) / tile, F);
@@ -1851,8 +1851,9 @@ cudaError_t rb_window(const T* coef, const T* s0, T* s_out, T* hist, long long s
             return cudaGetLastError();
         };
         return q <= 3 ? run(kd_rb_window<T, 3>) : run(kd_rb_window<T, 6>);
+    } else {
+        return cudaErrorInvalidValue;
     }
-    return cudaErrorInvalidValue;
 }
 
 cudaError_t reduce_slots(double* part, int F, long long n_slots, double* galpha, cudaStream_t st)

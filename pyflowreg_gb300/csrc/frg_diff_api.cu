@@ -212,9 +212,9 @@ int make_adj_tables(frg_diff_plan* pl)
 template <typename T>
 const frg::diff::AdjTable* window_table(const frg_diff_plan* pl, int n_half)
 {
-    if (sizeof(T) == 8 || !pl->adj_tile || !frg::diff::rb_window_pixels(n_half, pl->adj_tile)) return nullptr;
+    const bool serves = sizeof(T) == 4 && pl->adj_tile && frg::diff::rb_window_pixels(n_half, pl->adj_tile);
     for (int q = 0; q < 2; ++q)
-        if (pl->adj_nh[q] == n_half) return &pl->adj_tab[q];
+        if (serves && pl->adj_nh[q] == n_half) return &pl->adj_tab[q];
     return nullptr;
 }
 
