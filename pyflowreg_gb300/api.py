@@ -421,6 +421,8 @@ class LanePlan:
         self.device = torch.cuda.current_device()
         self.lane_frames = -(-int(max_frames) // int(lanes))
         self.plans = [Plan(params, H, W, K, self.lane_frames) for _ in range(int(lanes))]
+        for p in self.plans:
+            p.set_concurrency(len(self.plans))
         self.max_frames = self.lane_frames * len(self.plans)
         self.streams = [torch.cuda.Stream() for _ in self.plans]
 
@@ -482,7 +484,10 @@ class LanePlan:
         n = self.lane_frames
         if T <= n:
             self.plans[0].set_concurrency(1)
-            return self.plans[0].displacement(moving_t, uv_t, out_t, stream=stream)
+            try:
+                return self.plans[0].displacement(moving_t, uv_t, out_t, stream=stream)
+            finally:
+                self.plans[0].set_concurrency(len(self.plans))
         s = stream if stream is not None else torch.cuda.current_stream()
         start = torch.cuda.Event()
         start.record(s)

@@ -1052,30 +1052,64 @@ cudaError_t run_split32(const Sor32Args& A, const PassTable& T, int n_frames, cu
     });
 }
 
-// Whether k_sor_chain with one CTA per frame is the shorter launch; frames: of all
-// launches that share the GPU.  It issues fewer
-// instructions per pixel, but needs 16 warps on an SM to cover a step's chain, where
-// k_sor_split covers it with the warps that it divides the step among: so k_sor_chain
-// for large batches.  Times of a wavefront step, in units of 0.145 us: an SM holds 16
-// warps of k_sor_chain, and a round of r of them takes a + b r; k_sor_split takes one
-// unit per strip of 32 rows and SM (fewer with one strip per frame, more where the
-// clusters of tall levels leave SMs empty, and with four channels, whose folds spill).
-// Measured on 152 SMs for 1 to 16 strips, 0.5 to 64 strips per SM, one to four
-// channels: within 8 % of the shorter of both and 4 % of k_sor_split (which keeps 3 %
-// of advantage here), 5 % below it on average and 44 % at 16 strips per SM (152 frames of
-// 512 x 96, one channel: 8.8 ms against 4.95).  Passes of one to three iterations
-// favour k_sor_chain more, by up to three times.
-bool chain_is_shorter(int K, int strips, long long frames, int n_sms)
+// Whether k_sor_chain (one CTA per frame, or one per 512 rows) is the shorter launch, for
+// n_frames in each of `beside` launches that share the GPU.  It issues fewer instructions
+// per pixel, but needs 16 warps on an SM to cover a step's chain, where k_sor_split
+// covers it with the warps that it divides the step among: so k_sor_chain for large
+// batches.
+//
+// Times of a wavefront step in us.  An SM holds 16 warps of k_sor_chain, and a round of r
+// of them takes a + b r; launches beside one another fill each other's last rounds, but
+// take one at least.  Up to 512 rows k_sor_split takes 0.145 per strip of 32 rows and
+// SM (less with one strip per frame, more where the clusters of tall levels leave SMs
+// empty, and with four channels, whose folds spill).  Taller levels go in rounds of the
+// frames that the device holds (the driver's count), each of t2, or t1 with one CTA per
+// SM.  Measured on 152 SMs for 1 to 64 strips per frame, 0.5 to 64 per SM, one to four
+// channels: up to 512 rows within 8 % of the shorter of both and 4 % of k_sor_split
+// (which keeps 3 % of advantage), 5 % below it on average and 44 % at 16 strips per
+// SM (152 frames of 512 x 96, one channel: 8.8 ms against 4.95); 32 of 2048 x 128, two
+// channels: 27.2 ms against 16.0.  Passes of one to three iterations favour k_sor_chain
+// more, by up to three times.
+template <int K>
+bool chain_is_shorter(const DiagGeom& g, int n_frames, int beside, int dev, int n_sms)
 {
-    static constexpr float a[5] = {0.0f, 6.2f, 6.6f, 9.6f, 12.6f}, b[5] = {0.0f, 0.29f, 0.33f, 0.4f, 0.47f};
-    if (strips > kMaxLane / 32 || n_sms < 1) return false;
-    const int per_sm = kMaxLane / 32 / strips, at_once = per_sm * n_sms, rest = (int)(frames % at_once);
-    const long long full = frames / at_once;
-    const float chain = (float)full * (a[K] + b[K] * (float)(per_sm * strips)) +
-                        (rest ? a[K] + b[K] * (float)((rest + n_sms - 1) / n_sms * strips) : 0.0f);
-    const float x = (float)frames * (float)strips / (float)n_sms;
-    const float split = (strips == 1 ? 0.85f * x : (strips <= 10 ? x + 1.0f : 1.08f * x + 1.5f)) * (K == 4 ? 1.27f : 1.0f);
-    return 1.03f * chain < split;
+    static constexpr float as[5] = {0.0f, 0.90f, 0.96f, 1.39f, 1.83f}, bs[5] = {0.0f, 0.042f, 0.048f, 0.058f, 0.068f};
+    const int strips = g.P / 32;
+    const long long frames = (long long)n_frames * beside;
+    if (n_sms < 1 || beside < 1) return false;
+    const float lead = beside > 2 ? 0.95f : 1.03f;  // SMs that one launch leaves part empty take others' warps of k_sor_chain
+    if (strips <= kMaxLane / 32) {
+        const int per_sm = kMaxLane / 32 / strips, at_once = per_sm * n_sms, rest = n_frames % at_once;
+        const float round = as[K] + bs[K] * (float)(per_sm * strips);
+        float chain = (float)(n_frames / at_once) * round +
+                      (rest ? as[K] + bs[K] * (float)((rest + n_sms - 1) / n_sms * strips) : 0.0f);
+        if (beside > 1) chain = std::max(chain, (float)frames / (float)at_once * round);
+        const float x = (float)frames * (float)strips / (float)n_sms;
+        const float split =
+            0.145f * (strips == 1 ? 0.85f * x : (strips <= 10 ? x + 1.0f : 1.08f * x + 1.5f)) * (K == 4 ? 1.27f : 1.0f);
+        return lead * chain < split;
+    }
+    if constexpr (K <= 2) {
+        using Two = SplitLaunch<Ar32<K>, 2, 5, 4, 2>;
+        using Four = SplitLaunch<Ar32<K>, 4, 3, 2, 1>;
+        int nc, nt;
+        regs_split(K, g, &nc, &nt);
+        const bool four = strips > 2 * kMaxSplitCluster;
+        const int all = four ? Four::frames_at_once(dev, Four::ctas(g), 1) : Two::frames_at_once(dev, Two::ctas(g), 2);
+        const int one = four ? all : Two::frames_at_once(dev, Two::ctas(g), 1);
+        const int at_once = Four::frames_at_once(dev, nc, 1);  // one CTA per SM, as k_sor_chain's
+        if (all < 1 || one < 1 || at_once < 1) return false;
+        const float a = K == 1 ? 1.22f : 1.28f, b = K == 1 ? 0.041f : 0.054f;
+        const float t1 = K == 1 ? (four ? 0.565f : 0.42f) : (four ? 0.74f : 0.44f);
+        const float t2 = four ? t1 : (K == 1 ? 0.59f : 0.615f);
+        const int rest = (int)(frames % all);
+        float chain = (float)((n_frames + at_once - 1) / at_once);
+        if (beside > 1) chain = std::max(chain, (float)frames / (float)at_once);
+        chain *= a + b * (float)(nt / 32);
+        const float split = (float)(frames / all) * t2 + (rest == 0 ? 0.0f : (rest <= one ? t1 : t2));
+        return lead * chain < split;
+    }
+    return false;
 }
 
 }  // namespace
@@ -1110,7 +1144,10 @@ cudaError_t launch_sor_chain(const float* J, long long J_fs, const float* W, lon
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&n_sms, cudaDevAttrMultiProcessorCount, dev);
     if (e != cudaSuccess) return e;
     // up to 2048 rows: clusters of at most 16 CTAs of 128 rows
-    if (g.P / 32 <= kMaxSplitStrips && !chain_is_shorter(K, g.P / 32, (long long)n_frames * beside, n_sms)) {
+    const auto chain = [&](auto rule) { return rule(g, n_frames, beside, dev, n_sms); };
+    const bool shorter = K == 1 ? chain(chain_is_shorter<1>) : K == 2 ? chain(chain_is_shorter<2>)
+                       : K == 3 ? chain(chain_is_shorter<3>) : chain(chain_is_shorter<4>);
+    if (g.P / 32 <= kMaxSplitStrips && !shorter) {
         for (int p = 0; p < kMaxChain; ++p) TS.pk[p] = T.pk[p];
         Sor32Args S = {};
         S.J = J;
@@ -1141,7 +1178,7 @@ cudaError_t launch_sor_chain(const float* J, long long J_fs, const float* W, lon
             case 3: e = run_split32<3>(S, TS, n_frames, st); break;
             default: e = run_split32<4>(S, TS, n_frames, st); break;
         }
-        // refused clusters over 1024 rows: k_sor_chain's have at most 8 CTAs (K <= 2 there)
+        // refused clusters over 1024 rows: k_sor_chain's have at most four CTAs (K <= 2 there)
         if (e == cudaSuccess || strips_per_cta(g.P / 32, kPortableCluster) || K > 2) return e;
         cudaGetLastError();
     }

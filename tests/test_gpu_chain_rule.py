@@ -10,7 +10,7 @@ pytestmark = pytest.mark.gpu
 @pytest.mark.parametrize("H,W,K,T,its,lag", [
     (20, 12, 1, 1200, 8, 5), (20, 12, 2, 2432, 8, 5), (64, 9, 2, 1216, 7, 3), (40, 3, 1, 1216, 6, 1),
     (200, 10, 3, 300, 11, 11), (410, 8, 2, 152, 8, 5), (512, 8, 3, 152, 6, 4), (512, 7, 4, 160, 6, 5),
-    (512, 8, 1, 305, 6, 2)])
+    (512, 8, 1, 305, 6, 2), (900, 8, 2, 60, 6, 5), (1300, 8, 2, 30, 7, 3), (2040, 7, 1, 28, 6, 11)])
 def test_same_bits_on_both_sides(H, W, K, T, its, lag):
     from pyflowreg_gb300 import api
 
