@@ -828,7 +828,8 @@ def run_gb300(args):
     roofline = {
         "kernel": ("k_sor_split (float64 exact-order chained wavefront SOR, update and fold warps per 32 rows, "
                    "row strips as clusters)" if fp64
-                   else "k_sor_split (float32 exact-order chained wavefront SOR, update and fold warps per 32 "
+                   else "k_sor_chain and k_sor_split (float32 exact-order chained wavefront SOR; large batches with "
+                   "a CTA per frame, others with update and fold warps per 32 "
                    "rows, row strips as clusters)"),
         "bound": "hbm",
         "achieved": achieved,

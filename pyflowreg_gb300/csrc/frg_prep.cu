@@ -398,8 +398,8 @@ cudaError_t launch_preprocess(const float* raw, const double* raw64, int T, int 
         A.rx = A.rxk[k] > A.rx ? A.rxk[k] : A.rx;
     }
     // no temporal filter and a halo that fits the shared memory every launch has (three blocks and more per SM):
-    // both correlations in one kernel; else the two-kernel form, which normalises once per tap (4.6 times the time at
-    // sigma 1) but takes any radius
+    // both correlations in one kernel; else the two-kernel form, which normalises once per tap (3.0 times the time on
+    // ten frames of 512 x 512 x 4 at sigma 1) but takes any radius
     const size_t elem = f32_storage ? sizeof(float) : sizeof(double);
     const size_t cols = kPrepTile + 2 * (size_t)A.rx;
     const size_t smem = (size_t)(A.ry + A.rx + 2) * 16 + elem * cols * (2 * kPrepTile + 2 * (size_t)A.ry);
